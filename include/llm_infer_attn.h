@@ -288,8 +288,8 @@ int attn_argmax(uint32_t* out, const float* logits, uint32_t batch, uint32_t voc
 /* C[t][j] (+)= sum_i (a_hi[t][i] + a_lo[t][i]) * w[j][i]: t < m tokens, j < n_out, i < k. a_hi, a_lo fp16 [m][k] and
  * w fp16 [n_out][k] (the engine's weight layout, k fastest), c fp32 with row stride ldc. Replaces, for m tokens at
  * once, matmul() of include/kernels_cpu.hpp:69-80 / fused_gemv_clip of src/kernels.cu:229-239. a_lo may be NULL (one
- * MMA per k-step instead of two): a caller whose weights are not exact in fp16 (Q8_0) makes a second call with the
- * weights' residual, a_lo = NULL and accumulate = 1. k a multiple of 64, n_out a multiple of 32, pointers 16-byte
+ * MMA per k-step instead of two): a caller whose weights are not exact in fp16 (Q8_0) uses attn_gemm_pair, or
+ * makes a second call with the weights' residual, a_lo = NULL and accumulate = 1. k a multiple of 64, n_out a multiple of 32, pointers 16-byte
  * aligned. */
 typedef struct AttnGemmArgs {
     float* c;
@@ -302,6 +302,26 @@ typedef struct AttnGemmArgs {
     uint32_t* status;    /* optional device word for ATTN_STATUS_* bits */
 } AttnGemmArgs;
 int attn_gemm_f16(const AttnGemmArgs* args, void* stream);
+
+/* The same with weights that are themselves an fp16 pair (Q8_0 expanded by attn_dequant_q8_0_f16pair; w_lo may be NULL)
+ * in one pass: A_hi W_hi + A_lo W_hi + A_hi W_lo, the products with a residual summed in an accumulator of their own.
+ * With swiglu != 0 the matrix holds n_out gate rows followed by n_out up rows, and instead of c the call writes
+ * silu(gate) * up (src/model/block.cpp:206-210) as the fp16 pair out_hi, out_lo [m][n_out] (no accumulate). */
+typedef struct AttnGemmPairArgs {
+    float* c;            /* swiglu = 0: [m][ldc] fp32 */
+    void* out_hi;        /* swiglu = 1 */
+    void* out_lo;
+    const void* a_hi;    /* fp16 [m][k] */
+    const void* a_lo;    /* fp16 [m][k] or NULL */
+    const void* w_hi;    /* fp16 [n_out][k], swiglu: [2 n_out][k] */
+    const void* w_lo;    /* same shape or NULL */
+    uint64_t ldc;        /* floats between rows of c; 0 = n_out */
+    uint32_t m, n_out, k;
+    int32_t accumulate;
+    int32_t swiglu;
+    uint32_t* status;
+} AttnGemmPairArgs;
+int attn_gemm_pair(const AttnGemmPairArgs* args, void* stream);
 
 /* Row-wise RMSNorm (include/kernels_cpu.hpp:43-67) of x [rows][dim] fp32, written as the fp16 pair hi, lo [rows][dim]. */
 int attn_rmsnorm_f16pair(void* hi, void* lo, const float* x, const float* weight, uint32_t rows, uint32_t dim, float eps,
@@ -429,7 +449,8 @@ uint64_t attn_kernel_launch_count(void);
 
 /* sizeof() of an argument structure as this library was compiled, so that a foreign-function binding can check its own
  * mirror of the layout: 0 AttnDecodeArgs, 1 AttnDecodeShardedArgs, 2 AttnPrefillArgs, 3 AttnRopeInsertArgs,
- * 4 AttnGemvArgs, 5 AttnMergeArgs, 6 AttnGemmArgs, 7 AttnRopePromptArgs; 0 for any other index. */
+ * 4 AttnGemvArgs, 5 AttnMergeArgs, 6 AttnGemmArgs, 7 AttnRopePromptArgs,
+ * 8 AttnGemmPairArgs; 0 for any other index. */
 size_t attn_abi_struct_size(int which);
 
 #ifdef __cplusplus

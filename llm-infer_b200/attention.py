@@ -548,6 +548,40 @@ def gemm_f16(a_hi: torch.Tensor, a_lo, w: torch.Tensor, *, out: torch.Tensor, ac
     return out
 
 
+def gemm_pair(a_pair, w_pair, *, out, accumulate: bool = False, swiglu: bool = False, status=None, stream=None):
+    """gemm_f16 for weights that are an fp16 (value, residual) pair themselves (dequant_q8_0_pair; the residual may be
+    None), all products in one pass: a_pair = (a_hi, a_lo or None) fp16 [m, k], w_pair = (w_hi, w_lo or None) fp16
+    [n_out, k]. ``swiglu``: w holds n_out gate rows then n_out up rows and ``out`` is the fp16 pair [m, n_out] that
+    receives silu(gate) * up; otherwise ``out`` is fp32 [m, n_out] (rows may be strided)."""
+    (a_hi, a_lo), (w_hi, w_lo) = a_pair, w_pair
+    outs = tuple(out) if swiglu else (out,)
+    _require_cuda(a_hi, a_lo, w_hi, w_lo, *outs)
+    m, k = a_hi.shape
+    n_out = w_hi.shape[0] // 2 if swiglu else w_hi.shape[0]
+    for pair, shape in ((a_pair, (m, k)), (w_pair, (w_hi.shape[0], k)), (outs if swiglu else (), (m, n_out))):
+        for t in pair:
+            if t is not None and (t.shape != shape or t.dtype != torch.float16 or not t.is_contiguous()):
+                raise ValueError("pairs must be dense fp16: a [m, k], w [n_out, k] (swiglu: [2 n_out, k], out [m, n_out])")
+    a = _b.AttnGemmPairArgs()
+    if swiglu:
+        if accumulate or w_hi.shape[0] % 2 or len(outs) != 2:
+            raise ValueError("swiglu needs gate rows and up rows, a pair as output and no accumulate")
+        a.out_hi, a.out_lo = outs[0].data_ptr(), outs[1].data_ptr()
+    else:
+        if out.shape != (m, n_out) or out.dtype != torch.float32 or out.stride(1) != 1:
+            raise ValueError("out must be fp32 [m, n_out] with dense rows")
+        a.c, a.ldc = out.data_ptr(), out.stride(0)
+    a.a_hi, a.w_hi = a_hi.data_ptr(), w_hi.data_ptr()
+    a.a_lo = a_lo.data_ptr() if a_lo is not None else None
+    a.w_lo = w_lo.data_ptr() if w_lo is not None else None
+    a.m, a.n_out, a.k = m, n_out, k
+    a.accumulate, a.swiglu = int(bool(accumulate)), int(bool(swiglu))
+    a.status = status.data_ptr() if status is not None else None
+    with torch.cuda.device(a_hi.device):
+        _b.check(_b.load().attn_gemm_pair(C.byref(a), _stream_ptr(stream)), "attn_gemm_pair")
+    return out
+
+
 def rmsnorm_pair(x: torch.Tensor, weight: torch.Tensor, eps: float, *, out=None, stream=None):
     """RMSNorm of every row of x [rows, dim] fp32, written as the fp16 (value, residual) pair that gemm_f16 reads."""
     _require_cuda(x, weight)

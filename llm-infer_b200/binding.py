@@ -32,6 +32,7 @@ EXPORTED_SYMBOLS = (
     "attn_prefill_causal",
     "attn_rope_kv_insert",
     "attn_gemm_f16",
+    "attn_gemm_pair",
     "attn_rmsnorm_f16pair",
     "attn_split_f16pair",
     "attn_swiglu_f16pair",
@@ -229,6 +230,25 @@ class AttnGemmArgs(C.Structure):
     ]
 
 
+class AttnGemmPairArgs(C.Structure):
+    _fields_ = [
+        ("c", C.c_void_p),
+        ("out_hi", C.c_void_p),
+        ("out_lo", C.c_void_p),
+        ("a_hi", C.c_void_p),
+        ("a_lo", C.c_void_p),
+        ("w_hi", C.c_void_p),
+        ("w_lo", C.c_void_p),
+        ("ldc", C.c_uint64),
+        ("m", C.c_uint32),
+        ("n_out", C.c_uint32),
+        ("k", C.c_uint32),
+        ("accumulate", C.c_int32),
+        ("swiglu", C.c_int32),
+        ("status", C.c_void_p),
+    ]
+
+
 class AttnRopePromptArgs(C.Structure):
     _fields_ = [
         ("q_out", C.c_void_p),
@@ -318,6 +338,8 @@ def load() -> C.CDLL:
     lib.attn_merge.argtypes = [C.POINTER(AttnMergeArgs), C.c_void_p]
     lib.attn_gemm_f16.restype = C.c_int
     lib.attn_gemm_f16.argtypes = [C.POINTER(AttnGemmArgs), C.c_void_p]
+    lib.attn_gemm_pair.restype = C.c_int
+    lib.attn_gemm_pair.argtypes = [C.POINTER(AttnGemmPairArgs), C.c_void_p]
     lib.attn_rmsnorm_f16pair.restype = C.c_int
     lib.attn_rmsnorm_f16pair.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_uint32, C.c_uint32, C.c_float,
                                          C.c_void_p]
@@ -338,7 +360,7 @@ def load() -> C.CDLL:
     lib.attn_abi_struct_size.restype = C.c_size_t
     lib.attn_abi_struct_size.argtypes = [C.c_int]
     mirrors = (AttnDecodeArgs, AttnDecodeShardedArgs, AttnPrefillArgs, AttnRopeInsertArgs, AttnGemvArgs, AttnMergeArgs,
-               AttnGemmArgs, AttnRopePromptArgs)
+               AttnGemmArgs, AttnRopePromptArgs, AttnGemmPairArgs)
     for index, mirror in enumerate(mirrors):
         if lib.attn_abi_struct_size(index) != C.sizeof(mirror):
             raise RuntimeError(f"{mirror.__name__}: the ctypes mirror ({C.sizeof(mirror)} bytes) does not match the "

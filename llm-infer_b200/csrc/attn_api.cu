@@ -295,6 +295,7 @@ size_t attn_abi_struct_size(int which) {
         case 5: return sizeof(AttnMergeArgs);
         case 6: return sizeof(AttnGemmArgs);
         case 7: return sizeof(AttnRopePromptArgs);
+        case 8: return sizeof(AttnGemmPairArgs);
         default: return 0;
     }
 }

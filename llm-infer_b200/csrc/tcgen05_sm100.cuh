@@ -1,6 +1,7 @@
 // Inline-PTX wrappers for the 5th-generation tensor cores of sm_100a (tcgen05 + tensor memory) and the tiled TMA
 // copies that feed them, shared by the kernels that run a real contraction (causal prefill, the batched projection
-// GEMM). One CTA per tile group (cta_group::1) everywhere; no cluster multicast anywhere.
+// GEMM). cta_group::1 forms, and cta_group::2 forms for a pair of CTAs that share one tile (the two CTAs of a cluster of
+// two); every copy lands in the issuing CTA's own shared memory, none is multicast.
 #pragma once
 
 #include <cuda.h>
@@ -9,6 +10,18 @@
 
 namespace b200 {
 namespace tc {
+
+// One lane of the (converged) warp. The roles that issue tcgen05.mma and TMA copies are entered through this and not
+// through `lane == 0`: the compiler then knows that a single thread runs them and issues these instructions, whose
+// operands live in uniform registers, straight from the uniform datapath. Four 128 x 128 x 16 MMAs with the wait and the
+// commit around them take 267 clocks that way, 499 behind `lane == 0` (256 is the tensor pipe's own time).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
+    return p != 0;
+}
+// The warp's index in the block, in a form the compiler knows to be the same in all its lanes.
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x) >> 5, 0); }
 
 // ---- tiled TMA copies (coordinates innermost first; the innermost one times the element size must be a multiple
 //      of 16 bytes) ----
@@ -41,7 +54,60 @@ __device__ __forceinline__ void named_bar_sync(int id, int threads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
+// The two-CTA form: the copy lands in this CTA's shared memory, its bytes are counted on the barrier at the same
+// offset in the pair's leader (bit 24 of a shared-window address selects the odd CTA of the pair; cleared = leader).
+constexpr uint32_t kLeaderMask = 0xFEFFFFFFu;
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        ::"r"(dst), "l"(map), "r"(bar & kLeaderMask), "r"(c0), "r"(c1)
+        : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// Both CTAs of the cluster meet (every thread of both).
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// One arrival on the barrier at the same offset in CTA `cta` of the cluster.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar, uint32_t cta) {
+    asm volatile(
+        "{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, %1;\n\t"
+        "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [ra];\n\t}"
+        ::"r"(bar), "r"(cta)
+        : "memory");
+}
+
 // ---- tensor memory ----
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_dst, uint32_t cols) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(cols) : "memory");
+}
+__device__ __forceinline__ void tmem_relinquish_pair() {
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t cols) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
+}
+// The barrier at this offset receives one arrival in both CTAs of the pair when every MMA issued so far by this thread
+// has completed.
+__device__ __forceinline__ void commit_pair(uint32_t bar) {
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+        ::"r"(bar), "h"(static_cast<uint16_t>(3))
+        : "memory");
+}
+// D (+)= A * B over the pair: A rows 0-127 and half of B's rows in the leader's shared memory, A rows 128-255 and the
+// other half of B's rows at the same offsets in its partner; each CTA's tensor memory receives its own rows of D.
+__device__ __forceinline__ void mma_ss_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(acc)
+        : "memory");
+}
 __device__ __forceinline__ void tmem_alloc(uint32_t smem_dst, uint32_t cols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(cols) : "memory");
 }
@@ -86,6 +152,15 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&r)[32]) {
         : "r"(taddr)
         : "memory");
 }
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&r)[16]) {
+    uint32_t* u = reinterpret_cast<uint32_t*>(r);
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]),
+          "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15])
+        : "r"(taddr)
+        : "memory");
+}
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
@@ -98,7 +173,8 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo_bytes,
 
 // Instruction descriptor of kind::f16: fp32 accumulate, A format a_fmt and B format b_fmt (0 = f16, 1 = bf16; give
 // both the same value: a mixed pair raised an illegal-instruction error on B200), A K-major, B K-major (b_mn = 0) or
-// MN-major (b_mn = 1), M x N = m x n (m 64 or 128, n a multiple of 8 (m 64) or 16 (m 128) up to 256).
+// MN-major (b_mn = 1), M x N = m x n (m 64 or 128, n a multiple of 8 (m 64) or 16 (m 128) up to 256; over a pair of CTAs
+// m 256, n a multiple of 32 up to 256).
 __host__ __device__ constexpr uint32_t instr_desc(uint32_t a_fmt, uint32_t b_fmt, uint32_t b_mn, uint32_t m, uint32_t n) {
     return (1u << 4) | (a_fmt << 7) | (b_fmt << 10) | (b_mn << 16) | ((n >> 3) << 17) | ((m >> 4) << 24);
 }

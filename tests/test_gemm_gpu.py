@@ -57,6 +57,54 @@ def test_gemm_against_float64_and_accumulate(A, m, n_out, k):
     assert int(status.item()) == 0
 
 
+def _truncation_bound(k, products, scale):
+    """The tensor cores drop what lies below the accumulator's last bit once per k-step of 16 and product: at most
+    2^-23 of the running sum each, which stays below the largest output here."""
+    return (k / 16 * products * 2.0 ** -23 + 2.0 ** -20) * scale
+
+
+# one token, around 128 and 256 (single CTA / pair), several bands of rows, widths that leave part of a tile
+@pytest.mark.parametrize("m,n_out,k", [(1, 32, 64), (128, 96, 128), (129, 160, 192), (256, 256, 64), (257, 4128, 256),
+                                       (700, 1056, 512), (2500, 416, 14336)])
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_gemm_with_paired_weights(A, m, n_out, k, swiglu):
+    """attn_gemm_pair against float64: three products in one pass, accumulate, and the SwiGLU epilogue."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(m + n_out + k)
+    x = torch.randn((m, k), generator=g, device="cuda")
+    w = torch.randn((n_out * (2 if swiglu else 1), k), generator=g, device="cuda") * k ** -0.5
+    split = lambda t: (t.half(), (t - t.half().float()).half())  # noqa: E731
+    (ah, al), (wh, wl) = split(x), split(w)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    a64, w64 = ah.double() + al.double(), wh.double() + wl.double()
+    prod = a64 @ w64.T  # the product of the two residuals, 2^-24 of a term, is not part of the result
+    tol = _truncation_bound(k, 1, float(prod.abs().max()))
+    if swiglu:
+        out = tuple(torch.full((m, n_out), float("nan"), dtype=torch.float16, device="cuda") for _ in range(2))
+        A.gemm_pair((ah, al), (wh, wl), out=out, swiglu=True, status=status)
+        gate, up = prod[:, :n_out], prod[:, n_out:]
+        want = gate / (1 + torch.exp(-gate)) * up
+        # d(silu(g) u) <= 1.1 |u| dg + |g| du, and the pair's own 2^-21 of the value
+        bound = 1.1 * tol * (up.abs() + gate.abs()) + 2.0 ** -20 * want.abs() + 2.0 ** -24
+        assert bool(((out[0].double() + out[1].double() - want).abs() <= bound).all())
+        only = tuple(torch.empty_like(t) for t in out)
+        A.gemm_pair((ah, None), (wh, None), out=only, swiglu=True, status=status)
+        p1 = ah.double() @ wh.double().T
+        gate, up = p1[:, :n_out], p1[:, n_out:]
+        want = gate / (1 + torch.exp(-gate)) * up
+        bound = 1.1 * tol * (up.abs() + gate.abs()) + 2.0 ** -20 * want.abs() + 2.0 ** -24
+        assert bool(((only[0].double() + only[1].double() - want).abs() <= bound).all())
+    else:
+        wide = torch.zeros((m, n_out + 32), device="cuda")
+        A.gemm_pair((ah, al), (wh, wl), out=wide[:, :n_out], status=status)
+        assert float((wide[:, :n_out].double() - prod).abs().max()) <= tol
+        assert bool((wide[:, n_out:] == 0).all()), "nothing written past the row"
+        A.gemm_pair((ah, None), (wh, wl), out=wide[:, :n_out], accumulate=True, status=status)
+        want = prod + ah.double() @ w64.T
+        assert float((wide[:, :n_out].double() - want).abs().max()) <= 3 * tol
+    assert int(status.item()) == 0
+
+
 def test_gemm_rows_equal_the_engine_matmul(A, checker):
     """Each token's row of the GEMM against the engine's own per-token matmul() on the fp32 activations."""
     import torch
