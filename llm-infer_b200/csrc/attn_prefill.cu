@@ -37,6 +37,7 @@
 
 #include "attn_internal.cuh"
 #include "ptx_sm100.cuh"
+#include "tcgen05_sm100.cuh"
 #include "tma_tile.cuh"
 
 namespace b200 {
@@ -221,7 +222,7 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     volatile uint32_t* tmem_ptr_smem = reinterpret_cast<volatile uint32_t*>(smem + kSmemTmemPtr);
 
     const int tid = threadIdx.x;
-    const int warp = tid >> 5;
+    const int warp = tc::uniform_warp();
     const int lane = tid & 31;
     constexpr int HD = HDIM;
     constexpr uint32_t kLoadBytes = (HD / 64) * kSubTileBytes;  // bytes of one Q / K / V tile actually loaded
@@ -447,7 +448,7 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         }
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
-        if (warp == 8 && lane == 0) {
+        if (warp == 8 && tc::elect_one()) {
             // =============================== TMA producer ===============================
             uint32_t n_q = 0;
             for (int t = 0; t < 2; ++t) n_q += nblk[t] > 0;
@@ -477,7 +478,7 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 tma_load_4d(vdst, &tm_v, bar(BAR_V_FULL + st), 0, j * BN, kvh, b);
                 if (HD > 64) tma_load_4d(vdst + kSubTileBytes, &tm_v, bar(BAR_V_FULL + st), 64, j * BN, kvh, b);
             }
-        } else if (warp == 9 && lane == 0 && n_iter > 0) {
+        } else if (warp == 9 && n_iter > 0 && tc::elect_one()) {
             // =============================== MMA issuer ===============================
             constexpr uint32_t fmt = BF16 ? 1u : 0u;
             constexpr uint32_t idesc_qk = instr_desc(fmt, fmt, 0, BN);  // S: 128 rows x 128 keys
