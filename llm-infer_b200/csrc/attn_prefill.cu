@@ -13,16 +13,20 @@
 // same rows when the GQA group is even, else two consecutive row tiles of one head), 12 warps:
 //   warps 0-3   softmax of tile 0: thread r owns query row r (tensor-memory lane r), no shuffles needed
 //   warps 4-7   softmax of tile 1
-//   warp  8     TMA producer: Q tiles once, then K and V tiles (128 keys x 128 dims, 128-byte swizzle)
-//               through a 2-stage ring with separate barriers for K and V
+//   warp  8     TMA producer: Q tiles once, then K and V tiles (64 keys x 128 dims, 128-byte swizzle)
+//               through a 4-stage ring with separate barriers for K and V
 //   warp  9     one thread issues every tcgen05.mma: S_t = Q_t K^T (both operands in shared memory,
 //               accumulator in tensor memory) and O_t += P_t V (P read from tensor memory, V from shared
-//               memory as an MN-major operand), in the order PV_0(j), QK_0(j+1), PV_1(j), QK_1(j+1) so the
-//               softmax of one tile overlaps the tensor work of the other
+//               memory as an MN-major operand), in the order PV_0(j), QK_0(j+2), PV_1(j), QK_1(j+2)
 //   warps 10-11 idle (they only take part in the register re-allocation of their warpgroup)
-// Tensor memory (512 columns): S_0 | S_1 | O_0 | O_1, 128 fp32 columns each. P overwrites S in place as
-// packed 16-bit pairs in columns [0,64). Two ways to hand P to the tensor cores (template PMODE):
-//   kPResidual  P in the input type plus its rounding residual in columns [64,128) and a second PV MMA: ~2^-17,
+// Tensor memory (512 columns): two score buffers of 64 columns per tile, then O_0 | O_1, 128 fp32 columns each. With two
+// score buffers the softmax of block j+1 never waits for the products of block j: with one buffer of 128 keys a tile's
+// softmax (~ 2 000 clocks) and its 24 MMAs (1 536) took turns. An m128n64k16 MMA takes 48 clocks (its shared-memory
+// reads), so 128 keys cost 3 584 tensor clocks for both tiles instead of 3 072, which still is less than the turns.
+// 4 x 2048 rows, 32/8 heads of 128, bf16: 220 -> 196 us (701 TFLOP/s causal).
+// P overwrites S in place as packed 16-bit pairs in columns [0,32). Two ways to hand P to the tensor cores (template
+// PMODE):
+//   kPResidual  P in the input type plus its rounding residual in columns [32,64) and a second PV MMA: ~2^-17,
 //               the mode that meets the parity tolerance on every row (the default).
 //   kPInput     P rounded once to the input type (fp16: 2^-11, bf16: 2^-9 per element), one PV MMA.
 // A and B of one MMA must have the same 16-bit format: an fp16 P against a bf16 V (the instruction descriptor has
@@ -44,12 +48,14 @@ namespace b200 {
 namespace {
 
 constexpr int BM = 128;   // query rows per tile
-constexpr int BN = 128;   // keys per block
-constexpr int kMaxHD = 128;  // head_dim is 128 or 64 (template HDIM); shared memory is laid out for 128
+constexpr int BN = 64;    // keys per block
+// head_dim is 128 or 64 (template HDIM); shared memory is laid out for 128
 constexpr int kThreads = 384;
-constexpr uint32_t kSubTileBytes = 128 * 64 * 2;       // [128 rows][64 elements], 128-byte rows, swizzled
+constexpr uint32_t kSubTileBytes = BM * 64 * 2;        // [128 query rows][64 elements], 128-byte rows, swizzled
 constexpr uint32_t kTileBytes = 2 * kSubTileBytes;     // 128 x 128 16-bit elements (head_dim 64 fills the first half)
-constexpr int kStages = 2;
+constexpr uint32_t kKvSubBytes = BN * 64 * 2;          // the same of a key block
+constexpr uint32_t kKvBytes = 2 * kKvSubBytes;
+constexpr int kStages = 4;
 constexpr uint32_t kTmemCols = 512;
 #ifdef ATTN_TRACE
 float* g_prefill_debug = nullptr;
@@ -78,16 +84,18 @@ enum {
     BAR_V_FULL = BAR_K_FULL + kStages,
     BAR_K_EMPTY = BAR_V_FULL + kStages,
     BAR_V_EMPTY = BAR_K_EMPTY + kStages,
-    BAR_S_FULL = BAR_V_EMPTY + kStages,  // [2] per tile
-    BAR_P_FULL = BAR_S_FULL + 2,
-    BAR_O_FULL = BAR_P_FULL + 2,
-    BAR_COUNT = BAR_O_FULL + 2
+    BAR_S_FULL = BAR_V_EMPTY + kStages,
+    // [tile][block parity]: scores are there, probabilities are there, the block's PV product is complete. Two barriers
+    // each, because scores run two blocks ahead: a side may be one phase behind, which one parity bit cannot tell.
+    BAR_P_FULL = BAR_S_FULL + 4,
+    BAR_O_DONE = BAR_P_FULL + 4,
+    BAR_COUNT = BAR_O_DONE + 4
 };
 
 constexpr uint32_t kSmemQ = 0;
 constexpr uint32_t kSmemK = kSmemQ + 2 * kTileBytes;
-constexpr uint32_t kSmemV = kSmemK + kStages * kTileBytes;
-constexpr uint32_t kSmemStage = kSmemV + kStages * kTileBytes;   // per tile: [128 rows][128 B] output staging
+constexpr uint32_t kSmemV = kSmemK + kStages * kKvBytes;
+constexpr uint32_t kSmemStage = kSmemV + kStages * kKvBytes;   // per tile: [128 rows][128 B] output staging
 constexpr uint32_t kStageTileBytes = 128 * 128;
 constexpr uint32_t kSmemBars = kSmemStage + 2 * kStageTileBytes;
 constexpr uint32_t kSmemTmemPtr = kSmemBars + BAR_COUNT * 8;
@@ -204,6 +212,39 @@ __host__ __device__ constexpr uint32_t instr_desc(uint32_t a_fmt, uint32_t b_fmt
     return (1u << 4) | (a_fmt << 7) | (b_fmt << 10) | (b_mn << 16) | ((n >> 3) << 17) | ((128u >> 4) << 24);
 }
 
+// Two fp32 operations per instruction.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack_f32x2(float a, float b) {
+    f32x2 v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+    return v;
+}
+__device__ __forceinline__ void unpack_f32x2(f32x2 v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 fma_f32x2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f32x2 add_f32x2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&u)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+        ::"r"(taddr), "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]), "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7]), "r"(u[8]),
+          "r"(u[9]), "r"(u[10]), "r"(u[11]), "r"(u[12]), "r"(u[13]), "r"(u[14]), "r"(u[15])
+        : "memory");
+}
+
 __device__ __forceinline__ void report_timeout(uint32_t* status) {
     if (status) atomicOr(status, ATTN_STATUS_WAIT_TIMEOUT);
 }
@@ -225,7 +266,7 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     const int warp = tc::uniform_warp();
     const int lane = tid & 31;
     constexpr int HD = HDIM;
-    constexpr uint32_t kLoadBytes = (HD / 64) * kSubTileBytes;  // bytes of one Q / K / V tile actually loaded
+    constexpr uint32_t kLoadQ = (HD / 64) * kSubTileBytes, kLoadKv = (HD / 64) * kKvSubBytes;  // bytes of a tile actually loaded
 
     // ---- which two tiles does this CTA own ----
     // The row-tile index is the slowest-varying grid dimension and counts down, so every CTA with the longest
@@ -249,7 +290,7 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     uint32_t nblk[2];
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
-        nblk[t] = m0[t] < p.seq ? min(nblk_total, m0[t] / BN + 1) : 0u;
+        nblk[t] = m0[t] < p.seq ? min(nblk_total, (m0[t] + BM) / BN) : 0u;
     }
     const uint32_t n_iter = max(nblk[0], nblk[1]);
 
@@ -263,9 +304,12 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             mbar_init(bar(BAR_V_EMPTY + s), 1);
         }
         for (int t = 0; t < 2; ++t) {
-            mbar_init(bar(BAR_S_FULL + t), 1);
-            mbar_init(bar(BAR_P_FULL + t), 128);
-            mbar_init(bar(BAR_O_FULL + t), 1);
+            mbar_init(bar(BAR_S_FULL + 2 * t), 1);
+            mbar_init(bar(BAR_S_FULL + 2 * t + 1), 1);
+            mbar_init(bar(BAR_P_FULL + 2 * t), 128);
+            mbar_init(bar(BAR_P_FULL + 2 * t + 1), 128);
+            mbar_init(bar(BAR_O_DONE + 2 * t), 1);
+            mbar_init(bar(BAR_O_DONE + 2 * t + 1), 1);
         }
         mbar_init_fence();
     }
@@ -277,7 +321,7 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_ptr_smem;
-    auto tmem_s = [&](int t) { return tmem_base + static_cast<uint32_t>(t) * 128u; };
+    auto tmem_s = [&](int t, uint32_t buf) { return tmem_base + static_cast<uint32_t>(t) * 128u + buf * 64u; };
     auto tmem_o = [&](int t) { return tmem_base + 256u + static_cast<uint32_t>(t) * 128u; };
 
     if (warp < 8) {
@@ -286,41 +330,46 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         const int t = warp >> 2;                       // tile
         const int r = ((warp & 3) << 5) | lane;        // row inside the tile = tensor-memory lane
         const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) << 5) << 16;
-        const uint32_t q_row = m0[t] + r;              // row index inside the sequence
+        const uint32_t my_m0 = t ? m0[1] : m0[0], my_head = t ? head[1] : head[0], my_nblk = t ? nblk[1] : nblk[0];
+        const uint32_t q_row = my_m0 + r;              // row index inside the sequence
         float m_used = -INFINITY;                      // maximum the stored probabilities are relative to (log2 units)
         float l = 0.f;
         bool ok = true;
-        for (uint32_t j = 0; j < nblk[t] && ok; ++j) {
-            if (!mbar_wait(bar(BAR_S_FULL + t), j & 1)) { report_timeout(p.status); ok = false; break; }
+        for (uint32_t j = 0; j < my_nblk && ok; ++j) {
+            const uint32_t s_tmem = tmem_s(t, j & 1) + lane_addr;
+            if (!mbar_wait(bar(BAR_S_FULL + 2 * t + (j & 1)), (j >> 1) & 1)) { report_timeout(p.status); ok = false; break; }
             tc_fence_after();
-            float s[128];
+            float s[BN];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                tmem_ld32(tmem_s(t) + lane_addr + c * 32, *reinterpret_cast<float(*)[32]>(&s[c * 32]));
+            for (int c = 0; c < BN / 32; ++c) {
+                tmem_ld32(s_tmem + c * 32, *reinterpret_cast<float(*)[32]>(&s[c * 32]));
             }
             tmem_wait_ld();
 #ifdef ATTN_TRACE
-            if (p.debug && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == gridDim.z - 1 && t == 0 && j == 0) {
+            if (p.debug && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == gridDim.z - 1 && t == 0 && j < 2) {
 #pragma unroll
-                for (int c = 0; c < 128; ++c) p.debug[r * 128 + c] = s[c];
+                for (int c = 0; c < BN; ++c) p.debug[r * 128 + j * BN + c] = s[c];
             }
 #endif
-            // causal mask: only the diagonal block needs it (keys of later blocks are never visited)
+            // causal mask: only the diagonal blocks need it (keys of later blocks are never visited)
             if (j * BN + BN - 1 > q_row) {
 #pragma unroll
-                for (int c = 0; c < 128; ++c) {
+                for (int c = 0; c < BN; ++c) {
                     if (j * BN + c > q_row) s[c] = -INFINITY;
                 }
             }
-            // eight independent chains, then a tree: a single chain of 127 dependent max operations would
-            // leave this warp's scheduler idle most of the time (only two softmax warps share a scheduler)
-            float mx8[8];
+            // four independent chains of three-input maxima
+            float mx4[4];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) mx8[i] = s[i];
+            for (int i = 0; i < 4; ++i) mx4[i] = max3(s[i], s[4 + i], s[8 + i]);
 #pragma unroll
-            for (int c = 8; c < 128; ++c) mx8[c & 7] = fmaxf(mx8[c & 7], s[c]);
-            float mx = fmaxf(fmaxf(fmaxf(mx8[0], mx8[1]), fmaxf(mx8[2], mx8[3])),
-                             fmaxf(fmaxf(mx8[4], mx8[5]), fmaxf(mx8[6], mx8[7])));
+            for (int c = 12; c + 8 <= BN; c += 8) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) mx4[i] = max3(mx4[i], s[c + i], s[c + 4 + i]);
+            }
+            float mx = max3(fmaxf(mx4[0], mx4[1]), mx4[2], mx4[3]);
+#pragma unroll
+            for (int c = 12 + (BN - 12) / 8 * 8; c < BN; ++c) mx = fmaxf(mx, s[c]);
             mx *= p.scale_log2;
             // Rescale only when the maximum grew by more than 8 (probabilities stay below 2^8).
             float factor = 1.f;
@@ -328,9 +377,13 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 factor = fast_exp2(m_used - mx);  // 0 on the first block (m_used = -inf)
                 m_used = mx;
             }
+            // Products of earlier blocks: the scores of block j were issued behind PV(j-2), so that one is over (waiting
+            // for every phase in turn keeps the parities unambiguous); PV(j-1) may still be running and is
+            // waited for only when O has to be rescaled.
+            if (j >= 2 && !mbar_wait(bar(BAR_O_DONE + 2 * t + (j & 1)), ((j - 2) >> 1) & 1)) { report_timeout(p.status); ok = false; break; }
             if (j > 0 && __any_sync(0xffffffffu, factor != 1.f)) {
-                // O_t is stable here: the MMA that produced this S tile was issued after PV_t(j-1)
-                // and the tensor pipe completes in order.
+                if (!mbar_wait(bar(BAR_O_DONE + 2 * t + ((j - 1) & 1)), ((j - 1) >> 1) & 1)) { report_timeout(p.status); ok = false; break; }
+                tc_fence_after();
 #pragma unroll
                 for (int c = 0; c < HD / 32; ++c) {
                     float o[32];
@@ -343,49 +396,47 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 }
             }
             l *= factor;
-            // probabilities; P overwrites S in place (every S value of this row is already in registers)
-            float sum4[4] = {0.f, 0.f, 0.f, 0.f};
+            // probabilities; P overwrites S in place (every S value of this row is already in registers). Pairs of
+            // elements share one packed fp32 instruction (scale, residual, sum).
+            const f32x2 scale2 = pack_f32x2(p.scale_log2, p.scale_log2), m2 = pack_f32x2(-m_used, -m_used);
+            const f32x2 minus1 = pack_f32x2(-1.f, -1.f);
+            f32x2 sum2[2] = {pack_f32x2(0.f, 0.f), pack_f32x2(0.f, 0.f)};
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
+            for (int c = 0; c < BN / 32; ++c) {
                 uint32_t hi[16], lo[16];
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                    const float p0 = fast_exp2(fmaf(s[c * 32 + 2 * i], p.scale_log2, -m_used));
-                    const float p1 = fast_exp2(fmaf(s[c * 32 + 2 * i + 1], p.scale_log2, -m_used));
-                    sum4[i & 3] += p0 + p1;
+                    float p0, p1;
+                    unpack_f32x2(fma_f32x2(pack_f32x2(s[c * 32 + 2 * i], s[c * 32 + 2 * i + 1]), scale2, m2), p0, p1);
+                    p0 = fast_exp2(p0);
+                    p1 = fast_exp2(p1);
+                    const f32x2 pp = pack_f32x2(p0, p1);
+                    sum2[i & 1] = add_f32x2(sum2[i & 1], pp);
                     // Rounded pair by one packed convert; its fp32 value is recovered with integer / half-add
                     // operations so that no scalar convert (special-function pipe, already busy with exp2) is used.
                     hi[i] = pack2<BF16>(p0, p1);
                     if constexpr (PMODE == kPResidual) {
                         float h0, h1;
                         unpack2<BF16>(hi[i], h0, h1);
-                        lo[i] = pack2<BF16>(p0 - h0, p1 - h1);
+                        float r0, r1;
+                        unpack_f32x2(fma_f32x2(pack_f32x2(h0, h1), minus1, pp), r0, r1);
+                        lo[i] = pack2<BF16>(r0, r1);
                     }
                 }
-                // 32 keys -> 16 packed columns: rounded part at column 16c, residual at 64 + 16c
-                asm volatile(
-                    "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-                    ::"r"(tmem_s(t) + lane_addr + c * 16), "r"(hi[0]), "r"(hi[1]), "r"(hi[2]), "r"(hi[3]), "r"(hi[4]),
-                      "r"(hi[5]), "r"(hi[6]), "r"(hi[7]), "r"(hi[8]), "r"(hi[9]), "r"(hi[10]), "r"(hi[11]), "r"(hi[12]),
-                      "r"(hi[13]), "r"(hi[14]), "r"(hi[15])
-                    : "memory");
-                if constexpr (PMODE == kPResidual) {
-                    asm volatile(
-                        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-                        ::"r"(tmem_s(t) + lane_addr + 64 + c * 16), "r"(lo[0]), "r"(lo[1]), "r"(lo[2]), "r"(lo[3]),
-                          "r"(lo[4]), "r"(lo[5]), "r"(lo[6]), "r"(lo[7]), "r"(lo[8]), "r"(lo[9]), "r"(lo[10]), "r"(lo[11]),
-                          "r"(lo[12]), "r"(lo[13]), "r"(lo[14]), "r"(lo[15])
-                        : "memory");
-                }
+                // 32 keys -> 16 packed columns: rounded part at column 16c, residual at BN / 2 + 16c
+                tmem_st16(s_tmem + c * 16, hi);
+                if constexpr (PMODE == kPResidual) tmem_st16(s_tmem + BN / 2 + c * 16, lo);
             }
-            l += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
+            float s0, s1;
+            unpack_f32x2(add_f32x2(sum2[0], sum2[1]), s0, s1);
+            l += s0 + s1;
             tmem_wait_st();
             tc_fence_before();
-            mbar_arrive(bar(BAR_P_FULL + t));
+            mbar_arrive(bar(BAR_P_FULL + 2 * t + (j & 1)));
         }
         // ---- epilogue: O / l -> global ----
-        if (ok && nblk[t] > 0) {
-            if (!mbar_wait(bar(BAR_O_FULL + t), 0)) {
+        if (ok && my_nblk > 0) {
+            if (!mbar_wait(bar(BAR_O_DONE + 2 * t + ((my_nblk - 1) & 1)), ((my_nblk - 1) >> 1) & 1)) {
                 report_timeout(p.status);
             } else {
                 tc_fence_after();
@@ -436,7 +487,7 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                         fence_async_smem();
                         named_bar_sync(1 + t, 128);
                         if ((warp & 3) == 0 && lane == 0) {
-                            tma_store_4d(&tm_o, stage, pass * (f32_out ? 32 : 64), m0[t], head[t], b);
+                            tma_store_4d(&tm_o, stage, pass * (f32_out ? 32 : 64), my_m0, my_head, b);
                             tma_store_commit();
                             tma_store_wait_read();  // the staging tile may be overwritten after this
                         }
@@ -451,103 +502,108 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         if (warp == 8 && tc::elect_one()) {
             // =============================== TMA producer ===============================
             uint32_t n_q = 0;
+#pragma unroll
             for (int t = 0; t < 2; ++t) n_q += nblk[t] > 0;
-            mbar_arrive_expect_tx(bar(BAR_Q_FULL), n_q * kLoadBytes);
+            mbar_arrive_expect_tx(bar(BAR_Q_FULL), n_q * kLoadQ);
+#pragma unroll
             for (int t = 0; t < 2; ++t) {
                 if (nblk[t] == 0) continue;
                 const uint32_t dst = base + kSmemQ + t * kTileBytes;
                 tma_load_4d(dst, &tm_q, bar(BAR_Q_FULL), 0, m0[t], head[t], b);
                 if (HD > 64) tma_load_4d(dst + kSubTileBytes, &tm_q, bar(BAR_Q_FULL), 64, m0[t], head[t], b);
             }
+            uint32_t st = 0, phase = 0;
             for (uint32_t j = 0; j < n_iter; ++j) {
-                const uint32_t st = j % kStages;
-                if (j >= kStages && !mbar_wait(bar(BAR_K_EMPTY + st), ((j / kStages) - 1) & 1)) {
+                if (j >= kStages && !mbar_wait(bar(BAR_K_EMPTY + st), phase ^ 1)) {
                     report_timeout(p.status);
                     break;
                 }
-                const uint32_t kdst = base + kSmemK + st * kTileBytes;
-                mbar_arrive_expect_tx(bar(BAR_K_FULL + st), kLoadBytes);
+                const uint32_t kdst = base + kSmemK + st * kKvBytes;
+                mbar_arrive_expect_tx(bar(BAR_K_FULL + st), kLoadKv);
                 tma_load_4d(kdst, &tm_k, bar(BAR_K_FULL + st), 0, j * BN, kvh, b);
-                if (HD > 64) tma_load_4d(kdst + kSubTileBytes, &tm_k, bar(BAR_K_FULL + st), 64, j * BN, kvh, b);
-                if (j >= kStages && !mbar_wait(bar(BAR_V_EMPTY + st), ((j / kStages) - 1) & 1)) {
+                if (HD > 64) tma_load_4d(kdst + kKvSubBytes, &tm_k, bar(BAR_K_FULL + st), 64, j * BN, kvh, b);
+                if (j >= kStages && !mbar_wait(bar(BAR_V_EMPTY + st), phase ^ 1)) {
                     report_timeout(p.status);
                     break;
                 }
-                const uint32_t vdst = base + kSmemV + st * kTileBytes;
-                mbar_arrive_expect_tx(bar(BAR_V_FULL + st), kLoadBytes);
+                const uint32_t vdst = base + kSmemV + st * kKvBytes;
+                mbar_arrive_expect_tx(bar(BAR_V_FULL + st), kLoadKv);
                 tma_load_4d(vdst, &tm_v, bar(BAR_V_FULL + st), 0, j * BN, kvh, b);
-                if (HD > 64) tma_load_4d(vdst + kSubTileBytes, &tm_v, bar(BAR_V_FULL + st), 64, j * BN, kvh, b);
+                if (HD > 64) tma_load_4d(vdst + kKvSubBytes, &tm_v, bar(BAR_V_FULL + st), 64, j * BN, kvh, b);
+                if (++st == kStages) st = 0, phase ^= 1;
             }
         } else if (warp == 9 && n_iter > 0 && tc::elect_one()) {
             // =============================== MMA issuer ===============================
             constexpr uint32_t fmt = BF16 ? 1u : 0u;
-            constexpr uint32_t idesc_qk = instr_desc(fmt, fmt, 0, BN);  // S: 128 rows x 128 keys
+            constexpr uint32_t idesc_qk = instr_desc(fmt, fmt, 0, BN);  // S: 128 rows x 64 keys
             constexpr uint32_t idesc_pv = instr_desc(fmt, fmt, 1, HD);  // O: 128 rows x head_dim
-            // S_t = Q_t K^T: 8 MMAs of K = 16 over head_dim; operands K-major, 128-byte swizzle, 8-row groups 1024 B apart
-            auto issue_qk = [&](int t, uint32_t st) {
-                const uint32_t qa = base + kSmemQ + t * kTileBytes;
-                const uint32_t ka = base + kSmemK + st * kTileBytes;
+            const uint64_t q_desc = smem_desc(base + kSmemQ, 16, 1024), k_desc = smem_desc(base + kSmemK, 16, 1024);
+            const uint64_t v_desc = smem_desc(base + kSmemV, kKvSubBytes, 1024);
+            // S_t = Q_t K^T: MMAs of K = 16 over head_dim; operands K-major, 128-byte swizzle, 8-row groups 1024 B apart
+            // (descriptors count in 16 bytes)
+            auto issue_qk = [&](int t, uint32_t j, uint32_t st) {
+                const uint64_t qa = q_desc + t * (kTileBytes / 16), ka = k_desc + st * (kKvBytes / 16);
+                const uint32_t d = tmem_s(t, j & 1);
 #pragma unroll
                 for (int kc = 0; kc < HD / 16; ++kc) {
-                    const uint32_t off = (kc >> 2) * kSubTileBytes + (kc & 3) * 32;
-                    mma_ss(tmem_s(t), smem_desc(qa + off, 16, 1024), smem_desc(ka + off, 16, 1024), idesc_qk, kc > 0);
+                    mma_ss(d, qa + (kc >> 2) * (kSubTileBytes / 16) + (kc & 3) * 2,
+                           ka + (kc >> 2) * (kKvSubBytes / 16) + (kc & 3) * 2, idesc_qk, kc > 0);
                 }
-                tc_commit(bar(BAR_S_FULL + t));
+                tc_commit(bar(BAR_S_FULL + 2 * t + (j & 1)));
             };
-            // O_t += P_t V: 8 MMAs of K = 16 keys; A = P in tensor memory (8 packed columns per MMA), B = V as an
-            // MN-major operand: 64-dim halves 16 KB apart (leading offset), 8-key groups 1024 B apart (stride offset)
-            auto issue_pv = [&](int t, uint32_t st, bool accumulate) {
-                const uint32_t va = base + kSmemV + st * kTileBytes;
+            // O_t += P_t V: MMAs of K = 16 keys; A = P in tensor memory (8 packed columns per MMA), B = V as an
+            // MN-major operand: 64-dim halves one sub-tile apart (leading offset), 8-key groups 1024 B apart (stride)
+            auto issue_pv = [&](int t, uint32_t j, uint32_t st) {
+                const uint64_t va = v_desc + st * (kKvBytes / 16);
+                const uint32_t pa = tmem_s(t, j & 1);
 #pragma unroll
-                for (int kc = 0; kc < BN / 16; ++kc) {
-                    mma_ts(tmem_o(t), tmem_s(t) + kc * 8, smem_desc(va + kc * 2048, kSubTileBytes, 1024), idesc_pv,
-                           accumulate || kc > 0);
-                }
+                for (int kc = 0; kc < BN / 16; ++kc) mma_ts(tmem_o(t), pa + kc * 8, va + kc * 128, idesc_pv, j > 0 || kc > 0);
                 if constexpr (PMODE == kPResidual) {
 #pragma unroll
-                    for (int kc = 0; kc < BN / 16; ++kc) {
-                        mma_ts(tmem_o(t), tmem_s(t) + 64 + kc * 8, smem_desc(va + kc * 2048, kSubTileBytes, 1024),
-                               idesc_pv, 1);
-                    }
+                    for (int kc = 0; kc < BN / 16; ++kc) mma_ts(tmem_o(t), pa + BN / 2 + kc * 8, va + kc * 128, idesc_pv, 1);
                 }
+                tc_commit(bar(BAR_O_DONE + 2 * t + (j & 1)));
             };
-            bool ok = mbar_wait(bar(BAR_Q_FULL), 0) && mbar_wait(bar(BAR_K_FULL + 0), 0);
-            if (!ok) report_timeout(p.status);
-            if (ok) {
+            // Scores run two blocks ahead of the products: Q K^T of block j + 2 is issued right behind P V of block j
+            // (whose probabilities lie in the buffer it overwrites; the tensor pipe works in order).
+            bool ok = mbar_wait(bar(BAR_Q_FULL), 0);
+            auto scores = [&](uint32_t j) {  // the blocks of the prologue
+                ok = ok && mbar_wait(bar(BAR_K_FULL + j), 0);
+                if (!ok) return;
                 tc_fence_after();
+#pragma unroll
                 for (int t = 0; t < 2; ++t)
-                    if (nblk[t] > 0) issue_qk(t, 0);
-                tc_commit(bar(BAR_K_EMPTY + 0));
-            }
+                    if (j < nblk[t]) issue_qk(t, j, j);
+                tc_commit(bar(BAR_K_EMPTY + j));
+            };
+            scores(0);
+            if (n_iter > 1) scores(1);
+            uint32_t st = 0, phase = 0, st2 = 2 % kStages, phase2 = 2 / kStages;  // stage and phase of block j, j + 2
             for (uint32_t j = 0; j < n_iter && ok; ++j) {
-                const uint32_t st = j % kStages;
-                if (!mbar_wait(bar(BAR_V_FULL + st), (j / kStages) & 1)) { report_timeout(p.status); ok = false; break; }
-                bool k_next_ready = false;
-                for (int t = 0; t < 2 && ok; ++t) {
-                    if (j >= nblk[t]) continue;
-                    if (!mbar_wait(bar(BAR_P_FULL + t), j & 1)) { report_timeout(p.status); ok = false; break; }
+                if (!mbar_wait(bar(BAR_V_FULL + st), phase)) { ok = false; break; }
+                bool k_ready = false;
+#pragma unroll
+                for (int t = 0; t < 2; ++t) {
+                    if (!ok || j >= nblk[t]) continue;
+                    if (!mbar_wait(bar(BAR_P_FULL + 2 * t + (j & 1)), (j >> 1) & 1)) { ok = false; break; }
                     tc_fence_after();
-                    issue_pv(t, st, j > 0);
-                    if (j + 1 < nblk[t]) {
-                        const uint32_t st1 = (j + 1) % kStages;
-                        if (!k_next_ready) {
-                            if (!mbar_wait(bar(BAR_K_FULL + st1), ((j + 1) / kStages) & 1)) {
-                                report_timeout(p.status);
-                                ok = false;
-                                break;
-                            }
+                    issue_pv(t, j, st);
+                    if (j + 2 < nblk[t]) {
+                        if (!k_ready) {
+                            if (!mbar_wait(bar(BAR_K_FULL + st2), phase2)) { ok = false; break; }
                             tc_fence_after();
-                            k_next_ready = true;
+                            k_ready = true;
                         }
-                        issue_qk(t, st1);
-                    } else {
-                        tc_commit(bar(BAR_O_FULL + t));
+                        issue_qk(t, j + 2, st2);
                     }
                 }
                 if (!ok) break;
                 tc_commit(bar(BAR_V_EMPTY + st));
-                if (j + 1 < n_iter) tc_commit(bar(BAR_K_EMPTY + (j + 1) % kStages));
+                if (j + 2 < n_iter) tc_commit(bar(BAR_K_EMPTY + st2));
+                if (++st == kStages) st = 0, phase ^= 1;
+                if (++st2 == kStages) st2 = 0, phase2 ^= 1;
             }
+            if (!ok) report_timeout(p.status);
         }
     }
 
@@ -561,16 +617,16 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 }
 
 // ------------------------------------------------------------------------------------------------ host
-// [B][S][heads][head_dim] tensor viewed as (dim, row, head, batch); box = 128 bytes of 128 rows, 128-byte swizzle.
+// [B][S][heads][head_dim] tensor viewed as (dim, row, head, batch); box = 128 bytes of box_rows rows, 128-byte swizzle.
 int make_map(CUtensorMap* map, const void* ptr, int32_t dtype, uint32_t batch, uint32_t seq, uint32_t heads,
-             uint32_t HD) {
+             uint32_t HD, uint32_t box_rows) {
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return ATTN_ERR_CUDA;
     const cuuint64_t esz = dtype == ATTN_DTYPE_F32 ? 4 : 2;
     const cuuint64_t dims[4] = {HD, seq, heads, batch};
     const cuuint64_t strides[3] = {static_cast<cuuint64_t>(heads) * HD * esz, static_cast<cuuint64_t>(HD) * esz,
                                    static_cast<cuuint64_t>(seq) * heads * HD * esz};
-    const cuuint32_t box[4] = {static_cast<cuuint32_t>(128 / esz), BM, 1, 1};  // 128-byte rows
+    const cuuint32_t box[4] = {static_cast<cuuint32_t>(128 / esz), box_rows, 1, 1};  // 128-byte rows
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     const CUtensorMapDataType dt = dtype == ATTN_DTYPE_F32    ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
                                    : dtype == ATTN_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
@@ -606,10 +662,10 @@ extern "C" int attn_prefill_causal(const AttnPrefillArgs* a, void* stream_v) {
     if (dev.cc_major != 10) return ATTN_ERR_DEVICE;
 
     CUtensorMap tm_q, tm_k, tm_v, tm_o;
-    if ((rc = make_map(&tm_o, a->o, a->o_dtype, a->batch, a->seq_len, a->n_heads, a->head_dim)) != ATTN_OK) return rc;
-    if ((rc = make_map(&tm_q, a->q, a->dtype, a->batch, a->seq_len, a->n_heads, a->head_dim)) != ATTN_OK) return rc;
-    if ((rc = make_map(&tm_k, a->k, a->dtype, a->batch, a->seq_len, a->n_kv_heads, a->head_dim)) != ATTN_OK) return rc;
-    if ((rc = make_map(&tm_v, a->v, a->dtype, a->batch, a->seq_len, a->n_kv_heads, a->head_dim)) != ATTN_OK) return rc;
+    if ((rc = make_map(&tm_o, a->o, a->o_dtype, a->batch, a->seq_len, a->n_heads, a->head_dim, BM)) != ATTN_OK) return rc;
+    if ((rc = make_map(&tm_q, a->q, a->dtype, a->batch, a->seq_len, a->n_heads, a->head_dim, BM)) != ATTN_OK) return rc;
+    if ((rc = make_map(&tm_k, a->k, a->dtype, a->batch, a->seq_len, a->n_kv_heads, a->head_dim, BN)) != ATTN_OK) return rc;
+    if ((rc = make_map(&tm_v, a->v, a->dtype, a->batch, a->seq_len, a->n_kv_heads, a->head_dim, BN)) != ATTN_OK) return rc;
 
     PrefillParams p{};
     p.o = a->o;
