@@ -9,8 +9,11 @@
 // Layouts (dense, head_dim = 128 or 64, 16-bit elements): Q, O [B][S][H][D]; K, V [B][S][Hkv][D] — the engine's
 // cache layout [row][kv_head][head_dim] per sequence.
 //
-// One CTA = two 128-row query tiles that share one K/V stream (two query heads of the same kv head at the
-// same rows when the GQA group is even, else two consecutive row tiles of one head), 12 warps:
+// Work item = two 128-row query tiles that share one K/V stream (two query heads of the same kv head at the
+// same rows when the GQA group is even, else two consecutive row tiles of one head). Persistent, one CTA per SM: the
+// items are dealt longest causal span first, back and forth over the CTAs (4 x 2048 rows: 1024 items, no CTA more than
+// one item above another), and an item's loads and first score products run while the previous item's result is
+// written: 196 -> 181 us (758 TFLOP/s causal). 12 warps:
 //   warps 0-3   softmax of tile 0: thread r owns query row r (tensor-memory lane r), no shuffles needed
 //   warps 4-7   softmax of tile 1
 //   warp  8     TMA producer: Q tiles once, then K and V tiles (64 keys x 128 dims, 128-byte swizzle)
@@ -23,7 +26,7 @@
 // score buffers the softmax of block j+1 never waits for the products of block j: with one buffer of 128 keys a tile's
 // softmax (~ 2 000 clocks) and its 24 MMAs (1 536) took turns. An m128n64k16 MMA takes 48 clocks (its shared-memory
 // reads), so 128 keys cost 3 584 tensor clocks for both tiles instead of 3 072, which still is less than the turns.
-// 4 x 2048 rows, 32/8 heads of 128, bf16: 220 -> 196 us (701 TFLOP/s causal).
+// 4 x 2048 rows, 32/8 heads of 128, bf16: 220 -> 196 us before the CTAs were persistent.
 // P overwrites S in place as packed 16-bit pairs in columns [0,32). Two ways to hand P to the tensor cores (template
 // PMODE):
 //   kPResidual  P in the input type plus its rounding residual in columns [32,64) and a second PV MMA: ~2^-17,
@@ -38,6 +41,8 @@
 // Every wait is bounded; on expiry the role records ATTN_STATUS_WAIT_TIMEOUT, stops, and the CTA still
 // runs its common exit (final barrier, tensor-memory release).
 #include <cuda.h>
+
+#include <algorithm>
 
 #include "attn_internal.cuh"
 #include "ptx_sm100.cuh"
@@ -67,6 +72,8 @@ struct PrefillParams {
     int32_t in_dtype;  // ATTN_DTYPE_F16 | ATTN_DTYPE_BF16
     uint32_t batch, seq, n_heads, n_kv_heads, group;
     uint32_t m_tiles;     // ceil(seq / 128)
+    uint32_t heads_x;     // head pairs (or heads) per row-tile step
+    uint32_t items;       // work items of two tiles
     uint32_t pair_heads;  // 1: tiles are heads (2*hp, 2*hp+1) at the same rows; 0: rows (2*mp, 2*mp+1) of one head
     float scale_log2;
     uint32_t* status;
@@ -80,7 +87,8 @@ enum : int { kPResidual = 0, kPInput = 1 };
 // ---- barriers (8 bytes each) inside shared memory ----
 enum {
     BAR_Q_FULL = 0,
-    BAR_K_FULL = 1,                   // [kStages]
+    BAR_Q_EMPTY = 1,
+    BAR_K_FULL = 2,                   // [kStages]
     BAR_V_FULL = BAR_K_FULL + kStages,
     BAR_K_EMPTY = BAR_V_FULL + kStages,
     BAR_V_EMPTY = BAR_K_EMPTY + kStages,
@@ -249,6 +257,10 @@ __device__ __forceinline__ void report_timeout(uint32_t* status) {
     if (status) atomicOr(status, ATTN_STATUS_WAIT_TIMEOUT);
 }
 
+struct Item {
+    uint32_t b, head[2], m0[2], nblk[2], n_iter;  // n_iter = key blocks of the longer tile
+};
+
 template <bool BF16, int PMODE, int HDIM>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -268,35 +280,36 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     constexpr int HD = HDIM;
     constexpr uint32_t kLoadQ = (HD / 64) * kSubTileBytes, kLoadKv = (HD / 64) * kKvSubBytes;  // bytes of a tile actually loaded
 
-    // ---- which two tiles does this CTA own ----
-    // The row-tile index is the slowest-varying grid dimension and counts down, so every CTA with the longest
-    // causal span is dispatched before any shorter one and the kernel's tail is made of one-block CTAs.
-    const uint32_t b = blockIdx.y;
-    uint32_t head[2], m0[2];
-    if (p.pair_heads) {
-        const uint32_t mt = p.m_tiles - 1 - blockIdx.z;
-        head[0] = 2 * blockIdx.x;
-        head[1] = 2 * blockIdx.x + 1;
-        m0[0] = m0[1] = mt * BM;
-    } else {
-        const uint32_t pairs = (p.m_tiles + 1) / 2;
-        const uint32_t mp = pairs - 1 - blockIdx.z;
-        head[0] = head[1] = blockIdx.x;
-        m0[0] = (2 * mp) * BM;
-        m0[1] = (2 * mp + 1) * BM;
-    }
-    const uint32_t kvh = head[0] / p.group;
+    // ---- work items: two tiles each, dealt longest causal span first, back and forth over the CTAs ----
     const uint32_t nblk_total = (p.seq + BN - 1) / BN;
-    uint32_t nblk[2];
+    auto item_of = [&](uint32_t round, Item& w) {
+        const uint32_t pos = (round & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
+        const uint32_t idx = round * gridDim.x + pos;
+        if (idx >= p.items) return false;
+        const uint32_t per_span = p.heads_x * p.batch;
+        const uint32_t z = idx / per_span, rest = idx - z * per_span;
+        w.b = rest / p.heads_x;
+        const uint32_t x = rest - w.b * p.heads_x;
+        if (p.pair_heads) {
+            w.head[0] = 2 * x;
+            w.head[1] = 2 * x + 1;
+            w.m0[0] = w.m0[1] = (p.m_tiles - 1 - z) * BM;
+        } else {
+            const uint32_t mp = (p.m_tiles + 1) / 2 - 1 - z;
+            w.head[0] = w.head[1] = x;
+            w.m0[0] = 2 * mp * BM;
+            w.m0[1] = w.m0[0] + BM;
+        }
 #pragma unroll
-    for (int t = 0; t < 2; ++t) {
-        nblk[t] = m0[t] < p.seq ? min(nblk_total, (m0[t] + BM) / BN) : 0u;
-    }
-    const uint32_t n_iter = max(nblk[0], nblk[1]);
+        for (int t = 0; t < 2; ++t) w.nblk[t] = w.m0[t] < p.seq ? min(nblk_total, (w.m0[t] + BM) / BN) : 0u;
+        w.n_iter = max(w.nblk[0], w.nblk[1]);
+        return true;
+    };
 
     // ---- set-up: barriers, tensor memory ----
     if (tid == 0) {
         mbar_init(bar(BAR_Q_FULL), 1);
+        mbar_init(bar(BAR_Q_EMPTY), 1);
         for (int s = 0; s < kStages; ++s) {
             mbar_init(bar(BAR_K_FULL + s), 1);
             mbar_init(bar(BAR_V_FULL + s), 1);
@@ -330,14 +343,18 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         const int t = warp >> 2;                       // tile
         const int r = ((warp & 3) << 5) | lane;        // row inside the tile = tensor-memory lane
         const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) << 5) << 16;
-        const uint32_t my_m0 = t ? m0[1] : m0[0], my_head = t ? head[1] : head[0], my_nblk = t ? nblk[1] : nblk[0];
+        bool ok = true;
+        uint32_t g0 = 0;  // key blocks of this tile before the current item: buffer and barrier phases run on over the items
+        Item w;
+        for (uint32_t round = 0; ok && item_of(round, w); ++round) {
+        const uint32_t my_m0 = t ? w.m0[1] : w.m0[0], my_head = t ? w.head[1] : w.head[0], my_nblk = t ? w.nblk[1] : w.nblk[0];
         const uint32_t q_row = my_m0 + r;              // row index inside the sequence
         float m_used = -INFINITY;                      // maximum the stored probabilities are relative to (log2 units)
         float l = 0.f;
-        bool ok = true;
         for (uint32_t j = 0; j < my_nblk && ok; ++j) {
-            const uint32_t s_tmem = tmem_s(t, j & 1) + lane_addr;
-            if (!mbar_wait(bar(BAR_S_FULL + 2 * t + (j & 1)), (j >> 1) & 1)) { report_timeout(p.status); ok = false; break; }
+            const uint32_t g = g0 + j, buf = g & 1, par = (g >> 1) & 1;
+            const uint32_t s_tmem = tmem_s(t, buf) + lane_addr;
+            if (!mbar_wait(bar(BAR_S_FULL + 2 * t + buf), par)) { report_timeout(p.status); ok = false; break; }
             tc_fence_after();
             float s[BN];
 #pragma unroll
@@ -346,7 +363,7 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             }
             tmem_wait_ld();
 #ifdef ATTN_TRACE
-            if (p.debug && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == gridDim.z - 1 && t == 0 && j < 2) {
+            if (p.debug && w.b == 0 && my_head == 0 && my_m0 == 0 && t == 0 && j < 2) {
 #pragma unroll
                 for (int c = 0; c < BN; ++c) p.debug[r * 128 + j * BN + c] = s[c];
             }
@@ -380,9 +397,9 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             // Products of earlier blocks: the scores of block j were issued behind PV(j-2), so that one is over (waiting
             // for every phase in turn keeps the parities unambiguous); PV(j-1) may still be running and is
             // waited for only when O has to be rescaled.
-            if (j >= 2 && !mbar_wait(bar(BAR_O_DONE + 2 * t + (j & 1)), ((j - 2) >> 1) & 1)) { report_timeout(p.status); ok = false; break; }
+            if (g >= 2 && !mbar_wait(bar(BAR_O_DONE + 2 * t + buf), par ^ 1)) { report_timeout(p.status); ok = false; break; }
             if (j > 0 && __any_sync(0xffffffffu, factor != 1.f)) {
-                if (!mbar_wait(bar(BAR_O_DONE + 2 * t + ((j - 1) & 1)), ((j - 1) >> 1) & 1)) { report_timeout(p.status); ok = false; break; }
+                if (!mbar_wait(bar(BAR_O_DONE + 2 * t + (buf ^ 1)), ((g - 1) >> 1) & 1)) { report_timeout(p.status); ok = false; break; }
                 tc_fence_after();
 #pragma unroll
                 for (int c = 0; c < HD / 32; ++c) {
@@ -432,12 +449,14 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             l += s0 + s1;
             tmem_wait_st();
             tc_fence_before();
-            mbar_arrive(bar(BAR_P_FULL + 2 * t + (j & 1)));
+            mbar_arrive(bar(BAR_P_FULL + 2 * t + buf));
         }
+        g0 += my_nblk;
         // ---- epilogue: O / l -> global ----
         if (ok && my_nblk > 0) {
-            if (!mbar_wait(bar(BAR_O_DONE + 2 * t + ((my_nblk - 1) & 1)), ((my_nblk - 1) >> 1) & 1)) {
+            if (!mbar_wait(bar(BAR_O_DONE + 2 * t + ((g0 - 1) & 1)), ((g0 - 1) >> 1) & 1)) {
                 report_timeout(p.status);
+                ok = false;
             } else {
                 tc_fence_after();
                 const float inv = l > 0.f ? 1.f / l : 0.f;
@@ -487,52 +506,52 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                         fence_async_smem();
                         named_bar_sync(1 + t, 128);
                         if ((warp & 3) == 0 && lane == 0) {
-                            tma_store_4d(&tm_o, stage, pass * (f32_out ? 32 : 64), my_m0, my_head, b);
+                            tma_store_4d(&tm_o, stage, pass * (f32_out ? 32 : 64), my_m0, my_head, w.b);
                             tma_store_commit();
                             tma_store_wait_read();  // the staging tile may be overwritten after this
                         }
                         named_bar_sync(1 + t, 128);
                     }
                 }
-                if ((warp & 3) == 0 && lane == 0) tma_store_wait_all();
             }
         }
+        }
+        if ((warp & 3) == 0 && lane == 0) tma_store_wait_all();
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
         if (warp == 8 && tc::elect_one()) {
             // =============================== TMA producer ===============================
-            uint32_t n_q = 0;
+            uint32_t st = 0, phase = 0, it = 0;
+            bool ok = true;
+            Item w;
+            for (uint32_t round = 0; ok && item_of(round, w); ++round) {
+                // the query tiles are overwritten once every score product of the previous item has read them
+                if (round > 0 && !mbar_wait(bar(BAR_Q_EMPTY), (round - 1) & 1)) { ok = false; break; }
+                const uint32_t kvh = w.head[0] / p.group;
+                mbar_arrive_expect_tx(bar(BAR_Q_FULL), ((w.nblk[0] > 0) + (w.nblk[1] > 0)) * kLoadQ);
 #pragma unroll
-            for (int t = 0; t < 2; ++t) n_q += nblk[t] > 0;
-            mbar_arrive_expect_tx(bar(BAR_Q_FULL), n_q * kLoadQ);
-#pragma unroll
-            for (int t = 0; t < 2; ++t) {
-                if (nblk[t] == 0) continue;
-                const uint32_t dst = base + kSmemQ + t * kTileBytes;
-                tma_load_4d(dst, &tm_q, bar(BAR_Q_FULL), 0, m0[t], head[t], b);
-                if (HD > 64) tma_load_4d(dst + kSubTileBytes, &tm_q, bar(BAR_Q_FULL), 64, m0[t], head[t], b);
-            }
-            uint32_t st = 0, phase = 0;
-            for (uint32_t j = 0; j < n_iter; ++j) {
-                if (j >= kStages && !mbar_wait(bar(BAR_K_EMPTY + st), phase ^ 1)) {
-                    report_timeout(p.status);
-                    break;
+                for (int t = 0; t < 2; ++t) {
+                    if (w.nblk[t] == 0) continue;
+                    const uint32_t dst = base + kSmemQ + t * kTileBytes;
+                    tma_load_4d(dst, &tm_q, bar(BAR_Q_FULL), 0, w.m0[t], w.head[t], w.b);
+                    if (HD > 64) tma_load_4d(dst + kSubTileBytes, &tm_q, bar(BAR_Q_FULL), 64, w.m0[t], w.head[t], w.b);
                 }
-                const uint32_t kdst = base + kSmemK + st * kKvBytes;
-                mbar_arrive_expect_tx(bar(BAR_K_FULL + st), kLoadKv);
-                tma_load_4d(kdst, &tm_k, bar(BAR_K_FULL + st), 0, j * BN, kvh, b);
-                if (HD > 64) tma_load_4d(kdst + kKvSubBytes, &tm_k, bar(BAR_K_FULL + st), 64, j * BN, kvh, b);
-                if (j >= kStages && !mbar_wait(bar(BAR_V_EMPTY + st), phase ^ 1)) {
-                    report_timeout(p.status);
-                    break;
+                for (uint32_t j = 0; j < w.n_iter; ++j, ++it) {
+                    if (it >= kStages && !mbar_wait(bar(BAR_K_EMPTY + st), phase ^ 1)) { ok = false; break; }
+                    const uint32_t kdst = base + kSmemK + st * kKvBytes;
+                    mbar_arrive_expect_tx(bar(BAR_K_FULL + st), kLoadKv);
+                    tma_load_4d(kdst, &tm_k, bar(BAR_K_FULL + st), 0, j * BN, kvh, w.b);
+                    if (HD > 64) tma_load_4d(kdst + kKvSubBytes, &tm_k, bar(BAR_K_FULL + st), 64, j * BN, kvh, w.b);
+                    if (it >= kStages && !mbar_wait(bar(BAR_V_EMPTY + st), phase ^ 1)) { ok = false; break; }
+                    const uint32_t vdst = base + kSmemV + st * kKvBytes;
+                    mbar_arrive_expect_tx(bar(BAR_V_FULL + st), kLoadKv);
+                    tma_load_4d(vdst, &tm_v, bar(BAR_V_FULL + st), 0, j * BN, kvh, w.b);
+                    if (HD > 64) tma_load_4d(vdst + kKvSubBytes, &tm_v, bar(BAR_V_FULL + st), 64, j * BN, kvh, w.b);
+                    if (++st == kStages) st = 0, phase ^= 1;
                 }
-                const uint32_t vdst = base + kSmemV + st * kKvBytes;
-                mbar_arrive_expect_tx(bar(BAR_V_FULL + st), kLoadKv);
-                tma_load_4d(vdst, &tm_v, bar(BAR_V_FULL + st), 0, j * BN, kvh, b);
-                if (HD > 64) tma_load_4d(vdst + kKvSubBytes, &tm_v, bar(BAR_V_FULL + st), 64, j * BN, kvh, b);
-                if (++st == kStages) st = 0, phase ^= 1;
             }
-        } else if (warp == 9 && n_iter > 0 && tc::elect_one()) {
+            if (!ok) report_timeout(p.status);
+        } else if (warp == 9 && tc::elect_one()) {
             // =============================== MMA issuer ===============================
             constexpr uint32_t fmt = BF16 ? 1u : 0u;
             constexpr uint32_t idesc_qk = instr_desc(fmt, fmt, 0, BN);  // S: 128 rows x 64 keys
@@ -541,67 +560,86 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             const uint64_t v_desc = smem_desc(base + kSmemV, kKvSubBytes, 1024);
             // S_t = Q_t K^T: MMAs of K = 16 over head_dim; operands K-major, 128-byte swizzle, 8-row groups 1024 B apart
             // (descriptors count in 16 bytes)
+            uint32_t g0[2] = {0, 0};  // key blocks of each tile before the current item
             auto issue_qk = [&](int t, uint32_t j, uint32_t st) {
+                const uint32_t buf = (g0[t] + j) & 1;
                 const uint64_t qa = q_desc + t * (kTileBytes / 16), ka = k_desc + st * (kKvBytes / 16);
-                const uint32_t d = tmem_s(t, j & 1);
+                const uint32_t d = tmem_s(t, buf);
 #pragma unroll
                 for (int kc = 0; kc < HD / 16; ++kc) {
                     mma_ss(d, qa + (kc >> 2) * (kSubTileBytes / 16) + (kc & 3) * 2,
                            ka + (kc >> 2) * (kKvSubBytes / 16) + (kc & 3) * 2, idesc_qk, kc > 0);
                 }
-                tc_commit(bar(BAR_S_FULL + 2 * t + (j & 1)));
+                tc_commit(bar(BAR_S_FULL + 2 * t + buf));
             };
             // O_t += P_t V: MMAs of K = 16 keys; A = P in tensor memory (8 packed columns per MMA), B = V as an
             // MN-major operand: 64-dim halves one sub-tile apart (leading offset), 8-key groups 1024 B apart (stride)
             auto issue_pv = [&](int t, uint32_t j, uint32_t st) {
+                const uint32_t buf = (g0[t] + j) & 1;
                 const uint64_t va = v_desc + st * (kKvBytes / 16);
-                const uint32_t pa = tmem_s(t, j & 1);
+                const uint32_t pa = tmem_s(t, buf);
 #pragma unroll
                 for (int kc = 0; kc < BN / 16; ++kc) mma_ts(tmem_o(t), pa + kc * 8, va + kc * 128, idesc_pv, j > 0 || kc > 0);
                 if constexpr (PMODE == kPResidual) {
 #pragma unroll
                     for (int kc = 0; kc < BN / 16; ++kc) mma_ts(tmem_o(t), pa + BN / 2 + kc * 8, va + kc * 128, idesc_pv, 1);
                 }
-                tc_commit(bar(BAR_O_DONE + 2 * t + (j & 1)));
+                tc_commit(bar(BAR_O_DONE + 2 * t + buf));
             };
             // Scores run two blocks ahead of the products: Q K^T of block j + 2 is issued right behind P V of block j
             // (whose probabilities lie in the buffer it overwrites; the tensor pipe works in order).
-            bool ok = mbar_wait(bar(BAR_Q_FULL), 0);
-            auto scores = [&](uint32_t j) {  // the blocks of the prologue
-                ok = ok && mbar_wait(bar(BAR_K_FULL + j), 0);
-                if (!ok) return;
-                tc_fence_after();
-#pragma unroll
-                for (int t = 0; t < 2; ++t)
-                    if (j < nblk[t]) issue_qk(t, j, j);
-                tc_commit(bar(BAR_K_EMPTY + j));
-            };
-            scores(0);
-            if (n_iter > 1) scores(1);
-            uint32_t st = 0, phase = 0, st2 = 2 % kStages, phase2 = 2 / kStages;  // stage and phase of block j, j + 2
-            for (uint32_t j = 0; j < n_iter && ok; ++j) {
-                if (!mbar_wait(bar(BAR_V_FULL + st), phase)) { ok = false; break; }
-                bool k_ready = false;
-#pragma unroll
-                for (int t = 0; t < 2; ++t) {
-                    if (!ok || j >= nblk[t]) continue;
-                    if (!mbar_wait(bar(BAR_P_FULL + 2 * t + (j & 1)), (j >> 1) & 1)) { ok = false; break; }
+            // An item's first two score products are issued behind the previous item's last product, while the softmax
+            // warps still write that item's result.
+            bool ok = true;
+            uint32_t st = 0, phase = 0, kst = 0, kphase = 0;  // ring position of the next V block, of the next K block
+            Item w;
+            for (uint32_t round = 0; ok && item_of(round, w); ++round) {
+                ok = mbar_wait(bar(BAR_Q_FULL), round & 1);
+                auto next_k = [&]() {
+                    if (++kst == kStages) kst = 0, kphase ^= 1;
+                };
+                for (uint32_t j = 0; j < 2 && j < w.n_iter && ok; ++j) {
+                    ok = mbar_wait(bar(BAR_K_FULL + kst), kphase);
+                    if (!ok) break;
                     tc_fence_after();
-                    issue_pv(t, j, st);
-                    if (j + 2 < nblk[t]) {
-                        if (!k_ready) {
-                            if (!mbar_wait(bar(BAR_K_FULL + st2), phase2)) { ok = false; break; }
-                            tc_fence_after();
-                            k_ready = true;
+#pragma unroll
+                    for (int t = 0; t < 2; ++t)
+                        if (j < w.nblk[t]) issue_qk(t, j, kst);
+                    tc_commit(bar(BAR_K_EMPTY + kst));
+                    if (j + 1 == w.n_iter) tc_commit(bar(BAR_Q_EMPTY));
+                    next_k();
+                }
+                for (uint32_t j = 0; j < w.n_iter && ok; ++j) {
+                    if (!mbar_wait(bar(BAR_V_FULL + st), phase)) { ok = false; break; }
+                    const bool more = j + 2 < w.n_iter;
+                    bool k_ready = false;
+#pragma unroll
+                    for (int t = 0; t < 2; ++t) {
+                        if (!ok || j >= w.nblk[t]) continue;
+                        const uint32_t g = g0[t] + j;
+                        if (!mbar_wait(bar(BAR_P_FULL + 2 * t + (g & 1)), (g >> 1) & 1)) { ok = false; break; }
+                        tc_fence_after();
+                        issue_pv(t, j, st);
+                        if (j + 2 < w.nblk[t]) {
+                            if (!k_ready) {
+                                if (!mbar_wait(bar(BAR_K_FULL + kst), kphase)) { ok = false; break; }
+                                tc_fence_after();
+                                k_ready = true;
+                            }
+                            issue_qk(t, j + 2, kst);
                         }
-                        issue_qk(t, j + 2, st2);
+                    }
+                    if (!ok) break;
+                    tc_commit(bar(BAR_V_EMPTY + st));
+                    if (++st == kStages) st = 0, phase ^= 1;
+                    if (more) {
+                        tc_commit(bar(BAR_K_EMPTY + kst));
+                        if (j + 3 == w.n_iter) tc_commit(bar(BAR_Q_EMPTY));
+                        next_k();
                     }
                 }
-                if (!ok) break;
-                tc_commit(bar(BAR_V_EMPTY + st));
-                if (j + 2 < n_iter) tc_commit(bar(BAR_K_EMPTY + st2));
-                if (++st == kStages) st = 0, phase ^= 1;
-                if (++st2 == kStages) st2 = 0, phase2 ^= 1;
+                g0[0] += w.nblk[0];
+                g0[1] += w.nblk[1];
             }
             if (!ok) report_timeout(p.status);
         }
@@ -686,10 +724,12 @@ extern "C" int attn_prefill_causal(const AttnPrefillArgs* a, void* stream_v) {
 #endif
     if (a->p_mode > 1) return ATTN_ERR_INVALID_ARG;
 
-    dim3 grid;
-    if (p.pair_heads) grid = dim3(a->n_heads / 2, a->batch, p.m_tiles);
-    else grid = dim3(a->n_heads, a->batch, (p.m_tiles + 1) / 2);
-    if (grid.y > 65535u || grid.z > 65535u) return ATTN_ERR_UNSUPPORTED;
+    p.heads_x = p.pair_heads ? a->n_heads / 2 : a->n_heads;
+    const uint64_t spans = p.pair_heads ? p.m_tiles : (p.m_tiles + 1) / 2;
+    const uint64_t items = spans * p.heads_x * a->batch;
+    if (items > 0x7fffffffull || a->batch > 65535u || spans > 65535u) return ATTN_ERR_UNSUPPORTED;
+    p.items = static_cast<uint32_t>(items);
+    const dim3 grid(static_cast<uint32_t>(std::min<uint64_t>(items, static_cast<uint64_t>(dev.sm_count))));
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     auto launch = [&](auto kernel) -> int {
         B200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemAlloc)));
