@@ -236,8 +236,8 @@ class Llama:
 
     def prefill(self, prompts, exact: bool = True) -> None:
         """The prompt phase for all sequences at once instead of one token per step: the tokens of every prompt are
-        packed into one matrix of rows; per layer one tensor-core GEMM per projection (attn_gemm_f16; Q8_0 weights are
-        expanded per matrix into an fp16 value / residual pair first), the rotary kernel that also fills the KV caches,
+        packed into one matrix of rows; per layer one tensor-core GEMM per projection (attn_gemm_pair, the SwiGLU product as
+        its epilogue; Q8_0 weights are expanded per matrix into an fp16 value / residual pair first), the rotary kernel that also fills the KV caches,
         causal attention per sequence (attn_prefill_causal straight over that sequence's cache rows), and the
         row-wise norm / SwiGLU steps. Per token this is the engine's forward pass (src/model/block.cpp:105-223) with
         InferenceMode::Prefill for all but the last token of a prompt (src/model/model.cpp:74-76); the last tokens go
@@ -269,28 +269,24 @@ class Llama:
         qkv = e(T, q_dim + 2 * kv_dim)
         q16 = e(T, H, D, dtype=f16)
         att = e(T, H, D)
-        gate_up = e(T, 2 * c.hidden_dim)
         if q8:  # room for the largest matrix of a layer as an fp16 pair
             biggest = max(w[k].shape[1] * (w[k].shape[2] // 34 * 32) for k in ("wqkv", "wo", "w13", "w2"))
             w_hi, w_lo = e(biggest, dtype=f16), e(biggest, dtype=f16)
 
-        def project(a_pair, wmat, out, accumulate):
+        def project(a_pair, wmat, out, **kw):
+            w_pair = (wmat, None)
             if q8:
                 rows, n = wmat.shape[0], wmat.shape[1] // 34 * 32
-                pair = (w_hi[:rows * n].view(rows, n), w_lo[:rows * n].view(rows, n))
-                A.dequant_q8_0_pair(wmat, out=pair)
-                A.gemm_f16(a_pair[0], a_pair[1] if exact else None, pair[0], out=out, accumulate=accumulate,
-                           status=self.status)
-                if exact:
-                    A.gemm_f16(a_pair[0], None, pair[1], out=out, accumulate=True, status=self.status)
-            else:
-                A.gemm_f16(a_pair[0], a_pair[1] if exact else None, wmat, out=out, accumulate=accumulate,
-                           status=self.status)
+                w_pair = (w_hi[:rows * n].view(rows, n), w_lo[:rows * n].view(rows, n))
+                A.dequant_q8_0_pair(wmat, out=w_pair)
+            if not exact:
+                a_pair, w_pair = (a_pair[0], None), (w_pair[0], None)
+            A.gemm_pair(a_pair, w_pair, out=out, status=self.status, **kw)
 
         self._embed(w["embed"], tokens, out=x, status=self.status)
         for l in range(c.n_layers):
             A.rmsnorm_pair(x, w["rms_att"][l], c.norm_eps, out=pair_d)
-            project(pair_d, w["wqkv"][l], qkv, False)
+            project(pair_d, w["wqkv"][l], qkv)
             A.rope_prompt(qkv, q16, self.k_cache[l], self.v_cache[l], token_seq, token_pos, n_heads=H,
                           theta=c.rope_theta, rotary_dim=c.rotary_dim, qkv_clip=c.qkv_clip)
             for b in range(B):
@@ -298,11 +294,10 @@ class Llama:
                 A.attn_prefill_causal(q16[s0:s1].unsqueeze(0), self.k_cache[l, b, :n].unsqueeze(0),
                                       self.v_cache[l, b, :n].unsqueeze(0), out=att[s0:s1].unsqueeze(0), status=self.status)
             A.split_pair(att.view(T, q_dim), out=pair_q)
-            project(pair_q, w["wo"][l], x, True)                          # x += Wo att
+            project(pair_q, w["wo"][l], x, accumulate=True)               # x += Wo att
             A.rmsnorm_pair(x, w["rms_ffn"][l], c.norm_eps, out=pair_d)
-            project(pair_d, w["w13"][l], gate_up, False)                  # gate | up
-            A.swiglu_pair(gate_up, out=pair_h)
-            project(pair_h, w["w2"][l], x, True)                          # x += W2 (silu(gate) * up)
+            project(pair_d, w["w13"][l], pair_h, swiglu=True)             # silu(gate) * up
+            project(pair_h, w["w2"][l], x, accumulate=True)               # x += W2 (silu(gate) * up)
         # the last token of every prompt: final norm, classifier, greedy pick (the decode step's own kernels)
         A.gather_rows(x, last_rows, out=self.x)
         A.rmsnorm(self.x, w["rms_final"], c.norm_eps, out=self.xb)
