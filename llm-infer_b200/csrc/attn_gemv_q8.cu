@@ -152,38 +152,46 @@ __global__ void __launch_bounds__(NW * 32, 1) gemv_q8_0_kernel(const __grid_cons
     }
     __syncwarp();
 
-    auto issue = [&](uint32_t item) {
-        const uint32_t ci = item % cpw, q = item / cpw;
-        const uint32_t part = q % parts, q2 = q / parts;
-        const uint32_t gi = q2 % my_groups, slice = slice_begin + q2 / my_groups;
-        const uint32_t rg = cta + gi * ctas;
-        const uint32_t chunk = slice * slice_chunks + warp + ci * kWarps;
-        const uint32_t stage = item % p.stages;
+    // The next item to load, kept as counters: working its coordinates out of the item number costs six integer
+    // divisions, ~ 500 clocks in front of every refill (14336 x 4096 at batch 8: 16.4 -> 14.4 us without them, 128256 x 4096 105.8 -> 91.9).
+    uint32_t n_ci = 0, n_part = 0, n_gi = 0, n_slice = slice_begin, n_stage = 0;
+    auto issue = [&]() {
+        const uint32_t rg = cta + n_gi * ctas;
+        const uint32_t chunk = n_slice * slice_chunks + warp + n_ci * kWarps;
+        const uint32_t stage = n_stage;
         const uint32_t bar = bar0 + 8 * stage;
         if (lane == 0) {
             mbar_arrive_expect_tx(bar, kStageBytes);
             if constexpr (TILED) {
                 const uint8_t* src =
-                    p.w_tiles + (static_cast<size_t>(part * groups + rg) * p.row_chunks + chunk) * kStageBytes;
+                    p.w_tiles + (static_cast<size_t>(n_part * groups + rg) * p.row_chunks + chunk) * kStageBytes;
                 bulk_g2s(ring0 + stage * kStageBytes, src, kStageBytes, bar, policy);
-                return;
+            } else {
+                // x in 32-bit elements (a multiple of 4: 16-byte rule), y = first row of the group (rows past the
+                // tensor read as zeros)
+                tma_load_rows(ring0 + stage * kStageBytes, &tm_w, bar, static_cast<int>(chunk * (kSegBytes / 4)),
+                              static_cast<int>(n_part * p.d + rg * kRows), policy);
             }
-            // x in 32-bit elements (a multiple of 4: 16-byte rule), y = first row of the group (rows past the
-            // tensor read as zeros)
-            tma_load_rows(ring0 + stage * kStageBytes, &tm_w, bar, static_cast<int>(chunk * (kSegBytes / 4)),
-                          static_cast<int>(part * p.d + rg * kRows), policy);
+        }
+        if (++n_stage == p.stages) n_stage = 0;
+        if (++n_ci == cpw) {
+            n_ci = 0;
+            if (++n_part == parts) {
+                n_part = 0;
+                if (++n_gi == my_groups) n_gi = 0, ++n_slice;
+            }
         }
     };
     // The weights do not depend on the activations (no kernel writes them): start streaming them at once, let the next
     // kernel of the stream be scheduled, and only then wait for the previous kernel, whose output x (and out) are.
-    for (uint32_t i = 0; i < p.stages && i < total; ++i) issue(i);
+    for (uint32_t i = 0; i < p.stages && i < total; ++i) issue();
     grid_dep_launch_dependents();
     grid_dep_wait();
 
     const bool has_col = g < p.batch;  // lanes of the other columns feed zeros
     const uint32_t* my_x = s_x + (has_col ? g : 0) * p.x_col_pitch + t * 4;
     bool timed_out = false;
-    uint32_t item = 0, round = 0;
+    uint32_t item = 0, round = 0, stage = 0, phase = 0;
     uint4 xr[REGX ? CB : 1][2];
     if constexpr (REGX) {
         // B fragments of this warp's chunk (blocks [warp*CB, +CB) of sequence g), straight from global memory: the
@@ -244,8 +252,7 @@ __global__ void __launch_bounds__(NW * 32, 1) gemv_q8_0_kernel(const __grid_cons
             for (uint32_t part = 0; part < parts; ++part) {
                 float tot[4] = {0.f, 0.f, 0.f, 0.f};
                 for (uint32_t ci = 0; ci < cpw; ++ci, ++item) {
-                    const uint32_t stage = item % p.stages;
-                    if (!mbar_wait(bar0 + 8 * stage, (item / p.stages) & 1)) timed_out = true;
+                    if (!mbar_wait(bar0 + 8 * stage, phase)) timed_out = true;
                     const uint32_t seg_lo = ring0 + stage * kStageBytes + g * kSegPitch;
                     const uint32_t seg_hi = seg_lo + 8 * kSegPitch;
                     const uint32_t* xb = my_x + (warp + ci * kWarps) * kChunkBlocks * 32;
@@ -297,8 +304,9 @@ __global__ void __launch_bounds__(NW * 32, 1) gemv_q8_0_kernel(const __grid_cons
                     if (item + p.stages < total) {
                         // order this warp's reads of the stage before the asynchronous writes that refill it
                         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                        issue(item + p.stages);
+                        issue();
                     }
+                    if (++stage == p.stages) stage = 0, phase ^= 1;
                 }
                 store_partial<NW>(red, part, warp, g, t, tot);
             }
