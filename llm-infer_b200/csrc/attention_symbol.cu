@@ -88,7 +88,7 @@ attention(float* o, const float* q, const half* k, const half* v, uint32_t kv_to
     p.v = reinterpret_cast<const uint16_t*>(v);
     p.part_o = c.part_o;
     p.part_lse = c.part_lse;
-    p.seg_prefix = nullptr;
+    p.seg_ctas = nullptr;
     p.kv_len = nullptr;
     p.kv_len_uniform = kv_tokens;
     p.batch = 1;

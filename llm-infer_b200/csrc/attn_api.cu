@@ -123,7 +123,7 @@ int decode_impl(const AttnDecodeArgs* a, void* stream_v, const Exchange* xchg) {
     p.v = static_cast<const uint16_t*>(a->v);
     p.part_o = ws;
     p.part_lse = ws + plan.part_o_floats;
-    p.seg_prefix = reinterpret_cast<uint32_t*>(ws + plan.part_o_floats + plan.part_lse_floats);
+    p.seg_ctas = reinterpret_cast<uint32_t*>(ws + plan.part_o_floats + plan.part_lse_floats);
     p.kv_len = a->kv_len;
     p.kv_len_uniform = a->kv_len_uniform;
     p.batch = a->batch;
@@ -164,7 +164,7 @@ int decode_impl(const AttnDecodeArgs* a, void* stream_v, const Exchange* xchg) {
         p.o = a->o;
         p.lse = a->lse;
         p.o_dtype = a->o_dtype;
-        p.counters = p.seg_prefix + plan.prefix_words;
+        p.counters = p.seg_ctas + plan.prefix_words;
         B200_CUDA_TRY(cudaMemsetAsync(p.counters, 0, static_cast<size_t>(plan.nseg) * 4, stream));
     }
     rc = launch_decode_split(p, a->head_dim, plan.hpc, qsplit, kv_bf16, fused, plan.grid, plan.smem_bytes, stream);
@@ -194,7 +194,7 @@ int decode_impl(const AttnDecodeArgs* a, void* stream_v, const Exchange* xchg) {
 #endif
     m.max_ctas = p.max_ctas;
     m.min_tiles_per_cta = p.min_tiles_per_cta;
-    m.seg_prefix = p.seg_prefix;
+    m.seg_ctas = p.seg_ctas;
     m.status = a->status;
 #ifdef ATTN_TRACE
     m.trace = g_trace_merge;

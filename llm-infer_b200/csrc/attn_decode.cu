@@ -93,7 +93,7 @@ int make_decode_plan(uint32_t batch, uint32_t n_heads, uint32_t n_kv_heads, uint
     const size_t rows = slots * pl.ts * pl.hpc * pl.group;
     pl.part_o_floats = rows * head_dim;
     pl.part_lse_floats = (rows + 3) & ~static_cast<size_t>(3);
-    // partials, LSEs, tile prefix [nseg+1], arrival counters [nseg] of the single-launch mode, four words of which
+    // partials, LSEs, the segments' CTAs [nseg], arrival counters [nseg] of the single-launch mode, four words of which
     // the first is the status word of the engine's kernel symbol
     pl.prefix_words = (static_cast<size_t>(pl.nseg) + 1 + 3) & ~3ull;
     pl.workspace_bytes =

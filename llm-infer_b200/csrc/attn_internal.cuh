@@ -31,7 +31,7 @@ struct DecodeParams {
     const uint16_t* v;
     float* part_o;         // [slots*TS][HPC][G][D]
     float* part_lse;       // [slots*TS][HPC][G]
-    uint32_t* seg_prefix;  // [nseg+1] tile prefix written by CTA 0 when lengths are ragged
+    uint32_t* seg_ctas;    // [nseg] segment_ctas() words, written by CTA 0 for the merge pass when lengths are ragged
     const uint32_t* kv_len;
     uint32_t kv_len_uniform;
     uint32_t batch;
@@ -93,7 +93,7 @@ struct MergeParams {
     uint32_t kv_capacity;
     uint32_t max_ctas;
     uint32_t min_tiles_per_cta;
-    const uint32_t* seg_prefix;
+    const uint32_t* seg_ctas;  // ragged lengths: written by the split pass
 #ifdef ATTN_BOUNDS_CHECK
     uint64_t part_rows;
 #endif
@@ -140,11 +140,18 @@ __host__ __device__ inline uint32_t clamped_len(uint32_t len, uint32_t capacity)
     return (capacity && len > capacity) ? capacity : len;
 }
 
+// a / b for products that rarely leave 32 bits: the 64-bit division routine costs several hundred clocks, in front of
+// the first load of a launch.
+__host__ __device__ inline uint64_t div_mostly_32(uint64_t a, uint64_t b) {
+    if (((a | b) >> 32) == 0) return static_cast<uint32_t>(a) / static_cast<uint32_t>(b);
+    return a / b;
+}
+
 // Number of CTAs that actually take tiles, identical in the split and merge passes.
 __host__ __device__ inline uint32_t active_ctas(uint32_t grid, uint32_t max_ctas, uint32_t min_tiles, uint64_t nt) {
     uint64_t a = grid;
     if (max_ctas && max_ctas < a) a = max_ctas;
-    uint64_t by_work = nt / (min_tiles ? min_tiles : 1);
+    uint64_t by_work = div_mostly_32(nt, min_tiles ? min_tiles : 1);
     if (by_work < 1) by_work = 1;
     if (by_work < a) a = by_work;
     return static_cast<uint32_t>(a);
@@ -152,7 +159,15 @@ __host__ __device__ inline uint32_t active_ctas(uint32_t grid, uint32_t max_ctas
 
 // CTA that owns flat tile t when nt tiles are dealt to a CTAs as [c*nt/a, (c+1)*nt/a).
 __host__ __device__ inline uint32_t cta_of_tile(uint64_t t, uint64_t nt, uint64_t a) {
-    return static_cast<uint32_t>(((t + 1) * a - 1) / nt);
+    return static_cast<uint32_t>(div_mostly_32((t + 1) * a - 1, nt));
+}
+
+// Which CTAs of the split pass share a segment with the flat tiles [tile0, tile_end), in one word: the first of them
+// in the low half, their number in the high half (0: the segment is empty). A grid has at most one CTA per SM.
+__host__ __device__ inline uint32_t segment_ctas(uint64_t tile0, uint64_t tile_end, uint64_t nt, uint32_t active) {
+    if (tile_end == tile0) return 0u;
+    const uint32_t first = cta_of_tile(tile0, nt, active);
+    return first | (cta_of_tile(tile_end - 1, nt, active) - first + 1) << 16;
 }
 
 // ----------------------------------------------------------------------------

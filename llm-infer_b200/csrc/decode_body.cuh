@@ -239,9 +239,12 @@ __device__ __forceinline__ void decode_split_body(const DecodeParams& p, unsigne
         }
         __syncthreads();
         nt = prefix[nseg];
-        if (blockIdx.x == 0 && p.seg_prefix) {
+        if (blockIdx.x == 0 && p.seg_ctas) {
+            // for the merge pass, worked out here once: that pass would otherwise spend three loads and three 64-bit
+            // divisions per row between this grid's end and its first partial
+            const uint32_t a = active_ctas(gridDim.x, p.max_ctas, p.min_tiles_per_cta, nt);
             if (early) grid_dep_wait();  // the previous kernel may still be reading the old table
-            for (uint32_t s = tid; s <= nseg; s += kThreads) p.seg_prefix[s] = prefix[s];
+            for (uint32_t s = tid; s < nseg; s += kThreads) p.seg_ctas[s] = segment_ctas(prefix[s], prefix[s + 1], nt, a);
         }
     } else {
         tiles_uniform = (clamped_len(p.kv_len_uniform, p.kv_capacity) + TT - 1) / TT;
@@ -254,8 +257,8 @@ __device__ __forceinline__ void decode_split_body(const DecodeParams& p, unsigne
     const uint32_t active = active_ctas(gridDim.x, p.max_ctas, p.min_tiles_per_cta, nt);
     const uint32_t cta = blockIdx.x;
     if (cta >= active) return;
-    const uint32_t t_begin = static_cast<uint32_t>(static_cast<uint64_t>(cta) * nt / active);
-    const uint32_t t_end = static_cast<uint32_t>(static_cast<uint64_t>(cta + 1) * nt / active);
+    const uint32_t t_begin = static_cast<uint32_t>(div_mostly_32(cta * nt, active));
+    const uint32_t t_end = static_cast<uint32_t>(div_mostly_32((cta + 1) * nt, active));
     const uint32_t n_my = t_end - t_begin;
     if (n_my == 0) return;
 

@@ -86,7 +86,7 @@ __device__ __forceinline__ void warp_merge_row(const float* po, const float* pl,
 
 // Where the partials of output row `row` are: n of them, partial i at po + i * o_stride (head_dim floats) with its
 // LSE at pl + i * l_stride. For the decode split pass these are the consecutive slots the pass wrote for the row's
-// segment; with ragged lengths the tile prefix is read, which that pass writes: the wait for it happens in here.
+// segment; with ragged lengths the segment's CTAs are read, which that pass writes: the wait for it happens in here.
 __device__ __forceinline__ void locate_partials(const MergeParams& p, uint32_t row, const float*& po, const float*& pl,
                                                 uint64_t& o_stride, uint64_t& l_stride, uint32_t& n) {
     if (p.split_grid) {
@@ -98,28 +98,23 @@ __device__ __forceinline__ void locate_partials(const MergeParams& p, uint32_t r
         const uint32_t hh = kvh - hg * p.hpc;
         const uint32_t nseg = p.batch * p.head_groups;
         const uint32_t seg = b * p.head_groups + hg;
-        uint64_t nt, tile0, tile_end;
+        uint32_t ctas;
         if (p.kv_len) {
-            grid_dep_wait();  // the tile prefix is written by the split pass
-            nt = p.seg_prefix[nseg];
-            tile0 = p.seg_prefix[seg];
-            tile_end = p.seg_prefix[seg + 1];
+            grid_dep_wait();  // written by the split pass
+            ctas = __ldcg(p.seg_ctas + seg);
         } else {
             const uint64_t tu = (clamped_len(p.kv_len_uniform, p.kv_capacity) + p.tile_rows - 1) / p.tile_rows;
-            nt = tu * nseg;
-            tile0 = tu * seg;
-            tile_end = tile0 + tu;
+            const uint64_t nt = tu * nseg;
+            ctas = nt ? segment_ctas(tu * seg, tu * (seg + 1), nt, active_ctas(p.split_grid, p.max_ctas, p.min_tiles_per_cta, nt)) : 0u;
         }
-        if (tile_end == tile0) {
+        if (ctas == 0) {
             n = 0;
             po = nullptr;
             pl = nullptr;
             o_stride = l_stride = 0;
         } else {
-            const uint32_t a = active_ctas(p.split_grid, p.max_ctas, p.min_tiles_per_cta, nt);
-            const uint32_t c_first = cta_of_tile(tile0, nt, a);
-            const uint32_t c_last = cta_of_tile(tile_end - 1, nt, a);
-            n = (c_last - c_first + 1) * p.ts;
+            const uint32_t c_first = ctas & 0xffffu;
+            n = (ctas >> 16) * p.ts;
             const uint64_t first_slot = (static_cast<uint64_t>(c_first) + seg) * p.ts;
             const uint64_t row0 = (first_slot * p.hpc + hh) * p.group + g;
             l_stride = static_cast<uint64_t>(p.hpc) * p.group;
