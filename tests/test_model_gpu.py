@@ -246,3 +246,27 @@ def test_token_id_out_of_range_is_reported_not_read(M):
     A.embed_f16(table, torch.tensor([3, 10], dtype=torch.int32, device="cuda"), out=out, status=status)
     torch.cuda.synchronize()
     assert status.item() == 2 and (out[0] == 1).all() and (out[1] == -1).all()
+
+
+@pytest.mark.parametrize("vocab", [1, 7, 9, 1000, 8192, 65537, 128256])
+def test_argmax_first_index_over_a_cluster(pkg, built_lib, vocab):
+    """One row is cut into eight: ties inside and across the pieces, -inf rows, NaN in front and elsewhere, against the
+    engine's loop (start with element 0, replace when strictly greater)."""
+    import torch
+    from llm_infer_b200 import attention as A
+    g = torch.Generator().manual_seed(vocab)
+    rows = torch.randint(-3, 4, (6, vocab), generator=g).float()  # few values: ties everywhere
+    rows[1] = float("-inf")
+    rows[2, vocab // 2] = float("nan")
+    rows[3, 0] = float("nan")
+    rows[4] = torch.randn(vocab, generator=g)
+    rows[5, vocab - 1] = float("inf")
+
+    def loop(row):
+        best, at = row[0], 0
+        for i, v in enumerate(row):
+            if v > best:
+                best, at = v, i
+        return at
+
+    assert A.argmax(rows.cuda()).cpu().tolist() == [loop(r.tolist()) for r in rows]
