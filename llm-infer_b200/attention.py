@@ -28,9 +28,20 @@ def _dtype_code(t: torch.Tensor) -> int:
         raise TypeError(f"unsupported dtype {t.dtype}") from None
 
 
-def _stream_ptr(stream) -> int:
-    s = torch.cuda.current_stream() if stream is None else stream
-    return s.cuda_stream
+def _call(entry: str, device: torch.device, stream, *args, what: str | None = None) -> None:
+    """One C-ABI call on ``device`` and its current stream (or ``stream``). The raw accessors and the device switch only
+    when another device is current keep the host's share of a small call down (a device context and a Stream
+    object per call were 3 of the ~ 15 us that a decode of 512 rows took on the host)."""
+    index = device.index
+    ptr = torch._C._cuda_getCurrentRawStream(index) if stream is None else stream.cuda_stream
+    fn = getattr(_b.load(), entry)
+    if torch._C._cuda_getDevice() == index:
+        rc = fn(*args, ptr)
+    else:
+        with torch.cuda.device(index):
+            rc = fn(*args, ptr)
+    if rc:
+        _b.check(rc, what or entry)
 
 
 def _dense(t: torch.Tensor, stream, what: str) -> torch.Tensor:
@@ -86,29 +97,25 @@ def _decode_args(q, k_cache, v_cache, kv_len, out, lse, out_dtype, scale, worksp
     if workspace is None or workspace.key != (B, H, Hkv, D, q.device.index):
         workspace = DecodeWorkspace(B, H, Hkv, D, q.device)
 
-    a = _b.AttnDecodeArgs()
-    a.o, a.q, a.k, a.v = out.data_ptr(), q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr()
-    a.lse = lse.data_ptr() if lse is not None else None
-    a.o_dtype, a.q_dtype, a.kv_dtype = _dtype_code(out), _dtype_code(q), _dtype_code(k_cache)
-    a.batch, a.n_heads, a.n_kv_heads, a.head_dim = B, H, Hkv, D
+    kv_ptr, uniform = None, T
     if kv_len is None:
-        a.kv_len, a.kv_len_uniform = None, T
+        pass
     elif isinstance(kv_len, int):
         if kv_len > T:
             raise ValueError("kv_len exceeds the cache")
-        a.kv_len, a.kv_len_uniform = None, kv_len
+        uniform = kv_len
     else:
         if kv_len.dtype not in (torch.int32, torch.uint32) or kv_len.shape != (B,) or not kv_len.is_cuda:
             raise ValueError("kv_len must be an int32 CUDA tensor of shape [B]")
-        a.kv_len, a.kv_len_uniform = kv_len.data_ptr(), 0
-    a.kv_row_stride = k_cache.stride(1)
-    a.kv_batch_stride = k_cache.stride(0) if B > 1 else max(k_cache.stride(0), 0)
-    a.scale = float(scale)
-    a.max_ctas = int(max_ctas)
-    a.workspace, a.workspace_bytes = workspace.buf.data_ptr(), workspace.nbytes
-    a.status = workspace.status.data_ptr()
-    a.kv_early = int(bool(kv_early))
-    a.kv_capacity = T  # a device-side length beyond the cache is clamped and reported (ATTN_STATUS_BAD_SHAPE)
+        kv_ptr, uniform = kv_len.data_ptr(), 0
+    batch_stride, row_stride = k_cache.stride(0), k_cache.stride(1)
+    # (one positional construction: setting 23 fields by name costs three times as much)
+    a = _b.AttnDecodeArgs(
+        out.data_ptr(), q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), lse.data_ptr() if lse is not None else None,
+        _dtype_code(out), _dtype_code(q), _dtype_code(k_cache), B, H, Hkv, D, kv_ptr, uniform, row_stride,
+        batch_stride if B > 1 else max(batch_stride, 0), float(scale), int(max_ctas), workspace.buf.data_ptr(),
+        workspace.nbytes, workspace.status.data_ptr(), int(bool(kv_early)),
+        T)  # a device-side length beyond the cache is clamped and reported (ATTN_STATUS_BAD_SHAPE)
     return a, out, workspace, q
 
 
@@ -128,8 +135,7 @@ def attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, k
     """
     a, out, _, _q = _decode_args(q, k_cache, v_cache, kv_len, out, lse, out_dtype, scale, workspace, max_ctas, stream,
                                  kv_early)
-    with torch.cuda.device(out.device):
-        _b.check(_b.load().attn_decode(C.byref(a), _stream_ptr(stream)), "attn_decode")
+    _call("attn_decode", out.device, stream, C.byref(a))
     return out
 
 
@@ -148,8 +154,7 @@ def attn_decode_sharded(q, k_shard, v_shard, kv_len_local=None, *, peer_buffers,
     s.world_size, s.rank, s.step, s.poll_limit = world_size, rank, step, poll_limit
     for r in range(world_size):
         s.peer_buffers[r] = int(peer_buffers[r])
-    with torch.cuda.device(out.device):
-        _b.check(_b.load().attn_decode_sharded(C.byref(s), _stream_ptr(stream)), "attn_decode_sharded")
+    _call("attn_decode_sharded", out.device, stream, C.byref(s))
     return out
 
 
@@ -182,7 +187,6 @@ def attn_prefill_causal(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, ou
     rounded once to the input type.
     """
     _require_cuda(q, k, v)
-    lib = _b.load()
     B, S, H, D = q.shape
     Hkv = k.shape[2]
     if k.shape != (B, S, Hkv, D) or v.shape != k.shape or not (q.dtype == k.dtype == v.dtype):
@@ -192,14 +196,9 @@ def attn_prefill_causal(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, ou
         out = torch.empty((B, S, H, D), dtype=out_dtype or q.dtype, device=q.device)
     elif out.shape != (B, S, H, D) or not out.is_contiguous():
         raise ValueError("out must be a contiguous [B, S, H, D] tensor")
-    a = _b.AttnPrefillArgs()
-    a.o, a.q, a.k, a.v = out.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr()
-    a.o_dtype, a.dtype = _dtype_code(out), _dtype_code(q)
-    a.batch, a.seq_len, a.n_heads, a.n_kv_heads, a.head_dim = B, S, H, Hkv, D
-    a.scale, a.p_mode = float(scale), int(p_mode)
-    a.status = status.data_ptr() if status is not None else None
-    with torch.cuda.device(q.device):
-        _b.check(lib.attn_prefill_causal(C.byref(a), _stream_ptr(stream)), "attn_prefill_causal")
+    a = _b.AttnPrefillArgs(out.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), _dtype_code(out), _dtype_code(q), B, S,
+                           H, Hkv, D, float(scale), int(p_mode), status.data_ptr() if status is not None else None)
+    _call("attn_prefill_causal", q.device, stream, C.byref(a))
     return out
 
 
@@ -232,8 +231,7 @@ def rope_kv_insert(q, k, v, k_cache, v_cache, pos, kv_pos, *, theta: float, rota
     a.rotary_dim, a.kv_sink, a.theta = rotary_dim, kv_sink, float(theta)
     a.q_out_dtype = _dtype_code(q_out)
     a.pos_early = int(pos_early)  # pos was written before the previous kernel of the stream was launched
-    with torch.cuda.device(q.device):
-        _b.check(_b.load().attn_rope_kv_insert(C.byref(a), _stream_ptr(stream)), "attn_rope_kv_insert")
+    _call("attn_rope_kv_insert", q.device, stream, C.byref(a))
     return q_out
 
 
@@ -339,8 +337,7 @@ def _gemv(entry: str, x, w, n: int, out, out2, out3, out_dtype, clip, accumulate
     if out3 is not None:
         a.out3, a.split2 = out3.data_ptr(), d0 + out2.shape[1]
         a.out3_batch_stride = out3.stride(0) if B > 1 else out3.shape[1]
-    with torch.cuda.device(x.device):
-        _b.check(getattr(_b.load(), entry)(C.byref(a), _stream_ptr(stream)), entry)
+    _call(entry, x.device, stream, C.byref(a))
     return out
 
 
@@ -403,9 +400,7 @@ def repack_q8_0(w: torch.Tensor, *, stream=None) -> torch.Tensor:
     lib = _b.load()
     if lib.attn_q8_0_tiled_bytes(rows, n) != out.numel():
         raise RuntimeError("tiled size mismatch")
-    with torch.cuda.device(w.device):
-        _b.check(lib.attn_repack_q8_0_tiled(out.data_ptr(), w.data_ptr(), rows, n, _stream_ptr(stream)),
-                 "attn_repack_q8_0_tiled")
+    _call("attn_repack_q8_0_tiled", w.device, stream, out.data_ptr(), w.data_ptr(), rows, n)
     return out
 
 
@@ -418,10 +413,8 @@ def embed_f16(table: torch.Tensor, tokens: torch.Tensor, *, out=None, status=Non
     B = tokens.numel()
     if out is None:
         out = torch.empty((B, dim), dtype=torch.float32, device=table.device)
-    with torch.cuda.device(table.device):
-        _b.check(_b.load().attn_embed_f16(out.data_ptr(), table.data_ptr(), tokens.data_ptr(), B, dim, vocab,
-                                          status.data_ptr() if status is not None else None, _stream_ptr(stream)),
-                 "attn_embed_f16")
+    _call("attn_embed_f16", table.device, stream, out.data_ptr(), table.data_ptr(), tokens.data_ptr(), B, dim, vocab,
+                                          status.data_ptr() if status is not None else None)
     return out
 
 
@@ -436,10 +429,8 @@ def embed_q8_0(table: torch.Tensor, tokens: torch.Tensor, *, out=None, status=No
     B = tokens.numel()
     if out is None:
         out = torch.empty((B, dim), dtype=torch.float32, device=table.device)
-    with torch.cuda.device(table.device):
-        _b.check(_b.load().attn_embed_q8_0(out.data_ptr(), table.data_ptr(), tokens.data_ptr(), B, dim, vocab,
-                                           status.data_ptr() if status is not None else None, _stream_ptr(stream)),
-                 "attn_embed_q8_0")
+    _call("attn_embed_q8_0", table.device, stream, out.data_ptr(), table.data_ptr(), tokens.data_ptr(), B, dim, vocab,
+                                           status.data_ptr() if status is not None else None)
     return out
 
 
@@ -459,10 +450,9 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float, *, out=None, part
         if partials.dtype != torch.float32 or partials.shape[1:] != (B, dim) or not partials.is_contiguous():
             raise ValueError("partials must be dense fp32 [k, B, dim]")
         n_part, stride, pptr = partials.shape[0], B * dim, partials.data_ptr()
-    fn = _b.load().attn_rmsnorm_residual_split if out.dtype == torch.int32 else _b.load().attn_rmsnorm_residual
-    with torch.cuda.device(x.device):
-        _b.check(fn(out.data_ptr(), x.data_ptr(), pptr, n_part, stride, weight.data_ptr(), B, dim, float(eps),
-                    _stream_ptr(stream)), "attn_rmsnorm")
+    entry = "attn_rmsnorm_residual_split" if out.dtype == torch.int32 else "attn_rmsnorm_residual"
+    _call(entry, x.device, stream, out.data_ptr(), x.data_ptr(), pptr, n_part, stride, weight.data_ptr(), B, dim, float(eps),
+          what="attn_rmsnorm")
     return out
 
 
@@ -472,8 +462,7 @@ def swiglu_(hb: torch.Tensor, hb2: torch.Tensor, *, stream=None) -> torch.Tensor
     if hb.dtype != torch.float32 or hb2.dtype != torch.float32 or hb.shape != hb2.shape or \
             not (hb.is_contiguous() and hb2.is_contiguous()):
         raise ValueError("hb and hb2 must be dense fp32 tensors of one shape")
-    with torch.cuda.device(hb.device):
-        _b.check(_b.load().attn_swiglu(hb.data_ptr(), hb2.data_ptr(), hb.numel(), _stream_ptr(stream)), "attn_swiglu")
+    _call("attn_swiglu", hb.device, stream, hb.data_ptr(), hb2.data_ptr(), hb.numel())
     return hb
 
 
@@ -485,8 +474,7 @@ def argmax(logits: torch.Tensor, *, out=None, stream=None) -> torch.Tensor:
         raise ValueError("logits must be dense fp32 [B, vocab]")
     if out is None:
         out = torch.empty((B,), dtype=torch.int32, device=logits.device)
-    with torch.cuda.device(logits.device):
-        _b.check(_b.load().attn_argmax(out.data_ptr(), logits.data_ptr(), B, vocab, _stream_ptr(stream)), "attn_argmax")
+    _call("attn_argmax", logits.device, stream, out.data_ptr(), logits.data_ptr(), B, vocab)
     return out
 
 
@@ -513,8 +501,7 @@ def attn_merge(part_o: torch.Tensor, part_lse: torch.Tensor, *, out=None, lse=No
     a.o_part_stride = part_o.stride(0) if n > 1 else rows * D
     a.lse_part_stride = part_lse.stride(0) if n > 1 else rows
     a.n_parts, a.rows, a.head_dim, a.o_dtype = n, rows, D, _dtype_code(out)
-    with torch.cuda.device(part_o.device):
-        _b.check(lib.attn_merge(C.byref(a), _stream_ptr(stream)), "attn_merge")
+    _call("attn_merge", part_o.device, stream, C.byref(a))
     return out
 
 
@@ -543,8 +530,7 @@ def gemm_f16(a_hi: torch.Tensor, a_lo, w: torch.Tensor, *, out: torch.Tensor, ac
     a.ldc, a.m, a.n_out, a.k = out.stride(0), m, n_out, k
     a.accumulate = int(bool(accumulate))
     a.status = status.data_ptr() if status is not None else None
-    with torch.cuda.device(out.device):
-        _b.check(_b.load().attn_gemm_f16(C.byref(a), _stream_ptr(stream)), "attn_gemm_f16")
+    _call("attn_gemm_f16", out.device, stream, C.byref(a))
     return out
 
 
@@ -577,8 +563,7 @@ def gemm_pair(a_pair, w_pair, *, out, accumulate: bool = False, swiglu: bool = F
     a.m, a.n_out, a.k = m, n_out, k
     a.accumulate, a.swiglu = int(bool(accumulate)), int(bool(swiglu))
     a.status = status.data_ptr() if status is not None else None
-    with torch.cuda.device(a_hi.device):
-        _b.check(_b.load().attn_gemm_pair(C.byref(a), _stream_ptr(stream)), "attn_gemm_pair")
+    _call("attn_gemm_pair", a_hi.device, stream, C.byref(a))
     return out
 
 
@@ -587,9 +572,8 @@ def rmsnorm_pair(x: torch.Tensor, weight: torch.Tensor, eps: float, *, out=None,
     _require_cuda(x, weight)
     rows, dim = x.shape
     hi, lo = out if out is not None else _pair_like(x)
-    with torch.cuda.device(x.device):
-        _b.check(_b.load().attn_rmsnorm_f16pair(hi.data_ptr(), lo.data_ptr(), x.data_ptr(), weight.data_ptr(), rows, dim,
-                                                float(eps), _stream_ptr(stream)), "attn_rmsnorm_f16pair")
+    _call("attn_rmsnorm_f16pair", x.device, stream, hi.data_ptr(), lo.data_ptr(), x.data_ptr(), weight.data_ptr(), rows, dim,
+                                                float(eps))
     return hi, lo
 
 
@@ -599,9 +583,7 @@ def split_pair(x: torch.Tensor, *, out=None, stream=None):
     if x.dtype != torch.float32 or not x.is_contiguous():
         raise ValueError("x must be dense fp32")
     hi, lo = out if out is not None else _pair_like(x)
-    with torch.cuda.device(x.device):
-        _b.check(_b.load().attn_split_f16pair(hi.data_ptr(), lo.data_ptr(), x.data_ptr(), x.numel(), _stream_ptr(stream)),
-                 "attn_split_f16pair")
+    _call("attn_split_f16pair", x.device, stream, hi.data_ptr(), lo.data_ptr(), x.data_ptr(), x.numel())
     return hi, lo
 
 
@@ -613,9 +595,8 @@ def swiglu_pair(gate_up: torch.Tensor, *, out=None, stream=None):
         raise ValueError("gate_up must be fp32 [rows, 2 hidden] with dense rows")
     hidden = two_h // 2
     hi, lo = out if out is not None else _pair_like(gate_up, (rows, hidden))
-    with torch.cuda.device(gate_up.device):
-        _b.check(_b.load().attn_swiglu_f16pair(hi.data_ptr(), lo.data_ptr(), gate_up.data_ptr(), rows, hidden,
-                                               gate_up.stride(0), _stream_ptr(stream)), "attn_swiglu_f16pair")
+    _call("attn_swiglu_f16pair", gate_up.device, stream, hi.data_ptr(), lo.data_ptr(), gate_up.data_ptr(), rows, hidden,
+                                               gate_up.stride(0))
     return hi, lo
 
 
@@ -629,9 +610,7 @@ def dequant_q8_0_pair(w: torch.Tensor, *, out=None, stream=None):
     if out is None:
         out = (torch.empty((rows, n), dtype=torch.float16, device=w.device), torch.empty((rows, n), dtype=torch.float16, device=w.device))
     hi, lo = out
-    with torch.cuda.device(w.device):
-        _b.check(_b.load().attn_dequant_q8_0_f16pair(hi.data_ptr(), lo.data_ptr(), w.data_ptr(), rows, n,
-                                                     _stream_ptr(stream)), "attn_dequant_q8_0_f16pair")
+    _call("attn_dequant_q8_0_f16pair", w.device, stream, hi.data_ptr(), lo.data_ptr(), w.data_ptr(), rows, n)
     return hi, lo
 
 
@@ -654,17 +633,14 @@ def rope_prompt(qkv: torch.Tensor, q_out: torch.Tensor, k_cache: torch.Tensor, v
     a.ld, a.kv_row_stride, a.kv_batch_stride = qkv.stride(0), k_cache.stride(1), k_cache.stride(0)
     a.tokens, a.n_heads, a.n_kv_heads, a.head_dim = tokens, n_heads, Hkv, D
     a.rotary_dim, a.theta, a.qkv_clip = rotary_dim, float(theta), float(qkv_clip)
-    with torch.cuda.device(qkv.device):
-        _b.check(_b.load().attn_rope_prompt(C.byref(a), _stream_ptr(stream)), "attn_rope_prompt")
+    _call("attn_rope_prompt", qkv.device, stream, C.byref(a))
     return q_out
 
 
 def gather_rows(x: torch.Tensor, rows: torch.Tensor, *, out: torch.Tensor, stream=None) -> torch.Tensor:
     """out[r] = x[rows[r]] (fp32 rows; rows int32 on the device)."""
     _require_cuda(x, rows, out)
-    with torch.cuda.device(x.device):
-        _b.check(_b.load().attn_gather_rows(out.data_ptr(), x.data_ptr(), rows.data_ptr(), rows.numel(), x.shape[1],
-                                            _stream_ptr(stream)), "attn_gather_rows")
+    _call("attn_gather_rows", x.device, stream, out.data_ptr(), x.data_ptr(), rows.data_ptr(), rows.numel(), x.shape[1])
     return out
 
 
