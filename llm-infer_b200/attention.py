@@ -236,9 +236,11 @@ def rope_kv_insert(q, k, v, k_cache, v_cache, pos, kv_pos, *, theta: float, rota
 
 
 class HostDecodeStep:
-    """One decode step of the attention block driven from host buffers, as ONE CUDA-graph launch: the token's fp32
-    q, k, v are copied from pinned host memory (one copy), ``attn_rope_kv_insert`` rotates q and k and appends k, v to
-    the resident fp16 caches, ``attn_decode`` attends over them, and the output is copied back to pinned host memory.
+    """One decode step of the attention block driven from host buffers, as ONE CUDA-graph launch:
+    ``attn_rope_kv_insert`` reads the token's fp32 q, k, v from pinned host memory, rotates q and k and appends k, v to
+    the resident fp16 caches, ``attn_decode`` attends over them, and its merge pass writes the output to pinned host
+    memory. (Dense 16-byte aligned host buffers are read and written by these kernels over PCIe, without a copy in
+    front and behind: HOSTNOTE; others are copied through device buffers.)
     The engine drives its CUDA step the same way (a captured graph per step, include/model/device.hpp:161-262).
     Calling the object replays the graph and waits for the result.
 
@@ -260,21 +262,40 @@ class HostDecodeStep:
             raise ValueError("host_in must hold q, k, v of one token per sequence (fp32) and out_host be [B, H, D]")
         dev = k_cache.device
         self.host_in, self.out_host = host_in, out_host
-        self._dev_in = torch.empty(n_q + 2 * n_kv, dtype=torch.float32, device=dev)
-        q32 = self._dev_in[:n_q].view(B, H, D)
-        k32 = self._dev_in[n_q:n_q + n_kv].view(B, Hkv, D)
-        v32 = self._dev_in[n_q + n_kv:].view(B, Hkv, D)
+        _require_cuda(k_cache, v_cache, pos, kv_pos)
+        if k_cache.dtype != torch.float16:
+            raise TypeError("the caches must be fp16")
+        direct = host_in.is_contiguous() and out_host.is_contiguous() and out_host.dtype == torch.float32 and \
+            host_in.data_ptr() % 16 == 0 and out_host.data_ptr() % 16 == 0
+        self._dev_in = None if direct else torch.empty(n_q + 2 * n_kv, dtype=torch.float32, device=dev)
         self._q_rot = torch.empty((B, H, D), dtype=torch.float16, device=dev)
         self._out = torch.empty((B, H, D), dtype=torch.float32, device=dev)
         self.workspace = workspace if workspace is not None else DecodeWorkspace(B, H, Hkv, D, dev)
+        src = host_in if direct else self._dev_in
+        rope = _b.AttnRopeInsertArgs()
+        rope.q_out, rope.q = self._q_rot.data_ptr(), src.data_ptr()
+        rope.k, rope.v = src.data_ptr() + 4 * n_q, src.data_ptr() + 4 * (n_q + n_kv)
+        rope.k_cache, rope.v_cache = k_cache.data_ptr(), v_cache.data_ptr()
+        rope.pos, rope.kv_pos = pos.data_ptr(), kv_pos.data_ptr()
+        rope.kv_row_stride = k_cache.stride(1)
+        rope.kv_batch_stride = k_cache.stride(0) if B > 1 else max(k_cache.stride(0), 0)
+        rope.batch, rope.n_heads, rope.n_kv_heads, rope.head_dim = B, H, Hkv, D
+        rope.rotary_dim, rope.theta = rotary_dim, float(theta)
+        rope.q_out_dtype = _dtype_code(self._q_rot)
+        attn, _, _, _ = _decode_args(self._q_rot, k_cache, v_cache, kv_len, self._out, None, torch.float32, 0.0,
+                                     self.workspace, 0, None, kv_early)
+        if direct:
+            attn.o = out_host.data_ptr()
+        # (the graph reads and writes these whenever it is replayed)
+        self._keep = (k_cache, v_cache, pos, kv_pos, kv_len)
 
         def launches():
-            self._dev_in.copy_(host_in, non_blocking=True)
-            rope_kv_insert(q32, k32, v32, k_cache, v_cache, pos, kv_pos, theta=theta, rotary_dim=rotary_dim,
-                           q_out=self._q_rot)
-            attn_decode(self._q_rot, k_cache, v_cache, kv_len, out=self._out, workspace=self.workspace,
-                        kv_early=kv_early)
-            out_host.copy_(self._out, non_blocking=True)
+            if not direct:
+                self._dev_in.copy_(host_in, non_blocking=True)
+            _call("attn_rope_kv_insert", dev, None, C.byref(rope))
+            _call("attn_decode", dev, None, C.byref(attn))
+            if not direct:
+                out_host.copy_(self._out, non_blocking=True)
 
         with torch.cuda.device(dev):
             side = torch.cuda.Stream(dev)

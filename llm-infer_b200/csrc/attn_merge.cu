@@ -134,13 +134,23 @@ __global__ void __launch_bounds__(kMergeThreads, 4) merge_rows_kernel(const __gr
     const float zt = z * e0 + z1 * e1;
     const float inv_z = zt > 0.f ? 1.f / zt : 0.f;
     const size_t obase = static_cast<size_t>(row) * p.head_dim + lane * VEC;
+    // whole 16-byte stores where the output allows them (it may lie in pinned host memory: fewer, larger writes)
+    const bool wide = VEC == 4 && p.o_dtype == ATTN_DTYPE_F32 && (reinterpret_cast<uintptr_t>(p.o) & 15u) == 0;
 #pragma unroll
-    for (int c = 0; c < CHUNKS; ++c)
+    for (int c = 0; c < CHUNKS; ++c) {
+        float v[VEC];
 #pragma unroll
-        for (int e = 0; e < VEC; ++e) {
-            const float v = acc[c][e] * e0 + s_acc[rl][c * 32 * VEC + lane * VEC + e] * e1;
-            store_out(p.o, p.o_dtype, obase + c * 32 * VEC + e, v * inv_z);
+        for (int e = 0; e < VEC; ++e)
+            v[e] = (acc[c][e] * e0 + s_acc[rl][c * 32 * VEC + lane * VEC + e] * e1) * inv_z;
+        if constexpr (VEC == 4) {
+            if (wide) {
+                *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.o) + obase + c * 32 * VEC) = make_float4(v[0], v[1], v[2], v[3]);
+                continue;
+            }
         }
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) store_out(p.o, p.o_dtype, obase + c * 32 * VEC + e, v[e]);
+    }
     if (p.lse && lane == 0) p.lse[row] = zt > 0.f ? mx + logf(zt) : -INFINITY;
     MTRACE(3);
 }

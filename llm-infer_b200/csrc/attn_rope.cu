@@ -67,44 +67,58 @@ __global__ void __launch_bounds__(kRopeThreads) rope_kv_insert_kernel(const __gr
         s_tab[3 * half + i] = static_cast<float>(sin(static_cast<double>(deg1)));
     }
     if (p.pos_early) grid_dep_wait();
-    __syncthreads();
 
     const uint32_t D = p.head_dim, hp = D / 2;
+    const uint32_t n_q = p.n_heads * hp, n_kv = p.n_kv_heads * hp;  // pairs
+    // The token's values are requested together, in front of the barrier and of everything that uses them: they may
+    // lie in pinned host memory, a round trip of ~ 2 us each time they are waited for.
+    constexpr int kAhead = 2;  // query pairs per thread (32 heads of 128), one k and one v pair beside them
+    const float2* q2 = reinterpret_cast<const float2*>(p.q) + static_cast<size_t>(b) * n_q;
+    const float2* k2 = reinterpret_cast<const float2*>(p.k) + static_cast<size_t>(b) * n_kv;
+    const float2* v2 = reinterpret_cast<const float2*>(p.v) + static_cast<size_t>(b) * n_kv;
+    float2 xq[kAhead], xk = make_float2(0.f, 0.f), xv = xk;
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+        const uint32_t idx = tid + u * kRopeThreads;
+        xq[u] = idx < n_q ? q2[idx] : make_float2(0.f, 0.f);
+    }
+    if (static_cast<uint32_t>(tid) < n_kv) {
+        xk = k2[tid];
+        xv = v2[tid];
+    }
+    const uint32_t kv_pos = p.kv_pos[b];
+    __syncthreads();
+
+    auto rotate = [&](float2 x, uint32_t i) {
+        if (i < half) {
+            const float c = s_tab[i], s = s_tab[half + i];
+            return make_float2(x.x * c - x.y * s, x.x * s + x.y * c);
+        }
+        return x;
+    };
     // ---- Q: [n_heads][D/2] pairs
-    for (uint32_t idx = tid; idx < p.n_heads * hp; idx += kRopeThreads) {
-        const uint32_t h = idx / hp, i = idx - h * hp;
-        const size_t off = (static_cast<size_t>(b) * p.n_heads + h) * D + 2 * i;
-        const float2 x = *reinterpret_cast<const float2*>(p.q + off);
-        float y0 = x.x, y1 = x.y;
-        if (i < half) {
-            const float c = s_tab[i], s = s_tab[half + i];
-            y0 = x.x * c - x.y * s;
-            y1 = x.x * s + x.y * c;
-        }
-        if (p.q_out_dtype == ATTN_DTYPE_F32) {
-            *reinterpret_cast<float2*>(reinterpret_cast<float*>(p.q_out) + off) = make_float2(y0, y1);
-        } else if (p.q_out_dtype == ATTN_DTYPE_F16) {
-            *reinterpret_cast<__half2*>(reinterpret_cast<__half*>(p.q_out) + off) = __floats2half2_rn(y0, y1);
-        } else {
-            *reinterpret_cast<__nv_bfloat162*>(reinterpret_cast<__nv_bfloat16*>(p.q_out) + off) = __floats2bfloat162_rn(y0, y1);
-        }
+    auto put_q = [&](uint32_t idx, float2 x) {
+        const float2 y = rotate(x, idx % hp);
+        const size_t off = static_cast<size_t>(b) * n_q + idx;
+        if (p.q_out_dtype == ATTN_DTYPE_F32) reinterpret_cast<float2*>(p.q_out)[off] = y;
+        else if (p.q_out_dtype == ATTN_DTYPE_F16) reinterpret_cast<__half2*>(p.q_out)[off] = __floats2half2_rn(y.x, y.y);
+        else reinterpret_cast<__nv_bfloat162*>(p.q_out)[off] = __floats2bfloat162_rn(y.x, y.y);
+    };
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+        const uint32_t idx = tid + u * kRopeThreads;
+        if (idx < n_q) put_q(idx, xq[u]);
     }
+    for (uint32_t idx = tid + kAhead * kRopeThreads; idx < n_q; idx += kRopeThreads) put_q(idx, q2[idx]);
     // ---- K (rotated) and V (as is) of the current token -> fp16 cache row kv_pos
-    const size_t row = static_cast<size_t>(b) * p.kv_batch_stride + static_cast<size_t>(p.kv_pos[b]) * p.kv_row_stride;
-    for (uint32_t idx = tid; idx < p.n_kv_heads * hp; idx += kRopeThreads) {
-        const uint32_t h = idx / hp, i = idx - h * hp;
-        const size_t off = (static_cast<size_t>(b) * p.n_kv_heads + h) * D + 2 * i;
-        const float2 x = *reinterpret_cast<const float2*>(p.k + off);
-        float y0 = x.x, y1 = x.y;
-        if (i < half) {
-            const float c = s_tab[i], s = s_tab[half + i];
-            y0 = x.x * c - x.y * s;
-            y1 = x.x * s + x.y * c;
-        }
-        *reinterpret_cast<__half2*>(p.k_cache + row + h * D + 2 * i) = __floats2half2_rn(y0, y1);
-        const float2 vv = *reinterpret_cast<const float2*>(p.v + off);
-        *reinterpret_cast<__half2*>(p.v_cache + row + h * D + 2 * i) = __floats2half2_rn(vv.x, vv.y);
-    }
+    const size_t row = static_cast<size_t>(b) * p.kv_batch_stride + static_cast<size_t>(kv_pos) * p.kv_row_stride;
+    auto put_kv = [&](uint32_t idx, float2 k, float2 v) {
+        const float2 y = rotate(k, idx % hp);
+        *reinterpret_cast<__half2*>(p.k_cache + row + 2 * idx) = __floats2half2_rn(y.x, y.y);
+        *reinterpret_cast<__half2*>(p.v_cache + row + 2 * idx) = __floats2half2_rn(v.x, v.y);
+    };
+    if (static_cast<uint32_t>(tid) < n_kv) put_kv(tid, xk, xv);
+    for (uint32_t idx = tid + kRopeThreads; idx < n_kv; idx += kRopeThreads) put_kv(idx, k2[idx], v2[idx]);
     // ---- attention sinks: rows [0, kv_sink) of K move one position forward, in place on fp16 storage.
     // The reference inserts the new row first and rotates afterwards; the new row never is a sink row
     // (kv_pos >= kv_sink whenever kv_sink > 0, src/model/model.cpp:65-67), so the order does not matter here.

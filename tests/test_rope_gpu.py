@@ -144,3 +144,31 @@ def test_host_decode_step_graph_matches_the_eager_calls(built_lib, pkg):
         want = A.attn_decode(q, k_ref, v_ref, kv_len).cpu()
         assert torch.equal(got, want), trial
         assert torch.equal(k_cache, k_ref) and torch.equal(v_cache, v_ref)
+
+
+# pairs of q (k) below, at and above what a thread of the rotary kernel requests ahead; every shape once with buffers
+# the kernels may address directly and once with buffers that are off a 16-byte boundary (copied on the device)
+@pytest.mark.parametrize("B,H,Hkv,D", [(1, 4, 2, 64), (3, 32, 8, 128), (2, 64, 8, 128), (2, 40, 40, 64), (17, 16, 4, 128)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_host_decode_step_reads_and_writes_host_buffers(built_lib, pkg, B, H, Hkv, D, shift):
+    import torch
+    from llm_infer_b200 import attention as A
+    g = torch.Generator().manual_seed(B * H + D)
+    T, n_q, n_kv = 70, B * H * D, B * Hkv * D
+    k_cache = torch.randn(B, T, Hkv, D, generator=g).half().cuda()
+    v_cache = torch.randn(B, T, Hkv, D, generator=g).half().cuda()
+    k_ref, v_ref = k_cache.clone(), v_cache.clone()
+    pos = torch.arange(B, dtype=torch.int32).cuda() * 3 + 20
+    host_in = torch.zeros(n_q + 2 * n_kv + shift).pin_memory()[shift:]
+    out_host = torch.zeros(n_q + shift).pin_memory()[shift:].view(B, H, D)
+    step = A.HostDecodeStep(host_in, k_cache, v_cache, pos, pos, out_host, n_heads=H, theta=10000.0, kv_len=pos + 1)
+    fresh = torch.randn(host_in.numel(), generator=g)
+    host_in.copy_(fresh)
+    got = step().clone()
+    dev = fresh.cuda()
+    q = A.rope_kv_insert(dev[:n_q].view(B, H, D), dev[n_q:n_q + n_kv].view(B, Hkv, D), dev[n_q + n_kv:].view(B, Hkv, D),
+                         k_ref, v_ref, pos, pos, theta=10000.0, q_out_dtype=torch.float16)
+    assert torch.equal(got, A.attn_decode(q, k_ref, v_ref, pos + 1).cpu())
+    assert torch.equal(k_cache, k_ref) and torch.equal(v_cache, v_ref)
+    with pytest.raises(TypeError):
+        A.HostDecodeStep(host_in, k_cache.float(), v_cache.float(), pos, pos, out_host, n_heads=H, theta=10000.0)
