@@ -650,14 +650,14 @@ def run_single(args):
         return
 
     # ---- end to end through the public API with host buffers. One decode step of the engine's attention block:
-    # the token's fp32 q, k, v arrive from pinned host memory in one copy, attn_rope_kv_insert rotates q and k and
-    # appends k, v (fp16) to the resident cache, attn_decode attends over it, and the output is copied back and the
-    # stream synchronised before the next token. The KV cache itself stays in HBM, as the engine's per-layer cache does.
+    # the token's fp32 q, k, v are read from pinned host memory by attn_rope_kv_insert, which rotates q and k and
+    # appends k, v (fp16) to the resident cache, attn_decode attends over it and writes the output to pinned memory; the
+    # stream is synchronised before the next token. The KV cache itself stays in HBM, as the engine's per-layer cache does.
     n_q, n_kv = B * H * D, B * Hkv * D
     host_in = torch.randn(n_q + 2 * n_kv, dtype=torch.float32).pin_memory()
     pos_dev = torch.full((B,), T - 1, dtype=torch.int32, device=dev)
     out_host = torch.empty((B, H, D), dtype=torch.float32).pin_memory()
-    # the public call: one captured graph per cache (copy in, rope + insert, decode, copy out), replayed and waited for
+    # the public call: one captured graph per cache (rope + insert, decode), replayed and waited for
     host_steps = [attention.HostDecodeStep(host_in, ks[j], vs[j], pos_dev, pos_dev, out_host, n_heads=H, theta=500000.0,
                                            workspace=ws) for j in range(n_sets)]
 
@@ -672,8 +672,8 @@ def run_single(args):
     d2h = out_host.numel() * 4
     e2e = {"value": alg_bytes / (e2e_ms * 1e-3) / 1e9, "unit": "GB/s", "h2d_bytes_per_step": h2d,
            "d2h_bytes_per_step": d2h, "ms_per_step": e2e_ms,
-           "what": "attention.HostDecodeStep: fp32 q, k, v of the token copied from pinned host memory (one copy), "
-                   "attn_rope_kv_insert + attn_decode through the C ABI, output copied back to pinned host memory - "
+           "what": "attention.HostDecodeStep: fp32 q, k, v of the token read from pinned host memory over PCIe by "
+                   "attn_rope_kv_insert, attn_decode through the C ABI writing its output to pinned host memory - "
                    "one CUDA-graph launch per step, the stream synchronised every step; the KV cache itself stays "
                    "resident in HBM, as the engine's per-layer cache does"}
     q_host = qs[0].cpu().pin_memory()
