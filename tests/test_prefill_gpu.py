@@ -132,3 +132,29 @@ def test_unsupported_head_dim_is_refused(built_lib, pkg):
     a.o_dtype = a.dtype = b.DTYPE_F16
     a.batch, a.seq_len, a.n_heads, a.n_kv_heads, a.head_dim = 1, 16, 4, 4, 96
     assert built_lib.attn_prefill_causal(C.byref(a), None) == -2
+
+
+# more work items than SMs, so that every CTA takes several: head pairs (even group), row-tile pairs (odd group, with an
+# odd number of row tiles: the second tile of the last pair is empty), rows that end inside a key block
+@pytest.mark.parametrize("B,S,H,Hkv,D", [(2, 700, 32, 8, 128), (4, 650, 24, 8, 128), (3, 513, 48, 16, 64), (9, 129, 17, 17, 64)])
+@pytest.mark.parametrize("dtype,out", [("f16", "f32"), ("bf16", "bf16")])
+def test_several_items_per_cta_against_float64(built_lib, pkg, B, S, H, Hkv, D, dtype, out):
+    import torch
+    from llm_infer_b200 import attention as A
+    t = {"f16": torch.float16, "bf16": torch.bfloat16, "f32": torch.float32}
+    g = torch.Generator(device="cuda").manual_seed(S + H)
+    q, k, v = (torch.randn((B, S, h, D), generator=g, device="cuda").to(t[dtype]) for h in (H, Hkv, Hkv))
+    q[:, S // 2:] *= 6.0  # sharper rows: the running maximum moves by more than the lazy rescale tolerates
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    got = A.attn_prefill_causal(q, k, v, out_dtype=t[out], status=status)
+    kk, vv = (x.double().repeat_interleave(H // Hkv, dim=2) for x in (k, v))
+    s = torch.einsum("bqhd,bkhd->bhqk", q.double(), kk) / D ** 0.5
+    score_err = D / 16 * 2.0 ** -22 * float(s.abs().max())  # the accumulator is truncated at each of D / 16 k-steps
+    s.masked_fill_(torch.ones(S, S, dtype=torch.bool, device="cuda").triu_(1), float("-inf"))
+    want = torch.einsum("bhqk,bkhd->bqhd", torch.softmax(s, dim=-1), vv)
+    # value + residual probabilities: 2^-22 (fp16) or 2^-17 (bf16) of each, exp2 and the sums a few 2^-22, an error of a
+    # score is a relative error of its probability in numerator and sum; then the result's own rounding; |v| < 6
+    tol = 6 * ((2.0 ** -19 if dtype == "f16" else 2.0 ** -15) + 2 * score_err)
+    round_out = {"f32": 0.0, "f16": 2.0 ** -11, "bf16": 2.0 ** -8}[out]
+    assert bool(((got.double() - want).abs() <= tol + round_out * want.abs()).all())
+    assert int(status.item()) == 0
