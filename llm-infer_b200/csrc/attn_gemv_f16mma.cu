@@ -27,8 +27,7 @@ namespace {
 using namespace gemv_mma;
 
 constexpr uint32_t kChunkElems = 64;  // elements of one row per chunk: 32 bytes per lane, one 128-byte line per row
-constexpr int kF16Warps = 16;
-constexpr int kF16Threads = kF16Warps * 32;
+constexpr size_t kDualSmem = 96 * 1024; // shared memory of a CTA when two share an SM
 constexpr int kUnroll = 4;            // chunks in flight per warp: 2 x 4 loads of 32 bytes per lane
 
 struct alignas(32) W8 {
@@ -44,12 +43,15 @@ __device__ __forceinline__ W8 ld_stream32(const void* p) {
     return r;
 }
 
-__global__ void __launch_bounds__(kF16Threads, 1) gemv_f16_mma_kernel(const uint16_t* __restrict__ w, uint64_t w_rows,
+// WARPS: 16, one CTA per SM, or 8, two CTAs per SM: the barrier that ends a row group lets a CTA's loads run dry, and the
+// second CTA's keep the memory busy meanwhile.
+template <int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 16 / WARPS) gemv_f16_mma_kernel(const uint16_t* __restrict__ w, uint64_t w_rows,
                                                                       uint64_t n, const __grid_constant__ Params p) {
     extern __shared__ __align__(16) uint8_t smem[];
     // layout: [red: 2 x 2 x warps x 128 floats][acc: acc_groups x 2 x 128 floats][x fragments]
     float* s_red = reinterpret_cast<float*>(smem);
-    float* s_acc = s_red + 2 * 2 * kF16Warps * 128;
+    float* s_acc = s_red + 2 * 2 * WARPS * 128;
     uint32_t* s_x = reinterpret_cast<uint32_t*>(s_acc + p.acc_groups * 2 * 128);
 
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -75,7 +77,7 @@ __global__ void __launch_bounds__(kF16Threads, 1) gemv_f16_mma_kernel(const uint
         // so nobody still reads the old fragments.
         const float* xs = p.x + static_cast<size_t>(slice) * p.slice_units * kChunkElems;
         const uint32_t per_seq = p.slice_units * 16;  // groups of four elements per sequence
-        for (uint32_t i = tid; i < p.batch * per_seq; i += kF16Threads) {
+        for (uint32_t i = tid; i < p.batch * per_seq; i += WARPS * 32) {
             const uint32_t c = i / per_seq, r = i - c * per_seq;
             const uint32_t ch = r >> 4, j = (r >> 2) & 3, tt = r & 3;
             const float4 v = *reinterpret_cast<const float4*>(xs + c * p.x_batch_stride + 64 * ch + 16 * tt + 4 * j);
@@ -86,7 +88,7 @@ __global__ void __launch_bounds__(kF16Threads, 1) gemv_f16_mma_kernel(const uint
         const size_t slice_elem0 = static_cast<size_t>(slice) * p.slice_units * kChunkElems;
         for (uint32_t gi = 0; gi < my_groups; ++gi, ++round) {
             const uint32_t rg = cta + gi * ctas;
-            float* red = s_red + (round & 1) * 2 * kF16Warps * 128;
+            float* red = s_red + (round & 1) * 2 * WARPS * 128;
             for (uint32_t part = 0; part < parts; ++part) {
                 // rows g and g + 8 of the group; a ragged last group re-reads the last row (its results are dropped)
                 uint64_t row_lo = static_cast<uint64_t>(part) * p.d + rg * kRows + g, row_hi = row_lo + 8;
@@ -95,11 +97,11 @@ __global__ void __launch_bounds__(kF16Threads, 1) gemv_f16_mma_kernel(const uint
                 const uint16_t* w_lo = w + row_lo * n + slice_elem0 + 16 * t;
                 const uint16_t* w_hi = w + row_hi * n + slice_elem0 + 16 * t;
                 float tot[4] = {0.f, 0.f, 0.f, 0.f};
-                for (uint32_t c0 = warp; c0 < p.slice_units; c0 += kF16Warps * kUnroll) {
+                for (uint32_t c0 = warp; c0 < p.slice_units; c0 += WARPS * kUnroll) {
                     W8 alo[kUnroll], ahi[kUnroll];
 #pragma unroll
                     for (int u = 0; u < kUnroll; ++u) {
-                        const uint32_t ch = c0 + u * kF16Warps;
+                        const uint32_t ch = c0 + u * WARPS;
                         if (ch < p.slice_units) {
                             alo[u] = ld_stream32(w_lo + static_cast<size_t>(ch) * kChunkElems);
                             ahi[u] = ld_stream32(w_hi + static_cast<size_t>(ch) * kChunkElems);
@@ -107,7 +109,7 @@ __global__ void __launch_bounds__(kF16Threads, 1) gemv_f16_mma_kernel(const uint
                     }
 #pragma unroll
                     for (int u = 0; u < kUnroll; ++u) {
-                        const uint32_t ch = c0 + u * kF16Warps;
+                        const uint32_t ch = c0 + u * WARPS;
                         if (ch < p.slice_units) {
                             const uint32_t* xb = my_x + ch * 64;
 #pragma unroll
@@ -121,10 +123,10 @@ __global__ void __launch_bounds__(kF16Threads, 1) gemv_f16_mma_kernel(const uint
                         }
                     }
                 }
-                store_partial<kF16Warps>(red, part, warp, g, t, tot);
+                store_partial<WARPS>(red, part, warp, g, t, tot);
             }
             __syncthreads();
-            reduce_and_store<kF16Warps>(p, red, s_acc, tid, parts, gi, rg, slice, slice_begin, slice_end);
+            reduce_and_store<WARPS>(p, red, s_acc, tid, parts, gi, rg, slice, slice_begin, slice_end);
         }
     }
 }
@@ -144,28 +146,46 @@ int b200::launch_gemv_f16_mma(const AttnGemvArgs* a, cudaStream_t stream) {
     if (rc != ATTN_OK) return rc;
     const uint32_t n_chunks = a->n / kChunkElems;
     const uint32_t groups = (a->d + kRows - 1) / kRows;
-    const uint32_t set_max = static_cast<uint32_t>(dev.sm_count) / k_split;  // CTAs per k-slice set
-    if (set_max == 0) return ATTN_ERR_UNSUPPORTED;
-    const uint32_t set_ctas = groups < set_max ? groups : set_max;
-    const uint32_t grid = set_ctas * k_split;
-    const uint32_t groups_per_cta = (groups + set_ctas - 1) / set_ctas;
     const size_t budget = static_cast<size_t>(dev.max_smem_optin);
     // staged activations: 4 bytes per element and sequence, sequences 64 bytes apart modulo 128 (bank spread)
     auto x_bytes = [&](uint32_t chunks) { return static_cast<size_t>(a->batch) * (chunks * kChunkElems * 4 + 64); };
-    auto fixed_bytes = [&](uint32_t slices) {
-        return 2 * 2 * kF16Warps * 128 * sizeof(float) + ((slices > 1 && k_split == 1) ? groups_per_cta * 2 * 128 * sizeof(float) : 0);
+    struct Plan {
+        uint32_t grid, groups_per_cta, slices;
+        size_t smem;
     };
     // The activations are staged in equal slices of the inner dimension, as few as fit in shared memory; the partial
     // sums of the CTA's row groups are carried from slice to slice (or, with k_split, go to separate sets of CTAs).
-    uint32_t slices = k_split;
-    if (k_split > 1) {
-        if (n_chunks % k_split != 0 || fixed_bytes(1) + x_bytes(n_chunks / k_split) > budget) return ATTN_ERR_UNSUPPORTED;
-    } else {
-        while (slices <= n_chunks && (n_chunks % slices != 0 || fixed_bytes(slices) + x_bytes(n_chunks / slices) > budget)) ++slices;
-        if (slices > n_chunks) return ATTN_ERR_UNSUPPORTED;
-    }
-    const uint32_t slice_chunks = n_chunks / slices;
-    const size_t smem = fixed_bytes(slices) + x_bytes(slice_chunks);
+    auto make_plan = [&](uint32_t warps, uint32_t ctas_per_sm, uint32_t max_slices, Plan* out) {
+        const uint32_t set_max = static_cast<uint32_t>(dev.sm_count) * ctas_per_sm / k_split;  // CTAs per k-slice set
+        if (set_max == 0) return false;
+        const uint32_t set_ctas = groups < set_max ? groups : set_max;
+        const uint32_t per_cta = (groups + set_ctas - 1) / set_ctas;
+        const size_t room = ctas_per_sm > 1 ? kDualSmem : budget;
+        auto bytes = [&](uint32_t slices) {
+            return 2 * 2 * warps * 128 * sizeof(float) + ((slices > 1 && k_split == 1) ? per_cta * 2 * 128 * sizeof(float) : 0) +
+                   x_bytes(n_chunks / slices);
+        };
+        uint32_t slices = k_split;
+        if (k_split > 1) {
+            if (n_chunks % k_split != 0 || bytes(k_split) > room) return false;
+        } else {
+            while (slices <= max_slices && (n_chunks % slices != 0 || bytes(slices) > room)) ++slices;
+            if (slices > max_slices) return false;
+        }
+        *out = Plan{set_ctas * k_split, per_cta, slices, bytes(slices)};
+        return true;
+    };
+    Plan plan{};
+    // Two small CTAs per SM need row groups for more than one CTA per SM and activations that fit twice in one piece.
+    // Graph replay, 16 warps -> 2 x 8 warps: 14336 x 4096 batch 2 / 4 25.1 / 25.7 -> 23.3 / 24.6 us, 4096 x 4096 batch 2
+    // 9.8 -> 8.7, 28672 x 4096 with SwiGLU batch 1 / 4 42.9 / 44.1 -> 41.8 / 44.4, 4096 x 14336 split in four
+    // batch 1 / 4 25.3 / 26.2 -> 22.3 / 23.4; with one group per SM at most, 2048 x 5632 batch 2, 7.8 -> 9.7, and at
+    // batch 6 (115 KB per CTA, which do not share an SM) 27.0 -> 31.9 for 14336 x 4096: not there.
+    const bool dual = a->batch <= 4 && k_split <= static_cast<uint32_t>(dev.sm_count) &&
+                      groups > static_cast<uint32_t>(dev.sm_count) / k_split && make_plan(8, 2, 1, &plan);
+    if (!dual && (k_split > static_cast<uint32_t>(dev.sm_count) || !make_plan(16, 1, n_chunks, &plan))) return ATTN_ERR_UNSUPPORTED;
+    const uint32_t slices = plan.slices, slice_chunks = n_chunks / slices;
+    const size_t smem = plan.smem;
 
     Params p{};
     fill_common(p, a, k_split);
@@ -173,10 +193,11 @@ int b200::launch_gemv_f16_mma(const AttnGemvArgs* a, cudaStream_t stream) {
     p.n_slices = slices;
     p.stages = 0;
     p.x_col_pitch = slice_chunks * kChunkElems + 16;
-    p.acc_groups = (slices > 1 && k_split == 1) ? groups_per_cta : 0;
+    p.acc_groups = (slices > 1 && k_split == 1) ? plan.groups_per_cta : 0;
     const uint64_t w_rows = static_cast<uint64_t>(a->d) * (a->swiglu ? 2 : 1);
-    B200_CUDA_TRY(cudaFuncSetAttribute(gemv_f16_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    B200_CUDA_TRY(launch_dependent(gemv_f16_mma_kernel, dim3(grid), dim3(kF16Threads), smem, stream,
+    auto kernel = dual ? gemv_f16_mma_kernel<8> : gemv_f16_mma_kernel<16>;
+    B200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    B200_CUDA_TRY(launch_dependent(kernel, dim3(plan.grid), dim3(dual ? 256 : 512), smem, stream,
                                    static_cast<const uint16_t*>(a->w), w_rows, static_cast<uint64_t>(a->n), p));
     g_launch_count.fetch_add(1, std::memory_order_relaxed);
     return ATTN_OK;

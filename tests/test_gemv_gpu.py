@@ -381,3 +381,26 @@ def test_prepared_activations_from_every_producer(attention, pkg):
     ow = attention.attn_decode(q, kc, vc, out=torch.empty((B, H, D), dtype=torch.int32, device="cuda"))
     assert np.array_equal(ow.cpu().numpy().view(np.uint32).reshape(B, H * D),
                           _split16_words(o32.cpu().numpy().reshape(B, H * D)))
+
+
+# row groups around one per SM (148: 2368 rows; ragged last groups), batches around the line between one CTA and two per SM,
+# inner dimensions of one step and of a remainder of steps, sliced activations beside them
+@pytest.mark.parametrize("n,d", [(64, 2368), (576, 2369), (4096, 2400), (4096, 4736), (5632, 4753)])
+@pytest.mark.parametrize("batch", [2, 4, 5])
+def test_f16_one_or_two_ctas_per_sm_against_float64(attention, n, d, batch):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(n + d + batch)
+    x = torch.randn((batch, n), generator=g, device="cuda")
+    w = (torch.randn((2 * d, n), generator=g, device="cuda") * n ** -0.5).half()
+    want = x.double() @ w.double().T
+    # value + residual activations 2^-22 of a term, fp32 sums: a few 2^-24 of the largest partial sum per addition
+    tol = (n / 16 * 2.0 ** -23 + 2.0 ** -20) * float(want.abs().max())
+    assert float((attention.gemv_f16(x, w[:d]).double() - want[:, :d]).abs().max()) <= tol
+    if d % 16 == 0:
+        gate, up = want[:, :d], want[:, d:]
+        got = attention.gemv_f16(x, w, swiglu=True).double()
+        bound = 1.1 * tol * (up.abs() + gate.abs()) + 2.0 ** -21 * (gate * up).abs() + 1e-7
+        assert bool(((got - gate / (1 + torch.exp(-gate)) * up).abs() <= bound).all())
+    if n % 256 == 0:
+        parts = attention.gemv_f16(x, w[:d], k_split=2)
+        assert float((parts.double().sum(0) - want[:, :d]).abs().max()) <= tol
