@@ -66,7 +66,9 @@ class DecodeWorkspace:
 
     def __init__(self, batch: int, n_heads: int, n_kv_heads: int, head_dim: int, device=None):
         lib = _b.load()
-        device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
+        device = torch.device("cuda" if device is None else device)
+        if device.index is None:  # "cuda" is the current device; the key names it, as a tensor's device does
+            device = torch.device(device.type, torch.cuda.current_device())
         with torch.cuda.device(device):
             nbytes = lib.attn_decode_workspace_bytes(batch, n_heads, n_kv_heads, head_dim)
         if nbytes == 0:
@@ -270,7 +272,6 @@ class HostDecodeStep:
         self._dev_in = None if direct else torch.empty(n_q + 2 * n_kv, dtype=torch.float32, device=dev)
         self._q_rot = torch.empty((B, H, D), dtype=torch.float16, device=dev)
         self._out = torch.empty((B, H, D), dtype=torch.float32, device=dev)
-        self.workspace = workspace if workspace is not None else DecodeWorkspace(B, H, Hkv, D, dev)
         src = host_in if direct else self._dev_in
         rope = _b.AttnRopeInsertArgs()
         rope.q_out, rope.q = self._q_rot.data_ptr(), src.data_ptr()
@@ -282,8 +283,9 @@ class HostDecodeStep:
         rope.batch, rope.n_heads, rope.n_kv_heads, rope.head_dim = B, H, Hkv, D
         rope.rotary_dim, rope.theta = rotary_dim, float(theta)
         rope.q_out_dtype = _dtype_code(self._q_rot)
-        attn, _, _, _ = _decode_args(self._q_rot, k_cache, v_cache, kv_len, self._out, None, torch.float32, 0.0,
-                                     self.workspace, 0, None, kv_early)
+        # (a workspace made for another shape or device is replaced; the graph uses the one that comes back)
+        attn, _, self.workspace, _ = _decode_args(self._q_rot, k_cache, v_cache, kv_len, self._out, None, torch.float32, 0.0,
+                                                  workspace, 0, None, kv_early)
         if direct:
             attn.o = out_host.data_ptr()
         # (the graph reads and writes these whenever it is replayed)

@@ -172,3 +172,31 @@ def test_host_decode_step_reads_and_writes_host_buffers(built_lib, pkg, B, H, Hk
     assert torch.equal(k_cache, k_ref) and torch.equal(v_cache, v_ref)
     with pytest.raises(TypeError):
         A.HostDecodeStep(host_in, k_cache.float(), v_cache.float(), pos, pos, out_host, n_heads=H, theta=10000.0)
+
+
+@pytest.mark.parametrize("given", ["no device index", "other batch"])
+def test_host_decode_step_with_a_workspace_of_another_key(built_lib, pkg, given):
+    """The graph's partials, segment words and status live in a workspace that the step keeps: memory handed out between
+    the replays stays as it was written, and the results are those of the eager calls."""
+    import torch
+    from llm_infer_b200 import attention as A
+    B, H, Hkv, D, T = 3, 32, 8, 128, 600
+    workspace = A.DecodeWorkspace(B, H, Hkv, D, "cuda") if given == "no device index" else A.DecodeWorkspace(B + 1, H, Hkv, D)
+    g = torch.Generator().manual_seed(8)
+    k_cache, v_cache = (torch.randn(B, T, Hkv, D, generator=g).half().cuda() for _ in range(2))
+    pos = torch.tensor([599, 40, 301], dtype=torch.int32).cuda()
+    kv_len = pos + 1
+    host_in = torch.randn(B * (H + 2 * Hkv) * D, generator=g).pin_memory()
+    out_host = torch.empty(B, H, D).pin_memory()
+    step = A.HostDecodeStep(host_in, k_cache, v_cache, pos, pos, out_host, n_heads=H, theta=10000.0, kv_len=kv_len,
+                            workspace=workspace)
+    assert (step.workspace is workspace) == (given == "no device index")
+    held = [torch.full((step.workspace.nbytes,), 7, dtype=torch.uint8, device="cuda") for _ in range(8)]
+    held += [torch.full((1,), 7, dtype=torch.int32, device="cuda") for _ in range(64)]
+    for _ in range(2):
+        host_in.copy_(torch.randn(host_in.numel(), generator=g))
+        got = step().clone()
+        q, k, v = (t.view(B, -1, D) for t in host_in.cuda().split([B * H * D, B * Hkv * D, B * Hkv * D]))
+        q = A.rope_kv_insert(q, k, v, k_cache, v_cache, pos, pos, theta=10000.0, q_out_dtype=torch.float16)
+        assert torch.equal(got, A.attn_decode(q, k_cache, v_cache, kv_len).cpu())
+    assert all(bool((t == 7).all()) for t in held) and int(step.workspace.status.item()) == 0
