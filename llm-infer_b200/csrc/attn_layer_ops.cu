@@ -174,6 +174,10 @@ argmax_kernel(uint32_t* out, const float* logits, uint32_t vocab, uint32_t batch
     grid_dep_wait();
     const uint32_t rank = blockIdx.x % kArgmaxCtas;
     for (uint32_t b = blockIdx.x / kArgmaxCtas; b < batch; b += gridDim.x / kArgmaxCtas) {
+        // Until every CTA of the cluster has arrived here, the first one's shared memory may not be written: it may not
+        // run yet (a CTA with an empty slice gets to its store at once), or still be reading the previous row's
+        // results. The wait stands in front of the store, so the scan hides it.
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
         const float* row = logits + static_cast<size_t>(b) * vocab;
         const uint32_t per = (vocab + kArgmaxCtas - 1) / kArgmaxCtas;
         const uint32_t begin = min(rank * per, vocab), end = min(begin + per, vocab);
@@ -216,6 +220,7 @@ argmax_kernel(uint32_t* out, const float* logits, uint32_t vocab, uint32_t batch
             s_idx[warp] = best_i;
         }
         __syncthreads();
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         if (warp == 0) {
             best = s_val[lane];
             best_i = s_idx[lane];
@@ -238,8 +243,6 @@ argmax_kernel(uint32_t* out, const float* logits, uint32_t vocab, uint32_t batch
             out[b] = best_i == 0xffffffffu || first != first ? 0u : best_i;
         }
         __syncwarp();
-        // (the next row's results land in the same place)
-        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
 }
 

@@ -1,6 +1,7 @@
 """The C-ABI library: builds for sm_100a without a GPU, loads, exports every
 symbol the public header declares, and rejects bad arguments before touching CUDA."""
 import ctypes as C
+import glob
 import os
 import re
 
@@ -94,3 +95,19 @@ def test_ctypes_mirrors_have_the_library_struct_sizes(built_lib, pkg):
     for index, mirror in enumerate(mirrors):
         assert built_lib.attn_abi_struct_size(index) == C.sizeof(mirror), mirror.__name__
     assert built_lib.attn_abi_struct_size(99) == 0
+
+
+def test_a_cluster_barrier_stands_before_the_first_remote_shared_memory_store():
+    """Shared memory of another CTA may be written only once that CTA is known to run, which a cluster barrier shows and
+    being scheduled together does not. Read from the sources: in every kernel with a remote store, both halves of the
+    barrier come first."""
+    stores = 0
+    for path in sorted(glob.glob(os.path.join(ROOT, "llm-infer_b200", "csrc", "*.cu"))):
+        for kernel in re.split(r"(?=__global__ )", open(path).read())[1:]:
+            at = kernel.find("st.shared::cluster")
+            if at < 0:
+                continue
+            stores += 1
+            arrive, wait = kernel.find("barrier.cluster.arrive"), kernel.find("barrier.cluster.wait")
+            assert 0 <= arrive < wait < at, f"{os.path.basename(path)}: remote store ahead of the cluster barrier"
+    assert stores == 1  # argmax

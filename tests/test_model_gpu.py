@@ -270,3 +270,16 @@ def test_argmax_first_index_over_a_cluster(pkg, built_lib, vocab):
         return at
 
     assert A.argmax(rows.cuda()).cpu().tolist() == [loop(r.tolist()) for r in rows]
+
+
+@pytest.mark.parametrize("batch,vocab", [(1, 1), (3000, 3), (5000, 9), (2500, 8193), (70000, 17)])
+def test_argmax_many_clusters_with_empty_slices(pkg, built_lib, batch, vocab):
+    """More clusters than run at once (70000: several rows per cluster), slices without an element beside slices with some:
+    CTAs of a cluster start and finish at different times."""
+    import torch
+    from llm_infer_b200 import attention as A
+    g = torch.Generator(device="cuda").manual_seed(batch)
+    rows = torch.randint(-3, 4, (batch, vocab), generator=g, device="cuda").float()
+    at = torch.arange(vocab, device="cuda").expand(batch, -1)
+    first = torch.where(rows == rows.max(dim=1, keepdim=True).values, at, vocab).min(dim=1).values
+    assert torch.equal(A.argmax(rows).long(), first)
