@@ -264,7 +264,9 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_consta
             const uint32_t row = (PAIR ? mt * 2 * GM + rank * GM : mt * GM) + quarter * 32 + lane;
             const uint32_t n0 = nt * (p.swiglu ? half_rows : p.n_tile);
             const bool live = row < p.m;
-            if (!mbar_wait(bar(G_ACC_FULL + a), (local / p.acc_bufs) & 1)) {
+            // The vote brings the warp together again (lanes past m leave a tile early, and tcgen05.ld wants the whole warp)
+            // and lets all its lanes give up or go on.
+            if (!__all_sync(0xffffffffu, mbar_wait(bar(G_ACC_FULL + a), (local / p.acc_bufs) & 1))) {
                 if (lane == 0 && p.status) atomicOr(p.status, ATTN_STATUS_WAIT_TIMEOUT);
                 break;
             }

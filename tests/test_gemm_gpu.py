@@ -105,6 +105,46 @@ def test_gemm_with_paired_weights(A, m, n_out, k, swiglu):
     assert int(status.item()) == 0
 
 
+# Several tiles per CTA (the tests above give each at most one): accumulators handed back and forth between the MMAs and the
+# epilogue, and ring and barrier phases that run on over the tiles. Tiles in all / at once, at 148 SMs: pairs of CTAs 224 and
+# 256 wide with rows and columns that end inside a tile, 4 to 7 times (one accumulator at a time with three products, else
+# two); single CTAs 224 wide, 2 to 4 times; single CTAs (three products) or pairs 256 wide, 8 to 17 times over several bands;
+# 128 and 96 wide, 3 times, two accumulators with three products.
+@pytest.mark.parametrize("m,n_out,k", [(2500, 6144, 128), (2500, 6176, 128), (100, 57408, 128), (2600, 14336, 64),
+                                       (40001, 128, 64), (40001, 96, 128)])
+@pytest.mark.parametrize("form", ["f16", "pair", "swiglu", "swiglu pair"])
+def test_gemm_several_tiles_per_cta(A, m, n_out, k, form):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(m + n_out + k)
+    swiglu, paired = "swiglu" in form, "pair" in form
+    x = torch.randn((m, k), generator=g, device="cuda")
+    w = torch.randn((n_out * (2 if swiglu else 1), k), generator=g, device="cuda") * k ** -0.5
+    split = lambda t: (t.half(), (t - t.half().float()).half())  # noqa: E731
+    (ah, al), (wh, wl) = split(x), split(w)
+    w_pair = (wh, wl if paired else None)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = tuple(torch.empty((m, n_out), dtype=torch.float16, device="cuda") for _ in range(2)) if swiglu else \
+        torch.ones((m, n_out), device="cuda")
+    if swiglu:
+        A.gemm_pair((ah, al), w_pair, out=out, swiglu=True, status=status)
+    elif paired:
+        A.gemm_pair((ah, al), w_pair, out=out, accumulate=True, status=status)
+    else:
+        A.gemm_f16(ah, al, wh, out=out, accumulate=True, status=status)
+    w64 = wh.double() + wl.double() if paired else wh.double()
+    for r in range(0, m, 4000):  # (float64 blocks of rows)
+        prod = (ah[r:r + 4000].double() + al[r:r + 4000].double()) @ w64.T
+        tol = _truncation_bound(k, 1 if paired else 2, float(prod.abs().max()))
+        if swiglu:
+            gate, up = prod[:, :n_out], prod[:, n_out:]
+            want = gate / (1 + torch.exp(-gate)) * up
+            bound = 1.1 * tol * (up.abs() + gate.abs()) + 2.0 ** -20 * want.abs() + 2.0 ** -24
+            assert bool(((out[0][r:r + 4000].double() + out[1][r:r + 4000].double() - want).abs() <= bound).all())
+        else:  # the sum with what was there rounds once more
+            assert float((out[r:r + 4000].double() - 1.0 - prod).abs().max()) <= tol + 2.0 ** -24 * (float(prod.abs().max()) + 1)
+    assert int(status.item()) == 0
+
+
 def test_gemm_rows_equal_the_engine_matmul(A, checker):
     """Each token's row of the GEMM against the engine's own per-token matmul() on the fp32 activations."""
     import torch
