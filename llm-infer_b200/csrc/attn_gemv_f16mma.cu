@@ -14,8 +14,8 @@
 // staged swizzled TMA tiles in shared memory and read them with ldmatrix; it stopped at ~ 3.8 TB/s because the TMA
 // engine delivers the 128-byte rows of a tile at ~ 0.1 row per clock and SM.) B = the activations as fp16 value +
 // fp16 residual (two MMAs per k-step, ~ 22 significant bits; |x| clamped to the fp16 range), staged once per CTA in
-// shared memory in that order; fp32 accumulation in the MMA over the whole inner dimension. The warps' partial sums of
-// a row group are added in a fixed order. Row segments, the SwiGLU epilogue over stacked gate / up rows, in-kernel
+// shared memory in that order; fp32 accumulation in the MMA, even and odd k-steps and the residual products apart. The
+// warps' partial sums of a row group are added in a fixed order. Row segments, the SwiGLU epilogue over stacked gate / up rows, in-kernel
 // slices of the inner dimension and k_split work as in the Q8_0 kernel.
 //
 // Algorithmic bytes per call = rows * n * 2 + batch * (n*4 + d*sizeof(out)).
@@ -96,7 +96,11 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS) gemv_f16_mma_kernel(co
                 row_hi = row_hi < w_rows ? row_hi : w_rows - 1;
                 const uint16_t* w_lo = w + row_lo * n + slice_elem0 + 16 * t;
                 const uint16_t* w_hi = w + row_hi * n + slice_elem0 + 16 * t;
-                float tot[4] = {0.f, 0.f, 0.f, 0.f};
+                // Three chains of MMAs instead of one: the tensor cores drop what lies below the accumulator's last bit at
+                // every addition, so the error grows with the length of a chain, and the small residual products need
+                // not be added into the large sum. (14336 x 4096, relative error of the result: one chain 6.5e-7 with 16
+                // warps and 1.24e-6 with 8, whose chains are twice as long; three 2.1e-7 and 3.5e-7, and 2 to 3 % faster.)
+                float even[4] = {0.f, 0.f, 0.f, 0.f}, odd[4] = {0.f, 0.f, 0.f, 0.f}, res[4] = {0.f, 0.f, 0.f, 0.f};
                 for (uint32_t c0 = warp; c0 < p.slice_units; c0 += WARPS * kUnroll) {
                     W8 alo[kUnroll], ahi[kUnroll];
 #pragma unroll
@@ -117,13 +121,15 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS) gemv_f16_mma_kernel(co
                                 uint4 xv = make_uint4(0, 0, 0, 0);
                                 if (has_col) xv = *reinterpret_cast<const uint4*>(xb + j * 16);
                                 // a0 = row g, a1 = row g + 8 (first element pair); a2, a3 = the second pair
-                                mma_f16(tot, alo[u].v[2 * j], ahi[u].v[2 * j], alo[u].v[2 * j + 1], ahi[u].v[2 * j + 1], xv.z, xv.w);
-                                mma_f16(tot, alo[u].v[2 * j], ahi[u].v[2 * j], alo[u].v[2 * j + 1], ahi[u].v[2 * j + 1], xv.x, xv.y);
+                                mma_f16(res, alo[u].v[2 * j], ahi[u].v[2 * j], alo[u].v[2 * j + 1], ahi[u].v[2 * j + 1], xv.z, xv.w);
+                                mma_f16(j & 1 ? odd : even, alo[u].v[2 * j], ahi[u].v[2 * j], alo[u].v[2 * j + 1], ahi[u].v[2 * j + 1], xv.x, xv.y);
                             }
                         }
                     }
                 }
-                store_partial<WARPS>(red, part, warp, g, t, tot);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) even[i] += odd[i] + res[i];
+                store_partial<WARPS>(red, part, warp, g, t, even);
             }
             __syncthreads();
             reduce_and_store<WARPS>(p, red, s_acc, tid, parts, gi, rg, slice, slice_begin, slice_end);

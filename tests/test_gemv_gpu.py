@@ -404,3 +404,29 @@ def test_f16_one_or_two_ctas_per_sm_against_float64(attention, n, d, batch):
     if n % 256 == 0:
         parts = attention.gemv_f16(x, w[:d], k_split=2)
         assert float((parts.double().sum(0) - want[:, :d]).abs().max()) <= tol
+
+
+# 8 warps, two CTAs per SM (up to four sequences) and 16 warps (more); plain, SwiGLU and split sums, one step and several per warp
+@pytest.mark.parametrize("rows,n,swiglu,k_split", [(14336, 4096, False, 1), (28672, 4096, True, 1), (11264, 2048, True, 1),
+                                                   (4096, 14336, False, 4), (4096, 5632, False, 1), (2560, 2048, False, 1)])
+@pytest.mark.parametrize("batch", [2, 4, 5, 8])
+def test_f16_error_of_the_sums(attention, rows, n, swiglu, k_split, batch):
+    """The tensor cores drop what lies below the accumulator's last bit at each addition: 2^-24 of the running sum on
+    average, which for terms of random sign is 2/3 of the final one in the mean over a chain. A warp adds half of its k-steps'
+    value products (16 elements each) into one accumulator; the few sums behind that round to nearest."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(rows + n + batch)
+    x = torch.randn((batch, n), generator=g, device="cuda")
+    w = (torch.randn((rows, n), generator=g, device="cuda") * n ** -0.5).half()
+    want = x.double() @ w.double().T
+    got = attention.gemv_f16(x, w, swiglu=swiglu, k_split=k_split).double()
+    if k_split > 1:
+        got = got.sum(0)
+    chunks = n // k_split // 64
+    # (8 warps bring the longest chains; the 4 x 5632 activations do not fit twice on an SM and 16 warps do it)
+    chain = -(-chunks // (8 if batch <= 4 else 16)) * 2
+    bound = (2 / 3 * chain + 3) * 2.0 ** -24
+    if swiglu:  # the errors of gate and up have the sign of a loss and add up
+        want = want[:, :rows // 2] / (1 + torch.exp(-want[:, :rows // 2])) * want[:, rows // 2:]
+        bound *= 2
+    assert float((got - want).norm() / want.norm()) <= bound
