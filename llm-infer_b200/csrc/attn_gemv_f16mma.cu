@@ -5,8 +5,8 @@
 // activation on the CUDA cores and reads those activations from shared memory once per weight (batch 8: 1.5 TB/s),
 // whereas here a batch of up to 8 sequences is the N dimension of one m16n8k16 MMA and costs nothing extra.
 //
-// One persistent CTA per SM, 16 warps. A CTA owns groups of 16 consecutive rows; its warps split the inner dimension
-// in chunks of 64 elements. The weights go from global memory straight into the MMA's A registers: lane (g, t) of a
+// One persistent CTA of 16 warps per SM, or two of 8 (chosen in launch_gemv_f16_mma). A CTA owns groups of 16
+// consecutive rows; its warps split the inner dimension in chunks of 64 elements. The weights go from global memory straight into the MMA's A registers: lane (g, t) of a
 // warp reads 32 contiguous bytes of row g (and of row g + 8) - the four lanes of a row cover one 128-byte line - with
 // streaming 256-bit loads, eight in flight per lane (128 KB per SM), and those sixteen values are the lane's A
 // operands of four k-steps as they are: the order of the inner dimension inside a chunk is free as long as the
@@ -183,13 +183,23 @@ int b200::launch_gemv_f16_mma(const AttnGemvArgs* a, cudaStream_t stream) {
     };
     Plan plan{};
     // Two small CTAs per SM need row groups for more than one CTA per SM and activations that fit twice in one piece.
-    // Graph replay, 16 warps -> 2 x 8 warps: 14336 x 4096 batch 2 / 4 25.1 / 25.7 -> 23.3 / 24.6 us, 4096 x 4096 batch 2
-    // 9.8 -> 8.7, 28672 x 4096 with SwiGLU batch 1 / 4 42.9 / 44.1 -> 41.8 / 44.4, 4096 x 14336 split in four
-    // batch 1 / 4 25.3 / 26.2 -> 22.3 / 23.4; with one group per SM at most, 2048 x 5632 batch 2, 7.8 -> 9.7, and at
+    // Graph replay, 16 warps -> 2 x 8 warps: 14336 x 4096 batch 2 / 4 25.1 / 25.7 -> 22.5 / 23.7 us, 4096 x 4096 batch 2
+    // 9.8 -> 8.7, 28672 x 4096 with SwiGLU batch 1 / 4 41.3 / 42.5 -> 40.4 / 42.4, 4096 x 14336 split in four
+    // batch 1 / 4 24.3 / 25.2 -> 21.8 / 23.4; with one group per SM at most, 2048 x 5632 batch 2, 7.9 -> 9.6, and at
     // batch 6 (115 KB per CTA, which do not share an SM) 27.0 -> 31.9 for 14336 x 4096: not there.
-    const bool dual = a->batch <= 4 && k_split <= static_cast<uint32_t>(dev.sm_count) &&
-                      groups > static_cast<uint32_t>(dev.sm_count) / k_split && make_plan(8, 2, 1, &plan);
-    if (!dual && (k_split > static_cast<uint32_t>(dev.sm_count) || !make_plan(16, 1, n_chunks, &plan))) return ATTN_ERR_UNSUPPORTED;
+    const uint32_t sms = static_cast<uint32_t>(dev.sm_count);
+    bool dual = a->batch <= 4 && k_split <= sms && groups > sms / k_split;
+    // A group of a SwiGLU product holds twice the work, and whole groups are dealt: where the busiest SM gets a fifth more
+    // of them from twice as many CTAs (4 rounds instead of 3, 6 instead of 5), 16 warps are faster or equal: 12288 x 4096
+    // batch 1 / 4 20.6 / 22.4 against 20.0 / 20.9 us, 12288 x 3072 18.0 / 19.0 against 16.6 / 17.3, 22016 x 4096 31.6 / 33.7
+    // against 31.6 / 32.7; 8 rounds instead of 7 are still the other way (28672 above). Not with so few chunks that 16 warps
+    // have no more than two loads of a row in flight: 11264 x 2048 12.3 against 13.5.
+    if (a->swiglu && n_chunks > 32) {
+        const uint32_t rounds = (groups + sms - 1) / sms, dual_rounds = (groups + 2 * sms - 1) / (2 * sms);
+        dual = dual && 2 * dual_rounds * 5 < rounds * 6;
+    }
+    dual = dual && make_plan(8, 2, 1, &plan);
+    if (!dual && (k_split > sms || !make_plan(16, 1, n_chunks, &plan))) return ATTN_ERR_UNSUPPORTED;
     const uint32_t slices = plan.slices, slice_chunks = n_chunks / slices;
     const size_t smem = plan.smem;
 

@@ -430,3 +430,21 @@ def test_f16_error_of_the_sums(attention, rows, n, swiglu, k_split, batch):
         want = want[:, :rows // 2] / (1 + torch.exp(-want[:, :rows // 2])) * want[:, rows // 2:]
         bound *= 2
     assert float((got - want).norm() / want.norm()) <= bound
+
+
+# around the line between the two forms for SwiGLU products at 148 SMs: 2 | 2, 3 | 4, 3 | 4, 4 | 4 rounds of row groups, 32 and 33
+# chunks of the inner dimension
+@pytest.mark.parametrize("d", [4736, 4752, 7104, 7120])
+@pytest.mark.parametrize("n", [2048, 2112])
+@pytest.mark.parametrize("batch", [1, 4])
+def test_f16_swiglu_around_the_choice_of_ctas(attention, d, n, batch):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(n + d + batch)
+    x = torch.randn((batch, n), generator=g, device="cuda")
+    w = (torch.randn((2 * d, n), generator=g, device="cuda") * n ** -0.5).half()
+    want = x.double() @ w.double().T
+    gate, up = want[:, :d], want[:, d:]
+    got = attention.gemv_f16(x, w, swiglu=True).double()
+    tol = (n / 16 * 2.0 ** -24 + 2.0 ** -20) * float(want.abs().max())  # half a bit of the largest sum per k-step
+    bound = 1.1 * tol * (up.abs() + gate.abs()) + 2.0 ** -21 * (gate * up).abs() + 1e-7
+    assert bool(((got - gate / (1 + torch.exp(-gate)) * up).abs() <= bound).all())
