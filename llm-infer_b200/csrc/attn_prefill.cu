@@ -16,7 +16,7 @@
 // written: 196 -> 181 us (758 TFLOP/s causal). 12 warps:
 //   warps 0-3   softmax of tile 0: thread r owns query row r (tensor-memory lane r), no shuffles needed
 //   warps 4-7   softmax of tile 1
-//   warp  8     TMA producer: Q tiles once, then K and V tiles (64 keys x 128 dims, 128-byte swizzle)
+//   warp  8     TMA producer: an item's Q tiles, then its K and V tiles (64 keys x 128 dims, 128-byte swizzle)
 //               through a 4-stage ring with separate barriers for K and V
 //   warp  9     one thread issues every tcgen05.mma: S_t = Q_t K^T (both operands in shared memory,
 //               accumulator in tensor memory) and O_t += P_t V (P read from tensor memory, V from shared
@@ -51,6 +51,8 @@
 
 namespace b200 {
 namespace {
+
+using namespace tc;
 
 constexpr int BM = 128;   // query rows per tile
 constexpr int BN = 64;    // keys per block
@@ -110,72 +112,7 @@ constexpr uint32_t kSmemTmemPtr = kSmemBars + BAR_COUNT * 8;
 constexpr uint32_t kSmemTotal = kSmemTmemPtr + 16;
 constexpr uint32_t kSmemAlloc = kSmemTotal + 1024;  // slack to align the base to 1024 bytes
 
-// ---- tcgen05 / TMA wrappers ----
-__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2,
-                                            int c3) {
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
-        ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-        : "memory");
-}
-// Tile store shared -> global through the TMA engine (asynchronous; rows outside the tensor are clipped).
-__device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, uint32_t src, int c0, int c1, int c2, int c3) {
-    asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
-                 ::"l"(map), "r"(src), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-                 : "memory");
-}
-__device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-// the shared-memory source of every committed store has been read
-__device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-// every committed store is complete
-__device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void named_bar_sync(int id, int threads) {
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
-}
-
-__device__ __forceinline__ void tmem_alloc(uint32_t smem_dst, uint32_t cols) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(cols) : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish() {
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-// D(tmem) (+)= A(smem) * B(smem)
-__device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(acc)
-        : "memory");
-}
-// D(tmem) (+)= A(tmem) * B(smem)
-__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(acc)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&r)[32]) {
-    uint32_t* u = reinterpret_cast<uint32_t*>(r);
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,"
-        "%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-        : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]),
-          "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15]), "=r"(u[16]),
-          "=r"(u[17]), "=r"(u[18]), "=r"(u[19]), "=r"(u[20]), "=r"(u[21]), "=r"(u[22]), "=r"(u[23]), "=r"(u[24]),
-          "=r"(u[25]), "=r"(u[26]), "=r"(u[27]), "=r"(u[28]), "=r"(u[29]), "=r"(u[30]), "=r"(u[31])
-        : "r"(taddr)
-        : "memory");
-}
+// ---- tensor-memory stores (the other wrappers are in tcgen05_sm100.cuh) ----
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&u)[32]) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,"
@@ -186,8 +123,13 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&u)[32
           "r"(u[27]), "r"(u[28]), "r"(u[29]), "r"(u[30]), "r"(u[31])
         : "memory");
 }
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&u)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+        ::"r"(taddr), "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]), "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7]), "r"(u[8]),
+          "r"(u[9]), "r"(u[10]), "r"(u[11]), "r"(u[12]), "r"(u[13]), "r"(u[14]), "r"(u[15])
+        : "memory");
+}
 
 // Packed 16-bit pair -> two floats (exact).
 template <bool BF16>
@@ -206,18 +148,6 @@ __device__ __forceinline__ float fast_exp2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
-}
-
-// Shared-memory matrix descriptor, 128-byte swizzle, descriptor version 1 (sm_100).
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-    return static_cast<uint64_t>((addr & 0x3FFFFu) >> 4) | (static_cast<uint64_t>(lbo_bytes >> 4) << 16) |
-           (static_cast<uint64_t>(sbo_bytes >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
-
-// Instruction descriptor of kind::f16: fp32 accumulate, A format a_fmt and B format b_fmt (0 = f16, 1 = bf16; always
-// given the same value here), A K-major, B K-major (b_mn = 0) or MN-major (b_mn = 1), M = 128, N = n.
-__host__ __device__ constexpr uint32_t instr_desc(uint32_t a_fmt, uint32_t b_fmt, uint32_t b_mn, uint32_t n) {
-    return (1u << 4) | (a_fmt << 7) | (b_fmt << 10) | (b_mn << 16) | ((n >> 3) << 17) | ((128u >> 4) << 24);
 }
 
 // Two fp32 operations per instruction.
@@ -245,14 +175,6 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
     asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
     return d;
 }
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&u)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-        ::"r"(taddr), "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]), "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7]), "r"(u[8]),
-          "r"(u[9]), "r"(u[10]), "r"(u[11]), "r"(u[12]), "r"(u[13]), "r"(u[14]), "r"(u[15])
-        : "memory");
-}
-
 __device__ __forceinline__ void report_timeout(uint32_t* status) {
     if (status) atomicOr(status, ATTN_STATUS_WAIT_TIMEOUT);
 }
@@ -275,7 +197,7 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     volatile uint32_t* tmem_ptr_smem = reinterpret_cast<volatile uint32_t*>(smem + kSmemTmemPtr);
 
     const int tid = threadIdx.x;
-    const int warp = tc::uniform_warp();
+    const int warp = uniform_warp();
     const int lane = tid & 31;
     constexpr int HD = HDIM;
     constexpr uint32_t kLoadQ = (HD / 64) * kSubTileBytes, kLoadKv = (HD / 64) * kKvSubBytes;  // bytes of a tile actually loaded
@@ -330,9 +252,9 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_ptr_smem)), kTmemCols);
         tmem_relinquish();
     }
-    tc_fence_before();
+    fence_before();
     __syncthreads();
-    tc_fence_after();
+    fence_after();
     const uint32_t tmem_base = *tmem_ptr_smem;
     auto tmem_s = [&](int t, uint32_t buf) { return tmem_base + static_cast<uint32_t>(t) * 128u + buf * 64u; };
     auto tmem_o = [&](int t) { return tmem_base + 256u + static_cast<uint32_t>(t) * 128u; };
@@ -355,7 +277,7 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             const uint32_t g = g0 + j, buf = g & 1, par = (g >> 1) & 1;
             const uint32_t s_tmem = tmem_s(t, buf) + lane_addr;
             if (!mbar_wait(bar(BAR_S_FULL + 2 * t + buf), par)) { report_timeout(p.status); ok = false; break; }
-            tc_fence_after();
+            fence_after();
             float s[BN];
 #pragma unroll
             for (int c = 0; c < BN / 32; ++c) {
@@ -400,7 +322,7 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             if (g >= 2 && !mbar_wait(bar(BAR_O_DONE + 2 * t + buf), par ^ 1)) { report_timeout(p.status); ok = false; break; }
             if (j > 0 && __any_sync(0xffffffffu, factor != 1.f)) {
                 if (!mbar_wait(bar(BAR_O_DONE + 2 * t + (buf ^ 1)), ((g - 1) >> 1) & 1)) { report_timeout(p.status); ok = false; break; }
-                tc_fence_after();
+                fence_after();
 #pragma unroll
                 for (int c = 0; c < HD / 32; ++c) {
                     float o[32];
@@ -448,7 +370,7 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             unpack_f32x2(add_f32x2(sum2[0], sum2[1]), s0, s1);
             l += s0 + s1;
             tmem_wait_st();
-            tc_fence_before();
+            fence_before();
             mbar_arrive(bar(BAR_P_FULL + 2 * t + buf));
         }
         g0 += my_nblk;
@@ -458,7 +380,7 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 report_timeout(p.status);
                 ok = false;
             } else {
-                tc_fence_after();
+                fence_after();
                 const float inv = l > 0.f ? 1.f / l : 0.f;
                 // The tile leaves through shared memory and the TMA engine, 128 bytes of every row per pass: each
                 // thread writes its row's 16-byte chunks XOR-swizzled by the row (the 128-byte swizzle the tensor
@@ -519,7 +441,7 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         if ((warp & 3) == 0 && lane == 0) tma_store_wait_all();
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
-        if (warp == 8 && tc::elect_one()) {
+        if (warp == 8 && elect_one()) {
             // =============================== TMA producer ===============================
             uint32_t st = 0, phase = 0, it = 0;
             bool ok = true;
@@ -551,11 +473,11 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 }
             }
             if (!ok) report_timeout(p.status);
-        } else if (warp == 9 && tc::elect_one()) {
+        } else if (warp == 9 && elect_one()) {
             // =============================== MMA issuer ===============================
             constexpr uint32_t fmt = BF16 ? 1u : 0u;
-            constexpr uint32_t idesc_qk = instr_desc(fmt, fmt, 0, BN);  // S: 128 rows x 64 keys
-            constexpr uint32_t idesc_pv = instr_desc(fmt, fmt, 1, HD);  // O: 128 rows x head_dim
+            constexpr uint32_t idesc_qk = instr_desc(fmt, fmt, 0, BM, BN);  // S: 128 rows x 64 keys
+            constexpr uint32_t idesc_pv = instr_desc(fmt, fmt, 1, BM, HD);  // O: 128 rows x head_dim
             const uint64_t q_desc = smem_desc(base + kSmemQ, 16, 1024), k_desc = smem_desc(base + kSmemK, 16, 1024);
             const uint64_t v_desc = smem_desc(base + kSmemV, kKvSubBytes, 1024);
             // S_t = Q_t K^T: MMAs of K = 16 over head_dim; operands K-major, 128-byte swizzle, 8-row groups 1024 B apart
@@ -570,7 +492,7 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                     mma_ss(d, qa + (kc >> 2) * (kSubTileBytes / 16) + (kc & 3) * 2,
                            ka + (kc >> 2) * (kKvSubBytes / 16) + (kc & 3) * 2, idesc_qk, kc > 0);
                 }
-                tc_commit(bar(BAR_S_FULL + 2 * t + buf));
+                commit(bar(BAR_S_FULL + 2 * t + buf));
             };
             // O_t += P_t V: MMAs of K = 16 keys; A = P in tensor memory (8 packed columns per MMA), B = V as an
             // MN-major operand: 64-dim halves one sub-tile apart (leading offset), 8-key groups 1024 B apart (stride)
@@ -584,7 +506,7 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 #pragma unroll
                     for (int kc = 0; kc < BN / 16; ++kc) mma_ts(tmem_o(t), pa + BN / 2 + kc * 8, va + kc * 128, idesc_pv, 1);
                 }
-                tc_commit(bar(BAR_O_DONE + 2 * t + buf));
+                commit(bar(BAR_O_DONE + 2 * t + buf));
             };
             // Scores run two blocks ahead of the products: Q K^T of block j + 2 is issued right behind P V of block j
             // (whose probabilities lie in the buffer it overwrites; the tensor pipe works in order).
@@ -601,12 +523,12 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 for (uint32_t j = 0; j < 2 && j < w.n_iter && ok; ++j) {
                     ok = mbar_wait(bar(BAR_K_FULL + kst), kphase);
                     if (!ok) break;
-                    tc_fence_after();
+                    fence_after();
 #pragma unroll
                     for (int t = 0; t < 2; ++t)
                         if (j < w.nblk[t]) issue_qk(t, j, kst);
-                    tc_commit(bar(BAR_K_EMPTY + kst));
-                    if (j + 1 == w.n_iter) tc_commit(bar(BAR_Q_EMPTY));
+                    commit(bar(BAR_K_EMPTY + kst));
+                    if (j + 1 == w.n_iter) commit(bar(BAR_Q_EMPTY));
                     next_k();
                 }
                 for (uint32_t j = 0; j < w.n_iter && ok; ++j) {
@@ -618,23 +540,23 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                         if (!ok || j >= w.nblk[t]) continue;
                         const uint32_t g = g0[t] + j;
                         if (!mbar_wait(bar(BAR_P_FULL + 2 * t + (g & 1)), (g >> 1) & 1)) { ok = false; break; }
-                        tc_fence_after();
+                        fence_after();
                         issue_pv(t, j, st);
                         if (j + 2 < w.nblk[t]) {
                             if (!k_ready) {
                                 if (!mbar_wait(bar(BAR_K_FULL + kst), kphase)) { ok = false; break; }
-                                tc_fence_after();
+                                fence_after();
                                 k_ready = true;
                             }
                             issue_qk(t, j + 2, kst);
                         }
                     }
                     if (!ok) break;
-                    tc_commit(bar(BAR_V_EMPTY + st));
+                    commit(bar(BAR_V_EMPTY + st));
                     if (++st == kStages) st = 0, phase ^= 1;
                     if (more) {
-                        tc_commit(bar(BAR_K_EMPTY + kst));
-                        if (j + 3 == w.n_iter) tc_commit(bar(BAR_Q_EMPTY));
+                        commit(bar(BAR_K_EMPTY + kst));
+                        if (j + 3 == w.n_iter) commit(bar(BAR_Q_EMPTY));
                         next_k();
                     }
                 }
@@ -646,10 +568,10 @@ prefill_causal_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     }
 
     // ---- common exit: everybody meets, then the allocating warp releases tensor memory ----
-    tc_fence_before();
+    fence_before();
     __syncthreads();
     if (warp == 8) {
-        tc_fence_after();
+        fence_after();
         tmem_dealloc(tmem_base, kTmemCols);
     }
 }
