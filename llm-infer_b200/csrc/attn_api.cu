@@ -57,11 +57,6 @@ bool valid_out_dtype(int32_t d) { return valid_dtype(d) || d == ATTN_DTYPE_SPLIT
 // extra memory parallelism. (One sequence of 4096 rows: 19.5 us with 64, 17.3 us with 32, 17.4 us with 16.)
 constexpr uint32_t kMinRowsPerCta = 32;
 
-// Largest number of partials per segment for which attn_decode runs as one launch whose last-arriving CTAs merge
-// (the form the engine's kernel symbol always uses). 0 = never: at every shape measured the two-launch chain, whose
-// merge pass is already resident when the split pass ends, was faster (17.4 against 28.8 us for one sequence of 4096 rows).
-constexpr uint32_t kFusedMaxParts = 0;
-
 #ifdef ATTN_TRACE
 unsigned long long* g_trace_split = nullptr;
 unsigned long long* g_trace_merge = nullptr;
@@ -155,20 +150,10 @@ int decode_impl(const AttnDecodeArgs* a, void* stream_v, const Exchange* xchg) {
 
     const bool kv_bf16 = a->kv_dtype == ATTN_DTYPE_BF16;
     const bool qsplit = a->q_dtype != ATTN_DTYPE_F16;
-    // Single-launch mode: when every segment is shared by only a few CTAs (batched decode), the CTA that delivers a
-    // segment's last partial merges it and there is no merge pass. With many partials per segment (one long
-    // sequence) that one CTA would be slow, and the parallel merge pass is used instead.
-    const uint32_t parts_per_segment = (plan.grid + plan.nseg - 1) / plan.nseg + 1;
-    const bool fused = !xchg && !kv_bf16 && a->kv_len == nullptr && parts_per_segment <= kFusedMaxParts;
-    if (fused) {
-        p.o = a->o;
-        p.lse = a->lse;
-        p.o_dtype = a->o_dtype;
-        p.counters = p.seg_ctas + plan.prefix_words;
-        B200_CUDA_TRY(cudaMemsetAsync(p.counters, 0, static_cast<size_t>(plan.nseg) * 4, stream));
-    }
-    rc = launch_decode_split(p, a->head_dim, plan.hpc, qsplit, kv_bf16, fused, plan.grid, plan.smem_bytes, stream);
-    if (rc != ATTN_OK || fused) return rc;
+    // Always two launches: the merge pass is already resident when the split pass ends. (Merged by its last-arriving CTAs,
+    // as the engine's kernel symbol has to do it, one sequence of 4096 rows takes 28.8 us and not 17.4.)
+    rc = launch_decode_split(p, a->head_dim, plan.hpc, qsplit, kv_bf16, plan.grid, plan.smem_bytes, stream);
+    if (rc != ATTN_OK) return rc;
 
     MergeParams m{};
     m.o = a->o;

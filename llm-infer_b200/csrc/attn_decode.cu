@@ -9,16 +9,15 @@ namespace {
 using decode_detail::kConsumerWarps;
 using decode_detail::kThreads;
 
-// FUSED = the CTA that delivers a segment's last partial also merges it (single launch, no merge pass).
-template <int D, int HPC, bool QSPLIT, bool BF16, bool FUSED>
+template <int D, int HPC, bool QSPLIT, bool BF16>
 __global__ void __launch_bounds__(kThreads, 1) decode_split_kernel(const __grid_constant__ DecodeParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
-    decode_detail::decode_split_body<D, HPC, QSPLIT, BF16, FUSED>(p, smem);
+    decode_detail::decode_split_body<D, HPC, QSPLIT, BF16, /*FUSED=*/false>(p, smem);
 }
 
-template <int D, int HPC, bool QSPLIT, bool BF16, bool FUSED>
+template <int D, int HPC, bool QSPLIT, bool BF16>
 int launch_one(const DecodeParams& p, uint32_t grid, size_t smem_bytes, cudaStream_t stream) {
-    auto kernel = decode_split_kernel<D, HPC, QSPLIT, BF16, FUSED>;
+    auto kernel = decode_split_kernel<D, HPC, QSPLIT, BF16>;
     B200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(smem_bytes)));
     // launched as a programmatic dependent: the launch overlaps the previous kernel's tail; the kernel waits for that
@@ -28,39 +27,33 @@ int launch_one(const DecodeParams& p, uint32_t grid, size_t smem_bytes, cudaStre
     return ATTN_OK;
 }
 
-template <int D, bool QSPLIT, bool BF16, bool FUSED>
+template <int D, bool QSPLIT, bool BF16>
 int launch_hpc(const DecodeParams& p, uint32_t hpc, uint32_t grid, size_t smem_bytes, cudaStream_t stream) {
     switch (hpc) {
-        case 8: return launch_one<D, 8, QSPLIT, BF16, FUSED>(p, grid, smem_bytes, stream);
-        case 4: return launch_one<D, 4, QSPLIT, BF16, FUSED>(p, grid, smem_bytes, stream);
-        case 2: return launch_one<D, 2, QSPLIT, BF16, FUSED>(p, grid, smem_bytes, stream);
-        case 1: return launch_one<D, 1, QSPLIT, BF16, FUSED>(p, grid, smem_bytes, stream);
+        case 8: return launch_one<D, 8, QSPLIT, BF16>(p, grid, smem_bytes, stream);
+        case 4: return launch_one<D, 4, QSPLIT, BF16>(p, grid, smem_bytes, stream);
+        case 2: return launch_one<D, 2, QSPLIT, BF16>(p, grid, smem_bytes, stream);
+        case 1: return launch_one<D, 1, QSPLIT, BF16>(p, grid, smem_bytes, stream);
         default: return ATTN_ERR_UNSUPPORTED;
     }
 }
 
 template <int D>
-int launch_d(const DecodeParams& p, uint32_t hpc, bool qsplit, bool kv_bf16, bool fused, uint32_t grid,
-             size_t smem_bytes, cudaStream_t stream) {
-    if (kv_bf16) {
-        // bf16 MMA operands: Q and P always carry a residual term (8-bit significand otherwise); two-pass only
-        return launch_hpc<D, true, true, false>(p, hpc, grid, smem_bytes, stream);
-    }
-    if (fused) {
-        return qsplit ? launch_hpc<D, true, false, true>(p, hpc, grid, smem_bytes, stream)
-                      : launch_hpc<D, false, false, true>(p, hpc, grid, smem_bytes, stream);
-    }
-    return qsplit ? launch_hpc<D, true, false, false>(p, hpc, grid, smem_bytes, stream)
-                  : launch_hpc<D, false, false, false>(p, hpc, grid, smem_bytes, stream);
+int launch_d(const DecodeParams& p, uint32_t hpc, bool qsplit, bool kv_bf16, uint32_t grid, size_t smem_bytes,
+             cudaStream_t stream) {
+    // bf16 MMA operands: Q and P always carry a residual term (8-bit significand otherwise)
+    if (kv_bf16) return launch_hpc<D, true, true>(p, hpc, grid, smem_bytes, stream);
+    return qsplit ? launch_hpc<D, true, false>(p, hpc, grid, smem_bytes, stream)
+                  : launch_hpc<D, false, false>(p, hpc, grid, smem_bytes, stream);
 }
 
 }  // namespace
 
-int launch_decode_split(const DecodeParams& p, uint32_t head_dim, uint32_t hpc, bool qsplit, bool kv_bf16, bool fused,
-                        uint32_t grid, size_t smem_bytes, cudaStream_t stream) {
+int launch_decode_split(const DecodeParams& p, uint32_t head_dim, uint32_t hpc, bool qsplit, bool kv_bf16, uint32_t grid,
+                        size_t smem_bytes, cudaStream_t stream) {
     switch (head_dim) {
-        case 128: return launch_d<128>(p, hpc, qsplit, kv_bf16, fused, grid, smem_bytes, stream);
-        case 64: return launch_d<64>(p, hpc, qsplit, kv_bf16, fused, grid, smem_bytes, stream);
+        case 128: return launch_d<128>(p, hpc, qsplit, kv_bf16, grid, smem_bytes, stream);
+        case 64: return launch_d<64>(p, hpc, qsplit, kv_bf16, grid, smem_bytes, stream);
         default: return ATTN_ERR_UNSUPPORTED;
     }
 }

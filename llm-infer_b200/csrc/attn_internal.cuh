@@ -216,8 +216,8 @@ struct DeviceInfo {
 // Properties of the current device (cached per device; no allocation).
 int current_device_info(DeviceInfo* out);
 
-int launch_decode_split(const DecodeParams& p, uint32_t head_dim, uint32_t hpc, bool qsplit, bool kv_bf16, bool fused,
-                        uint32_t grid, size_t smem_bytes, cudaStream_t stream);
+int launch_decode_split(const DecodeParams& p, uint32_t head_dim, uint32_t hpc, bool qsplit, bool kv_bf16, uint32_t grid,
+                        size_t smem_bytes, cudaStream_t stream);
 int launch_merge(const MergeParams& p, cudaStream_t stream, bool dependent_launch);
 // fp16-weight GEMV on the tensor cores (attn_gemv_f16mma.cu): batches and the fused forms of attn_gemv_f16.
 int launch_gemv_f16_mma(const AttnGemvArgs* a, cudaStream_t stream);

@@ -136,6 +136,7 @@ __device__ __forceinline__ void load_q_fragments(const T* q_head0, int D, int G,
 // LOW8: the caller guarantees at most eight query heads per kv head. Rows 8-15 of every MMA are then empty, and the
 // query fragments, score and output accumulators of those rows (half of each: 64 registers with value + residual
 // queries and head_dim 128) are not kept at all.
+// FUSED = single launch: the CTA that delivers a segment's last partial also merges it (the engine's kernel symbol).
 template <int D, int HPC, bool QSPLIT, bool BF16, bool FUSED, bool LOW8 = false>
 __device__ __forceinline__ void decode_split_body(const DecodeParams& p, unsigned char* smem) {
     constexpr int TS = kConsumerWarps / HPC;     // row sub-tiles per kv head
