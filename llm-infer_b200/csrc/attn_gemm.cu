@@ -414,7 +414,8 @@ int launch_gemm(GemmParams& p, const void* a_hi, const void* a_lo, const void* w
     p.n_tile = t.n_tile;
     p.m_tiles = t.m_tiles;
     p.n_tiles = t.n_tiles;
-    // rows of A of a band: up to ~ 36 MB of operands, a quarter of L2, stay there while W streams past
+    // rows of A of a band: up to ~ 36 MB of operands, a quarter of L2, stay there while W streams past, but at least four
+    // row tiles, so that a W tile is used that often (k = 14336, a pair, value and residual: 59 MB)
     const uint64_t row_tile_bytes = static_cast<uint64_t>(t.pair ? 2 : 1) * GM * p.k * 2 * (1 + alo);
     p.band = static_cast<uint32_t>(std::min<uint64_t>(t.m_tiles, std::max<uint64_t>(4, (36ull << 20) / row_tile_bytes)));
     p.acc_cols = t.n_tile <= 128 ? 128 : 256;

@@ -134,7 +134,8 @@ __global__ void __launch_bounds__(kMergeThreads, 4) merge_rows_kernel(const __gr
     const float zt = z * e0 + z1 * e1;
     const float inv_z = zt > 0.f ? 1.f / zt : 0.f;
     const size_t obase = static_cast<size_t>(row) * p.head_dim + lane * VEC;
-    // whole 16-byte stores where the output allows them (it may lie in pinned host memory: fewer, larger writes)
+    // whole 16-byte stores where the output allows them (it may lie in pinned host memory: fewer, larger writes);
+    // head_dim 64 has two values per lane and stores them one by one
     const bool wide = VEC == 4 && p.o_dtype == ATTN_DTYPE_F32 && (reinterpret_cast<uintptr_t>(p.o) & 15u) == 0;
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c) {

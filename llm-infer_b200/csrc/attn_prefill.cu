@@ -13,7 +13,7 @@
 // same rows when the GQA group is even, else two consecutive row tiles of one head). Persistent, one CTA per SM: the
 // items are dealt longest causal span first, back and forth over the CTAs (4 x 2048 rows: 1024 items, no CTA more than
 // one item above another), and an item's loads and first score products run while the previous item's result is
-// written: 196 -> 181 us (758 TFLOP/s causal). 12 warps:
+// written: 196 -> 181 us in a burst (758 TFLOP/s causal; 209 us in a sustained loop under the power cap). 12 warps:
 //   warps 0-3   softmax of tile 0: thread r owns query row r (tensor-memory lane r), no shuffles needed
 //   warps 4-7   softmax of tile 1
 //   warp  8     TMA producer: an item's Q tiles, then its K and V tiles (64 keys x 128 dims, 128-byte swizzle)
