@@ -150,6 +150,12 @@ int decode_impl(const AttnDecodeArgs* a, void* stream_v, const Exchange* xchg) {
 
     const bool kv_bf16 = a->kv_dtype == ATTN_DTYPE_BF16;
     const bool qsplit = a->q_dtype != ATTN_DTYPE_F16;
+    // Up to eight query heads per kv head leave half of the MMAs' rows to the residual products (decode_body.cuh, PACK8): 7
+    // sequences up to 2999 rows 18.6 -> 16.2 us, 8 x 2048 19.1 -> 17.6, 16 x 4096 49.3 -> 46.9 (graphs of calls). Sums come out in
+    // another order. The prepared output form is what a generation step takes between its layers, and a step's results (cache
+    // rows, picked tokens) stay what they were bit for bit: it keeps the form without.
+    const bool prepared = a->o_dtype == ATTN_DTYPE_SPLIT16;
+    p.pack8 = plan.group <= 8 && !prepared ? 1u : 0u;
     // Always two launches: the merge pass is already resident when the split pass ends. (Merged by its last-arriving CTAs,
     // as the engine's kernel symbol has to do it, one sequence of 4096 rows takes 28.8 us and not 17.4.)
     rc = launch_decode_split(p, a->head_dim, plan.hpc, qsplit, kv_bf16, plan.grid, plan.smem_bytes, stream);

@@ -9,15 +9,15 @@ namespace {
 using decode_detail::kConsumerWarps;
 using decode_detail::kThreads;
 
-template <int D, int HPC, bool QSPLIT, bool BF16>
+template <int D, int HPC, bool QSPLIT, bool BF16, bool PACK8>
 __global__ void __launch_bounds__(kThreads, 1) decode_split_kernel(const __grid_constant__ DecodeParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
-    decode_detail::decode_split_body<D, HPC, QSPLIT, BF16, /*FUSED=*/false>(p, smem);
+    decode_detail::decode_split_body<D, HPC, QSPLIT, BF16, /*FUSED=*/false, /*LOW8=*/false, PACK8>(p, smem);
 }
 
 template <int D, int HPC, bool QSPLIT, bool BF16>
 int launch_one(const DecodeParams& p, uint32_t grid, size_t smem_bytes, cudaStream_t stream) {
-    auto kernel = decode_split_kernel<D, HPC, QSPLIT, BF16>;
+    auto kernel = p.pack8 ? decode_split_kernel<D, HPC, QSPLIT, BF16, true> : decode_split_kernel<D, HPC, QSPLIT, BF16, false>;
     B200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(smem_bytes)));
     // launched as a programmatic dependent: the launch overlaps the previous kernel's tail; the kernel waits for that

@@ -46,6 +46,7 @@ struct DecodeParams {
     uint32_t max_ctas;
     uint32_t min_tiles_per_cta;
     uint32_t nstages;
+    uint32_t pack8;        // split pass: the MMAs' rows 8-15 carry the residual products
     uint32_t kv_early;     // AttnDecodeArgs.kv_early
     uint32_t kv_capacity;  // rows a sequence's caches hold, 0 = not stated (lengths beyond it are clamped and reported)
 #ifdef ATTN_BOUNDS_CHECK

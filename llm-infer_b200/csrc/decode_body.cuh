@@ -136,8 +136,11 @@ __device__ __forceinline__ void load_q_fragments(const T* q_head0, int D, int G,
 // LOW8: the caller guarantees at most eight query heads per kv head. Rows 8-15 of every MMA are then empty, and the
 // query fragments, score and output accumulators of those rows (half of each: 64 registers with value + residual
 // queries and head_dim 128) are not kept at all.
+// PACK8: the same condition, and rows 8-15 carry the residuals: A's rows 0-7 are the value halves of the heads' queries (or
+// probabilities), its rows 8-15 the residual halves, so one MMA does what takes two otherwise. The two sums of a head lie in the
+// same lane (rows g and g + 8) and are added at the end.
 // FUSED = single launch: the CTA that delivers a segment's last partial also merges it (the engine's kernel symbol).
-template <int D, int HPC, bool QSPLIT, bool BF16, bool FUSED, bool LOW8 = false>
+template <int D, int HPC, bool QSPLIT, bool BF16, bool FUSED, bool LOW8 = false, bool PACK8 = false>
 __device__ __forceinline__ void decode_split_body(const DecodeParams& p, unsigned char* smem) {
     constexpr int TS = kConsumerWarps / HPC;     // row sub-tiles per kv head
     constexpr int TT = 16 * TS;                  // rows per tile
@@ -363,7 +366,7 @@ __device__ __forceinline__ void decode_split_body(const DecodeParams& p, unsigne
     const int gq = lane >> 2;        // MMA row owned by this lane (and gq + 8)
     const int cq = lane & 3;
     const uint32_t G = p.group;
-    const bool ghi = !LOW8 && G > 8;  // rows 8..15 of the MMA hold real heads
+    const bool ghi = !LOW8 && !PACK8 && G > 8;  // rows 8..15 of the MMA hold real heads
 
     // per-lane ldmatrix row addresses inside a tile (stage base added per tile)
     const uint32_t k_lane_off = (ts * 16 + ((lane >> 4) << 3) + (lane & 7)) * PITCH + hh * (D * 2) + (((lane >> 3) & 1) << 4);
@@ -414,7 +417,18 @@ __device__ __forceinline__ void decode_split_body(const DecodeParams& p, unsigne
         return true;
     };
 
+    // PACK8: value and residual products of a head into one
+    auto join_halves = [&]() {
+        if constexpr (PACK8) {
+#pragma unroll
+            for (int dn = 0; dn < DN; ++dn) {
+                o[dn][0] += o[dn][2];
+                o[dn][1] += o[dn][3];
+            }
+        }
+    };
     auto end_segment = [&]() {
+        join_halves();
         // quad-reduce the row sums, normalise, write this warp's partial
         l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
         l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
@@ -587,7 +601,11 @@ __device__ __forceinline__ void decode_split_body(const DecodeParams& p, unsigne
         for (int kc = 0; kc < KC; ++kc) {
             uint32_t b0, b1, b2, b3;
             ldmatrix_x4(b0, b1, b2, b3, kbase + k_lane_off + kc * 32);
-            if constexpr (LOW8) {
+            if constexpr (PACK8) {
+                const uint32_t a[4] = {qhi[kc][0], QSPLIT ? qlo[QSPLIT ? kc : 0][0] : 0u, qhi[kc][2], QSPLIT ? qlo[QSPLIT ? kc : 0][2] : 0u};
+                mma_16816<BF16>(s[0], a, b0, b1);
+                mma_16816<BF16>(s[1], a, b2, b3);
+            } else if constexpr (LOW8) {
                 mma_16816_low8<BF16>(s[0][0], s[0][1], qhi[kc][0], qhi[kc][2], b0, b1);
                 mma_16816_low8<BF16>(s[1][0], s[1][1], qhi[kc][0], qhi[kc][2], b2, b3);
                 if constexpr (QSPLIT) {
@@ -604,12 +622,20 @@ __device__ __forceinline__ void decode_split_body(const DecodeParams& p, unsigne
             }
         }
 
+        if constexpr (PACK8 && QSPLIT) {
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+                s[n][0] += s[n][2];
+                s[n][1] += s[n][3];
+            }
+        }
+
         // ---- scale, mask rows past the sequence end ----
         const uint32_t tok = (gt - seg.tile0) * TT + ts * 16 + cq * 2;  // row of s[0][0]; s[1][*] is +8
 #pragma unroll
         for (int n = 0; n < 2; ++n) {
 #pragma unroll
-            for (int e = 0; e < (LOW8 ? 2 : 4); ++e) {
+            for (int e = 0; e < (LOW8 || PACK8 ? 2 : 4); ++e) {
                 const uint32_t r = tok + n * 8 + (e & 1);
                 s[n][e] = r < seg.len ? s[n][e] * p.scale_log2 : -INFINITY;
             }
@@ -664,8 +690,8 @@ __device__ __forceinline__ void decode_split_body(const DecodeParams& p, unsigne
                 o[dn][0] *= sc0;
                 o[dn][1] *= sc0;
                 if constexpr (!LOW8) {
-                    o[dn][2] *= sc1;
-                    o[dn][3] *= sc1;
+                    o[dn][2] *= PACK8 ? sc0 : sc1;
+                    o[dn][3] *= PACK8 ? sc0 : sc1;
                 }
             }
         }
@@ -680,7 +706,11 @@ __device__ __forceinline__ void decode_split_body(const DecodeParams& p, unsigne
         for (int d2 = 0; d2 < DN / 2; ++d2) {
             uint32_t b0, b1, b2, b3;
             ldmatrix_x4_trans(b0, b1, b2, b3, vbase + v_lane_off + d2 * 32);
-            if constexpr (LOW8) {
+            if constexpr (PACK8) {
+                const uint32_t a[4] = {pa[0], pb[0], pa[2], pb[2]};
+                mma_16816<BF16>(o[2 * d2], a, b0, b1);
+                mma_16816<BF16>(o[2 * d2 + 1], a, b2, b3);
+            } else if constexpr (LOW8) {
                 mma_16816_low8<BF16>(o[2 * d2][0], o[2 * d2][1], pa[0], pa[2], b0, b1);
                 mma_16816_low8<BF16>(o[2 * d2 + 1][0], o[2 * d2 + 1][1], pa[0], pa[2], b2, b3);
                 mma_16816_low8<BF16>(o[2 * d2][0], o[2 * d2][1], pb[0], pb[2], b0, b1);
