@@ -156,7 +156,21 @@ int decode_impl(const AttnDecodeArgs* a, void* stream_v, const Exchange* xchg) {
     // rows, picked tokens) stay what they were bit for bit: it keeps the form without.
     const bool prepared = a->o_dtype == ATTN_DTYPE_SPLIT16;
     p.pack8 = plan.group <= 8 && !prepared ? 1u : 0u;
-    // Always two launches: the merge pass is already resident when the split pass ends. (Merged by its last-arriving CTAs,
+    const uint32_t rows = a->kv_len ? a->kv_capacity : clamped_len(a->kv_len_uniform, a->kv_capacity);
+    DecodeClusterPlan cl{};
+    if (!xchg && !prepared && a->max_ctas == 0 &&
+        pick_decode_cluster(a->batch, a->n_heads, a->n_kv_heads, a->head_dim, rows, a->kv_len != nullptr, dev, &cl)) {
+        DecodeParams c = p;
+        c.head_groups = a->n_kv_heads / cl.hpc;
+        c.nstages = cl.stages;
+        c.o = a->o;
+        c.lse = a->lse;
+        c.o_dtype = a->o_dtype;
+        c.cluster = cl.cluster;
+        rc = launch_decode_cluster(c, cl, a->head_dim, qsplit, kv_bf16, stream);
+        if (rc != kClusterNotTaken) return rc;
+    }
+    // Otherwise two launches: the merge pass is already resident when the split pass ends. (Merged by its last-arriving CTAs,
     // as the engine's kernel symbol has to do it, one sequence of 4096 rows takes 28.8 us and not 17.4.)
     rc = launch_decode_split(p, a->head_dim, plan.hpc, qsplit, kv_bf16, plan.grid, plan.smem_bytes, stream);
     if (rc != ATTN_OK) return rc;

@@ -54,10 +54,12 @@ struct DecodeParams {
     uint64_t group_slots;  // group records / group counters that exist (single-launch mode)
 #endif
     uint32_t* status;
-    // single-launch (fused merge) mode only: final output and per-segment arrival counters
+    // single-launch modes only: final output
     void* o;
     float* lse;
     int32_t o_dtype;
+    uint32_t cluster;    // CTAs per segment (cluster mode)
+    // fused merge: per-segment arrival counters
     uint32_t* counters;  // [nseg], zero before the first launch; the kernel leaves them zero
     // two-level merge of the single-launch mode (segments shared by many CTAs): first-level groups of CTAs merge
     // their partials into group records, the last group to finish merges the records. nullptr = one level only.
@@ -220,6 +222,20 @@ int current_device_info(DeviceInfo* out);
 int launch_decode_split(const DecodeParams& p, uint32_t head_dim, uint32_t hpc, bool qsplit, bool kv_bf16, uint32_t grid,
                         size_t smem_bytes, cudaStream_t stream);
 int launch_merge(const MergeParams& p, cudaStream_t stream, bool dependent_launch);
+// The same in one launch of clusters, one cluster per segment (decode_cluster.cu). pick_decode_cluster says whether a call
+// should take it and fills the plan.
+struct DecodeClusterPlan {
+    uint32_t rows;      // rows that a sequence's caches hold at least
+    uint32_t hpc;       // kv heads per CTA
+    uint32_t cluster;   // CTAs per segment
+    uint32_t stages, segments;
+    size_t smem_bytes;
+};
+bool pick_decode_cluster(uint32_t batch, uint32_t n_heads, uint32_t n_kv_heads, uint32_t head_dim, uint32_t rows, bool ragged,
+                         const DeviceInfo& dev, DecodeClusterPlan* plan);
+constexpr int kClusterNotTaken = 1;  // nothing was launched: the other form has to serve the call
+int launch_decode_cluster(const DecodeParams& p, const DecodeClusterPlan& plan, uint32_t head_dim, bool qsplit, bool kv_bf16,
+                          cudaStream_t stream);
 // fp16-weight GEMV on the tensor cores (attn_gemv_f16mma.cu): batches and the fused forms of attn_gemv_f16.
 int launch_gemv_f16_mma(const AttnGemvArgs* a, cudaStream_t stream);
 

@@ -28,6 +28,8 @@
 // last tile of a segment), Q once per (CTA, segment), partials once.
 #pragma once
 
+#include <cuda.h>
+
 #include "attn_internal.cuh"
 #include "merge_device.cuh"
 #include "ptx_sm100.cuh"
@@ -140,12 +142,22 @@ __device__ __forceinline__ void load_q_fragments(const T* q_head0, int D, int G,
 // probabilities), its rows 8-15 the residual halves, so one MMA does what takes two otherwise. The two sums of a head lie in the
 // same lane (rows g and g + 8) and are added at the end.
 // FUSED = single launch: the CTA that delivers a segment's last partial also merges it (the engine's kernel symbol).
-template <int D, int HPC, bool QSPLIT, bool BF16, bool FUSED, bool LOW8 = false, bool PACK8 = false>
-__device__ __forceinline__ void decode_split_body(const DecodeParams& p, unsigned char* smem) {
+// CLUSTER = single launch over clusters of CTAs, one per segment: every CTA takes an equal share of the segment's tiles,
+// leaves its partials in its own shared memory, and after a cluster barrier the CTAs merge a share of the rows each, reading
+// the others' partials over distributed shared memory. K and V tiles come as ONE tiled TMA copy each (tensor maps tm_k, tm_v:
+// [sequence][kv head][128-byte part of a head][row][64 elements], 128-byte swizzle) in place of a bulk copy per cache row, which
+// the copy engine takes one of per ~ 30 ns + 12 ns per KB: a 64 KB tile in 1.75 us (HPC 8) to 9 us (HPC 1).
+template <int D, int HPC, bool QSPLIT, bool BF16, bool FUSED, bool LOW8 = false, bool PACK8 = false, bool CLUSTER = false>
+__device__ __forceinline__ void decode_split_body(const DecodeParams& p, unsigned char* smem, const CUtensorMap* tm_k = nullptr,
+                                                  const CUtensorMap* tm_v = nullptr) {
+    // single-launch modes meet at barriers after the loop: a warp whose bounded wait ran out stays, see wait_failed
+    constexpr bool STAY = FUSED || CLUSTER;
     constexpr int TS = kConsumerWarps / HPC;     // row sub-tiles per kv head
     constexpr int TT = 16 * TS;                  // rows per tile
     constexpr int ROWB = HPC * D * 2;            // bytes of one cache row slice (HPC kv heads)
-    constexpr int PITCH = ROWB + 16;             // shared-memory row pitch
+    constexpr int PITCH = CLUSTER ? ROWB : ROWB + 16;  // shared-memory row pitch (cluster mode: swizzled instead of padded)
+    constexpr int PART = TT * 128;               // cluster mode: one 128-byte part of a head over a tile's rows
+    constexpr int HEADB = PART * (D / 64);       // ... and a whole head
     constexpr int TILEB = TT * PITCH;            // one K (or V) tile
     constexpr int KC = D / 16;                   // k-chunks of the QK^T contraction
     constexpr int DN = D / 8;                    // n-tiles of the PV product
@@ -198,7 +210,7 @@ __device__ __forceinline__ void decode_split_body(const DecodeParams& p, unsigne
         mbar_init(bar_q_full, 1);
         mbar_init(bar_q_empty, kConsumerWarps);
         mbar_init_fence();
-        if constexpr (FUSED) *s_abort = 0u;
+        if constexpr (STAY) *s_abort = 0u;
     }
     // This grid waits for the kernel before it (which wrote q, the newest cache row and possibly the lengths) before
     // it reads any of them. With kv_early the caller vouches that the lengths were in place before that kernel was
@@ -217,7 +229,10 @@ __device__ __forceinline__ void decode_split_body(const DecodeParams& p, unsigne
     // ---- tile prefix over segments (ragged lengths only) --------------------
     uint64_t nt;
     uint32_t tiles_uniform = 0;
-    if (p.kv_len) {
+    if constexpr (CLUSTER) {
+        nt = 0;
+        __syncthreads();
+    } else if (p.kv_len) {
         for (uint32_t s = tid; s < nseg; s += kThreads) {
             const uint32_t stated = p.kv_len[s / p.head_groups];
             const uint32_t len = clamped_len(stated, p.kv_capacity);
@@ -255,19 +270,34 @@ __device__ __forceinline__ void decode_split_body(const DecodeParams& p, unsigne
         nt = static_cast<uint64_t>(tiles_uniform) * nseg;
         __syncthreads();
     }
-    if (nt == 0) return;
-    if (tid == 0) DTRACE(2);
-
-    const uint32_t active = active_ctas(gridDim.x, p.max_ctas, p.min_tiles_per_cta, nt);
-    const uint32_t cta = blockIdx.x;
-    if (cta >= active) return;
-    const uint32_t t_begin = static_cast<uint32_t>(div_mostly_32(cta * nt, active));
-    const uint32_t t_end = static_cast<uint32_t>(div_mostly_32((cta + 1) * nt, active));
-    const uint32_t n_my = t_end - t_begin;
-    if (n_my == 0) return;
-
     SegTable<TT> table{p, prefix, tiles_uniform};
-    SegInfo seg = table.load(table.find(t_begin, nseg));
+    SegInfo seg;
+    uint32_t active = 1, t_begin, t_end;
+    const uint32_t cta = blockIdx.x;
+    if constexpr (CLUSTER) {
+        // this cluster's segment, its tiles counted from 0; a CTA may be left without any, and merges all the same
+        seg.seg = blockIdx.x / p.cluster;
+        seg.b = seg.seg / p.head_groups;
+        seg.hg = seg.seg - seg.b * p.head_groups;
+        const uint32_t stated = p.kv_len ? p.kv_len[seg.b] : p.kv_len_uniform;
+        seg.len = clamped_len(stated, p.kv_capacity);
+        if (p.kv_len && seg.len != stated && tid == 0 && p.status) atomicOr(p.status, ATTN_STATUS_BAD_SHAPE);
+        seg.tile0 = 0;
+        seg.tile_end = (seg.len + TT - 1) / TT;
+        const uint32_t rank = cta - seg.seg * p.cluster;
+        t_begin = static_cast<uint32_t>(static_cast<uint64_t>(rank) * seg.tile_end / p.cluster);
+        t_end = static_cast<uint32_t>(static_cast<uint64_t>(rank + 1) * seg.tile_end / p.cluster);
+    } else {
+        if (nt == 0) return;
+        if (tid == 0) DTRACE(2);
+        active = active_ctas(gridDim.x, p.max_ctas, p.min_tiles_per_cta, nt);
+        if (cta >= active) return;
+        t_begin = static_cast<uint32_t>(div_mostly_32(cta * nt, active));
+        t_end = static_cast<uint32_t>(div_mostly_32((cta + 1) * nt, active));
+        if (t_end == t_begin) return;
+        seg = table.load(table.find(t_begin, nseg));
+    }
+    const uint32_t n_my = t_end - t_begin;
 
     if (warp == kConsumerWarps) {
         // ===================== producer warp =====================
@@ -285,7 +315,13 @@ __device__ __forceinline__ void decode_split_body(const DecodeParams& p, unsigne
             if (lane == 0) {
                 mbar_arrive_expect_tx(bar_full_k + 8 * st, TT * ROWB);
                 mbar_arrive_expect_tx(bar_full_v + 8 * st, TT * ROWB);
+                if constexpr (CLUSTER) {
+                    const int row = static_cast<int>(tok0), head = static_cast<int>(seg.hg * HPC), b = static_cast<int>(seg.b);
+                    tma_load_5d_hint(kdst, tm_k, bar_full_k + 8 * st, row, 0, head, b, policy);
+                    tma_load_5d_hint(vdst, tm_v, bar_full_v + 8 * st, row, 0, head, b, policy);
+                }
             }
+            if constexpr (CLUSTER) return;
             __syncwarp();
             // Rows past the end of the sequence re-read its last valid row: the
             // tile is always full (constant byte count) and always finite; those
@@ -369,8 +405,17 @@ __device__ __forceinline__ void decode_split_body(const DecodeParams& p, unsigne
     const bool ghi = !LOW8 && !PACK8 && G > 8;  // rows 8..15 of the MMA hold real heads
 
     // per-lane ldmatrix row addresses inside a tile (stage base added per tile)
-    const uint32_t k_lane_off = (ts * 16 + ((lane >> 4) << 3) + (lane & 7)) * PITCH + hh * (D * 2) + (((lane >> 3) & 1) << 4);
-    const uint32_t v_lane_off = (ts * 16 + (((lane >> 3) & 1) << 3) + (lane & 7)) * PITCH + hh * (D * 2) + ((lane >> 4) << 4);
+    const uint32_t k_row = ts * 16 + ((lane >> 4) << 3) + (lane & 7), v_row = ts * 16 + (((lane >> 3) & 1) << 3) + (lane & 7);
+    const uint32_t k_lane_off = CLUSTER ? hh * HEADB + k_row * 128 : k_row * PITCH + hh * (D * 2) + (((lane >> 3) & 1) << 4);
+    const uint32_t v_lane_off = CLUSTER ? hh * HEADB + v_row * 128 : v_row * PITCH + hh * (D * 2) + ((lane >> 4) << 4);
+    // cluster mode: the 16-byte chunk c of a row lies at chunk c ^ (row & 7)
+    const uint32_t k_chunk = (((lane >> 3) & 1) ^ (lane & 7)) << 4, v_chunk = ((lane >> 4) ^ (lane & 7)) << 4;
+    auto k_addr = [&](uint32_t tile, int kc) {
+        return CLUSTER ? tile + k_lane_off + (kc >> 2) * PART + (k_chunk ^ ((kc & 3) << 5)) : tile + k_lane_off + kc * 32;
+    };
+    auto v_addr = [&](uint32_t tile, int d2) {
+        return CLUSTER ? tile + v_lane_off + (d2 >> 2) * PART + (v_chunk ^ ((d2 & 3) << 5)) : tile + v_lane_off + d2 * 32;
+    };
 
     uint32_t qhi[KC][4];
     uint32_t qlo[QSPLIT ? KC : 1][4];
@@ -380,11 +425,11 @@ __device__ __forceinline__ void decode_split_body(const DecodeParams& p, unsigne
     uint32_t n_seg = 0;  // segments this CTA has started (parity of the query-row barriers)
     bool failed = false;
     // What a warp does when one of its bounded waits runs out: two-pass mode has no barrier after this point, so the
-    // warp simply leaves (its partials are missing and the status bit says so); in single-launch mode it stays, see
-    // fused_merge below.
+    // warp simply leaves (its partials are missing and the status bit says so); in the single-launch modes it stays, see
+    // fused_merge and cluster_merge below.
     auto wait_failed = [&]() {
         if (lane == 0 && p.status) atomicOr(p.status, ATTN_STATUS_WAIT_TIMEOUT);
-        if constexpr (FUSED) {
+        if constexpr (STAY) {
             *s_abort = 1u;
             failed = true;
         }
@@ -564,14 +609,126 @@ __device__ __forceinline__ void decode_split_body(const DecodeParams& p, unsigne
         }
     };
 
-    if (!begin_segment()) {
-        if constexpr (!FUSED) return;
+    // Cluster mode: every CTA leaves its warps' partials in its own shared memory (over the tile ring, which nobody reads any
+    // more), the cluster meets, and thread t of the cluster merges one float4 of a row from every S-th partial, S neighbouring
+    // lanes sharing an item. The second barrier keeps a CTA's partials alive until all have read them. A warp whose wait
+    // ran out meets both barriers too; its CTA's mark keeps the whole segment's output untouched.
+    auto cluster_merge = [&]() {
+        if constexpr (CLUSTER) {
+            static_assert(PACK8, "rows 8-15 of the MMA hold no head here");
+            constexpr int PD = D + 8;  // row pitch: the eight rows of a warp's float2 stores fall into different banks
+            constexpr float kLn2 = 0.6931471805599453f;
+            constexpr uint32_t F4 = D / 4;
+            const uint32_t R = HPC * G, C = p.cluster, rank = cta - seg.seg * C;
+            float* s_part = reinterpret_cast<float*>(tiles);  // [TS][R][PD], then the LSEs [TS][R]
+            float* s_lse = s_part + static_cast<size_t>(TS) * R * PD;
+            join_halves();
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
+            l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
+            if (gq < static_cast<int>(G)) {
+                const float inv0 = l0 > 0.f ? 1.f / l0 : 0.f;
+                const uint32_t prow = ts * R + hh * G + gq;
+                float* dst = s_part + prow * PD + cq * 2;
+#pragma unroll
+                for (int dn = 0; dn < DN; ++dn)
+                    *reinterpret_cast<float2*>(dst + dn * 8) = make_float2(o[dn][0] * inv0, o[dn][1] * inv0);
+                if (cq == 0) s_lse[prow] = l0 > 0.f ? (m0 + log2f(l0)) * kLn2 : -INFINITY;
+            }
+            __syncwarp();
+            cluster_arrive();
+            cluster_wait();
+            const uint32_t part0 = smem_u32(s_part), lse0 = smem_u32(s_lse);
+            const uint32_t lane_abort =
+                lane < static_cast<int>(C) ? ld_cluster_u32(cluster_address(smem_u32(const_cast<uint32_t*>(s_abort)), lane)) : 0u;
+            const uint32_t items = R * F4, P = C * TS, threads = C * kConsumerWarps * 32;
+            uint32_t S = 1;
+            while (S < 32 && 2 * S <= P && 2 * S * items <= threads) S *= 2;
+            const uint32_t gid = rank * kConsumerWarps * 32 + tid, sub = gid & (S - 1);
+            const bool aborted = __any_sync(0xffffffffu, lane_abort != 0u);
+            for (uint32_t it0 = 0; it0 < items && !aborted; it0 += threads / S) {
+                const uint32_t item = it0 + gid / S;
+                const bool live = item < items;
+                const uint32_t r = item / F4, f = item - r * F4;
+                float m = -INFINITY, z = 0.f;
+                float acc[4] = {0.f, 0.f, 0.f, 0.f};
+                for (uint32_t p0 = sub; live && p0 < P; p0 += 4 * S) {
+                    float lw[4];
+                    float4 x[4];
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) {
+                        const uint32_t pi = p0 + b * S;
+                        lw[b] = -INFINITY;
+                        x[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (pi < P) {
+                            const uint32_t from = pi / TS, prow = (pi - from * TS) * R + r;
+                            lw[b] = __uint_as_float(ld_cluster_u32(cluster_address(lse0 + prow * 4, from)));
+                            x[b] = ld_cluster_f4(cluster_address(part0 + (prow * PD + f * 4) * 4, from));
+                        }
+                    }
+                    const float bm = fmaxf(fmaxf(lw[0], lw[1]), fmaxf(lw[2], lw[3]));
+                    if (bm > m) {
+                        const float sc = __expf(m - bm);  // 0 when nothing was folded yet
+                        z *= sc;
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) acc[e] *= sc;
+                        m = bm;
+                    }
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) {
+                        const float w = lw[b] == -INFINITY ? 0.f : __expf(lw[b] - m);
+                        z += w;
+                        acc[0] = fmaf(w, x[b].x, acc[0]);
+                        acc[1] = fmaf(w, x[b].y, acc[1]);
+                        acc[2] = fmaf(w, x[b].z, acc[2]);
+                        acc[3] = fmaf(w, x[b].w, acc[3]);
+                    }
+                }
+                float mx = m;
+                for (uint32_t off = S / 2; off; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+                const float sc = m == -INFINITY ? 0.f : __expf(m - mx);
+                z *= sc;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[e] *= sc;
+                for (uint32_t off = S / 2; off; off >>= 1) {
+                    z += __shfl_xor_sync(0xffffffffu, z, off);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], off);
+                }
+                if (live && sub == 0) {
+                    const float inv = z > 0.f ? 1.f / z : 0.f;
+                    const size_t orow = static_cast<size_t>(seg.b) * p.n_heads + static_cast<size_t>(seg.hg) * R + r;
+                    const size_t idx = orow * D + f * 4;
+                    // whole 16-byte stores where the output allows them (it may lie in pinned host memory)
+                    if (p.o_dtype == ATTN_DTYPE_F32 && (reinterpret_cast<uintptr_t>(p.o) & 15u) == 0) {
+                        *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.o) + idx) =
+                            make_float4(acc[0] * inv, acc[1] * inv, acc[2] * inv, acc[3] * inv);
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) store_out(p.o, p.o_dtype, idx + e, acc[e] * inv);
+                    }
+                    if (p.lse && f == 0) p.lse[orow] = z > 0.f ? mx + logf(z) : -INFINITY;
+                }
+            }
+            __syncwarp();
+            cluster_arrive();
+            cluster_wait();
+        }
+    };
+
+    if (CLUSTER && n_my == 0) {
+#pragma unroll
+        for (int dn = 0; dn < DN; ++dn) o[dn][0] = o[dn][1] = o[dn][2] = o[dn][3] = 0.f;
+        m0 = m1 = -INFINITY;
+        l0 = l1 = 0.f;
+    } else if (!begin_segment()) {
+        if constexpr (!STAY) return;
     }
     if (warp == 0 && lane == 0) DTRACE(3);
 
     for (uint32_t i = 0; i < n_my; ++i) {
         const uint32_t gt = t_begin + i;
-        if (gt >= seg.tile_end) {
+        if (!CLUSTER && gt >= seg.tile_end) {
             if (!failed) end_segment();
             fused_merge();
             do { seg = table.load(seg.seg + 1); } while (gt >= seg.tile_end);
@@ -579,7 +736,7 @@ __device__ __forceinline__ void decode_split_body(const DecodeParams& p, unsigne
                 if constexpr (!FUSED) return;
             }
         }
-        if constexpr (FUSED) {
+        if constexpr (STAY) {
             if (failed) continue;
         }
         const uint32_t st = i % nst;
@@ -589,7 +746,7 @@ __device__ __forceinline__ void decode_split_body(const DecodeParams& p, unsigne
 
         if (!mbar_wait(bar_full_k + 8 * st, par)) {
             wait_failed();
-            if constexpr (FUSED) continue; else return;
+            if constexpr (STAY) continue; else return;
         }
         if (i == 0 && warp == 0 && lane == 0) DTRACE(4);
 
@@ -600,7 +757,7 @@ __device__ __forceinline__ void decode_split_body(const DecodeParams& p, unsigne
 #pragma unroll
         for (int kc = 0; kc < KC; ++kc) {
             uint32_t b0, b1, b2, b3;
-            ldmatrix_x4(b0, b1, b2, b3, kbase + k_lane_off + kc * 32);
+            ldmatrix_x4(b0, b1, b2, b3, k_addr(kbase, kc));
             if constexpr (PACK8) {
                 const uint32_t a[4] = {qhi[kc][0], QSPLIT ? qlo[QSPLIT ? kc : 0][0] : 0u, qhi[kc][2], QSPLIT ? qlo[QSPLIT ? kc : 0][2] : 0u};
                 mma_16816<BF16>(s[0], a, b0, b1);
@@ -698,14 +855,27 @@ __device__ __forceinline__ void decode_split_body(const DecodeParams& p, unsigne
 
         if (!mbar_wait(bar_full_v + 8 * st, par)) {
             wait_failed();
-            if constexpr (FUSED) continue; else return;
+            if constexpr (STAY) continue; else return;
+        }
+
+        if constexpr (CLUSTER) {
+            // Rows past the end of the sequence hold whatever the cache holds there: their probability is zero, but zero times
+            // a NaN is not. This warp's rows of the segment's last tile are cleared first (nobody else reads them).
+            const uint32_t row0 = (gt - seg.tile0) * TT + ts * 16;
+            if (row0 + 16 > seg.len) {
+                for (uint32_t c = lane; c < 16 * (D / 8); c += 32) {
+                    const uint32_t r = c / (D / 8), at = c & (D / 8 - 1);
+                    if (row0 + r >= seg.len) st_shared_zero16(vbase + hh * HEADB + (at >> 3) * PART + (ts * 16 + r) * 128 + (at & 7) * 16);
+                }
+                __syncwarp();
+            }
         }
 
         // ---- O += P V : 16 (heads) x D, contraction over this sub-tile's 16 rows ----
 #pragma unroll
         for (int d2 = 0; d2 < DN / 2; ++d2) {
             uint32_t b0, b1, b2, b3;
-            ldmatrix_x4_trans(b0, b1, b2, b3, vbase + v_lane_off + d2 * 32);
+            ldmatrix_x4_trans(b0, b1, b2, b3, v_addr(vbase, d2));
             if constexpr (PACK8) {
                 const uint32_t a[4] = {pa[0], pb[0], pa[2], pb[2]};
                 mma_16816<BF16>(o[2 * d2], a, b0, b1);
@@ -727,7 +897,11 @@ __device__ __forceinline__ void decode_split_body(const DecodeParams& p, unsigne
         if (lane == 0) mbar_arrive(bar_empty + 8 * st);
     }
     if (warp == 0 && lane == 0) DTRACE(5);
-    if (!failed) end_segment();
+    if constexpr (CLUSTER) {
+        cluster_merge();
+    } else {
+        if (!failed) end_segment();
+    }
     if (warp == 0 && lane == 0) DTRACE(6);
     fused_merge();
 #undef DTRACE

@@ -280,6 +280,46 @@ def test_residuals_in_the_idle_rows_against_products_of_their_own(attention, wl,
     assert int(ws.status.item()) == 0
 
 
+# One launch of clusters against the split pass and its merge (which a stated number of CTAs keeps): one to eight kv heads per
+# CTA, clusters of one to eight, sub-tiles shared by several warps, CTAs without a tile, empty sequences, odd query groups,
+# and NaN in the caches behind the valid rows.
+@pytest.mark.parametrize("B,H,Hkv,D,T,lens", [
+    (1, 32, 8, 128, 1, None), (1, 32, 4, 64, 512, None), (1, 8, 1, 128, 700, None), (2, 10, 5, 128, 333, [333, 0]),
+    (3, 21, 7, 64, 1111, [1, 1111, 64]), (6, 32, 8, 128, 1500, [374, 1499, 17, 1500, 0, 128]), (8, 16, 16, 64, 1000, None),
+    (8, 64, 8, 128, 700, [700, 1, 15, 16, 17, 333, 699, 32]), (12, 24, 12, 128, 129, None), (16, 32, 8, 128, 300, None),
+    (16, 32, 8, 128, 2100, None)])
+@pytest.mark.parametrize("q_dtype,kv_dtype,out", [("f32", "f16", "float32"), ("f16", "f16", "float16"), ("f32", "bf16", "bfloat16")])
+def test_cluster_form_against_the_split_form(attention, wl, B, H, Hkv, D, T, lens, q_dtype, kv_dtype, out):
+    import torch
+    from gpu_util import to_device
+    q, k, v = _rand(wl, B * 100 + H + T, B, H, Hkv, D, T, q_dtype, kv_dtype)
+    qd, kd, vd = to_device(q, q_dtype), to_device(k, kv_dtype), to_device(v, kv_dtype)
+    kv_len = None if lens is None else torch.tensor(lens, dtype=torch.int32, device="cuda")
+    for b, n in enumerate(lens or []):
+        kd[b, n:], vd[b, n:] = float("nan"), float("nan")
+    ws = attention.DecodeWorkspace(B, H, Hkv, D)
+    got, launches = [], []
+    for cap in (148, 0):
+        o = torch.empty((B, H, D), dtype=getattr(torch, out), device="cuda")
+        lse = torch.full((B, H), float("nan"), device="cuda")
+        before = attention.kernel_launch_count()
+        attention.attn_decode(qd, kd, vd, kv_len, out=o, lse=lse, workspace=ws, max_ctas=cap)
+        launches.append(attention.kernel_launch_count() - before)
+        got.append((o.double(), lse.double()))
+    assert launches == [2, 1]
+    (o0, l0), (o1, l1) = got
+    # fp32 sums in another order (2^-24 per addition, a few hundred of them at most), bf16 probabilities and residuals (2^-17),
+    # then the output type's own rounding
+    rms = float(o0.pow(2).mean().sqrt()) + 1e-30
+    step = {"float32": 0.0, "float16": 2.0 ** -10, "bfloat16": 2.0 ** -7}[out]
+    assert float((o0 - o1).abs().max()) <= 3e-5 * rms + step * float(o0.abs().max())
+    finite = torch.isfinite(l0)
+    assert torch.equal(finite, torch.isfinite(l1)) and float((l0 - l1)[finite].abs().max()) <= 2e-5
+    for b, n in enumerate(lens or []):
+        assert n > 0 or (bool((o1[b] == 0).all()) and bool(torch.isneginf(l1[b]).all()))
+    assert int(ws.status.item()) == 0
+
+
 def test_merge_entry_point(attention, wl, port):
     import torch
     q, k, v = wl.decode_inputs(wl.C4, kv_len=999)
