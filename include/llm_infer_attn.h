@@ -323,6 +323,30 @@ typedef struct AttnGemmPairArgs {
 } AttnGemmPairArgs;
 int attn_gemm_pair(const AttnGemmPairArgs* args, void* stream);
 
+/* Q8_0 weights without expanding them to an fp16 pair: q fp16 [rows][k] holds the blocks' int8 values (exact) and d
+ * fp16 [rows][pitch] their scales, pitch = k/32 rounded up to a multiple of 8 (attn_expand_q8_0 writes both).
+ * C[t][j] (+)= sum over blocks of fp32(d) * (sum_i (a_hi[t][i] + a_lo[t][i]) * q[j][i]): the tensor cores add up a block of
+ * 32, the scaled sums are added in fp32. Two MMAs per product in place of attn_gemm_pair's three, and a smaller error.
+ * With swiglu != 0 the matrix holds n_out gate rows followed by n_out up rows and the call writes silu(gate) * up as the fp16
+ * pair out_hi, out_lo [m][n_out]. k a multiple of 64; a_hi, a_lo, q, d 16-byte aligned. */
+typedef struct AttnGemmQ8Args {
+    float* c;            /* swiglu = 0: [m][ldc] fp32 */
+    void* out_hi;        /* swiglu = 1 */
+    void* out_lo;
+    const void* a_hi;    /* fp16 [m][k] */
+    const void* a_lo;    /* fp16 [m][k] */
+    const void* q;       /* fp16 [n_out][k], swiglu: [2 n_out][k] */
+    const void* d;       /* fp16 [n_out][pitch], swiglu: [2 n_out][pitch] */
+    uint64_t ldc;        /* floats between rows of c; 0 = n_out */
+    uint32_t m, n_out, k;
+    int32_t accumulate;
+    int32_t swiglu;
+    uint32_t* status;
+} AttnGemmQ8Args;
+int attn_gemm_q8_0(const AttnGemmQ8Args* args, void* stream);
+/* Q8_0 rows (GGML blocks, see attn_gemv_q8_0) -> q fp16 [rows][n] and d fp16 [rows][pitch] as attn_gemm_q8_0 reads them. */
+int attn_expand_q8_0(void* q, void* d, const void* w, uint64_t rows, uint32_t n, void* stream);
+
 /* Row-wise RMSNorm (include/kernels_cpu.hpp:43-67) of x [rows][dim] fp32, written as the fp16 pair hi, lo [rows][dim]. */
 int attn_rmsnorm_f16pair(void* hi, void* lo, const float* x, const float* weight, uint32_t rows, uint32_t dim, float eps,
                          void* stream);
@@ -450,7 +474,7 @@ uint64_t attn_kernel_launch_count(void);
 /* sizeof() of an argument structure as this library was compiled, so that a foreign-function binding can check its own
  * mirror of the layout: 0 AttnDecodeArgs, 1 AttnDecodeShardedArgs, 2 AttnPrefillArgs, 3 AttnRopeInsertArgs,
  * 4 AttnGemvArgs, 5 AttnMergeArgs, 6 AttnGemmArgs, 7 AttnRopePromptArgs,
- * 8 AttnGemmPairArgs; 0 for any other index. */
+ * 8 AttnGemmPairArgs, 9 AttnGemmQ8Args; 0 for any other index. */
 size_t attn_abi_struct_size(int which);
 
 #ifdef __cplusplus

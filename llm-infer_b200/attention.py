@@ -589,6 +589,58 @@ def gemm_pair(a_pair, w_pair, *, out, accumulate: bool = False, swiglu: bool = F
     return out
 
 
+def q8_planes(rows: int, n: int, device) -> tuple:
+    """Buffers for expand_q8_0: q fp16 [rows, n] and d fp16 [rows, n/32 rounded up to a multiple of 8]."""
+    return (torch.empty((rows, n), dtype=torch.float16, device=device),
+            torch.empty((rows, (n // 32 + 7) // 8 * 8), dtype=torch.float16, device=device))
+
+
+def expand_q8_0(w: torch.Tensor, *, out=None, stream=None):
+    """Q8_0 rows uint8 [rows, n/32*34] -> (q, d) as q8_planes() lays them out: the int8 values as fp16 numbers and the
+    scales of their blocks, which gemm_q8_0 multiplies."""
+    _require_cuda(w)
+    rows, n = w.shape[0], w.shape[1] // 34 * 32
+    if w.dtype != torch.uint8 or w.shape[1] % 34 or not w.is_contiguous():
+        raise ValueError("w must be dense uint8 [rows, n/32*34]")
+    q, d = q8_planes(rows, n, w.device) if out is None else out
+    if q.shape != (rows, n) or d.shape != (rows, (n // 32 + 7) // 8 * 8) or q.dtype != torch.float16 or \
+            d.dtype != torch.float16 or not (q.is_contiguous() and d.is_contiguous()):
+        raise ValueError("out must be the buffers of q8_planes(rows, n)")
+    _call("attn_expand_q8_0", w.device, stream, q.data_ptr(), d.data_ptr(), w.data_ptr(), rows, n)
+    return q, d
+
+
+def gemm_q8_0(a_pair, w_planes, *, out, accumulate: bool = False, swiglu: bool = False, status=None, stream=None):
+    """gemm_pair for Q8_0 weights as expand_q8_0 lays them out: a_pair = (a_hi, a_lo) fp16 [m, k], w_planes = (q, d). Same
+    outputs and forms as gemm_pair with two MMAs per product in place of three, and block sums added in fp32."""
+    (a_hi, a_lo), (q, d) = a_pair, w_planes
+    outs = tuple(out) if swiglu else (out,)
+    _require_cuda(a_hi, a_lo, q, d, *outs)
+    m, k = a_hi.shape
+    w_rows = q.shape[0]
+    n_out = w_rows // 2 if swiglu else w_rows
+    for group, shape in ((a_pair, (m, k)), ((q,), (w_rows, k)), ((d,), (w_rows, (k // 32 + 7) // 8 * 8)),
+                         (outs if swiglu else (), (m, n_out))):
+        for t in group:
+            if t.shape != shape or t.dtype != torch.float16 or not t.is_contiguous():
+                raise ValueError("dense fp16: a [m, k] twice, q [n_out, k], d as q8_planes() (swiglu: 2 n_out rows, out [m, n_out] twice)")
+    a = _b.AttnGemmQ8Args()
+    if swiglu:
+        if accumulate or w_rows % 2 or len(outs) != 2:
+            raise ValueError("swiglu needs gate rows and up rows, a pair as output and no accumulate")
+        a.out_hi, a.out_lo = outs[0].data_ptr(), outs[1].data_ptr()
+    else:
+        if out.shape != (m, n_out) or out.dtype != torch.float32 or out.stride(1) != 1:
+            raise ValueError("out must be fp32 [m, n_out] with dense rows")
+        a.c, a.ldc = out.data_ptr(), out.stride(0)
+    a.a_hi, a.a_lo, a.q, a.d = a_hi.data_ptr(), a_lo.data_ptr(), q.data_ptr(), d.data_ptr()
+    a.m, a.n_out, a.k = m, n_out, k
+    a.accumulate, a.swiglu = int(bool(accumulate)), int(bool(swiglu))
+    a.status = status.data_ptr() if status is not None else None
+    _call("attn_gemm_q8_0", a_hi.device, stream, C.byref(a))
+    return out
+
+
 def rmsnorm_pair(x: torch.Tensor, weight: torch.Tensor, eps: float, *, out=None, stream=None):
     """RMSNorm of every row of x [rows, dim] fp32, written as the fp16 (value, residual) pair that gemm_f16 reads."""
     _require_cuda(x, weight)

@@ -33,10 +33,12 @@ EXPORTED_SYMBOLS = (
     "attn_rope_kv_insert",
     "attn_gemm_f16",
     "attn_gemm_pair",
+    "attn_gemm_q8_0",
     "attn_rmsnorm_f16pair",
     "attn_split_f16pair",
     "attn_swiglu_f16pair",
     "attn_dequant_q8_0_f16pair",
+    "attn_expand_q8_0",
     "attn_rope_prompt",
     "attn_gather_rows",
     "attn_gemv_f16",
@@ -249,6 +251,25 @@ class AttnGemmPairArgs(C.Structure):
     ]
 
 
+class AttnGemmQ8Args(C.Structure):
+    _fields_ = [
+        ("c", C.c_void_p),
+        ("out_hi", C.c_void_p),
+        ("out_lo", C.c_void_p),
+        ("a_hi", C.c_void_p),
+        ("a_lo", C.c_void_p),
+        ("q", C.c_void_p),
+        ("d", C.c_void_p),
+        ("ldc", C.c_uint64),
+        ("m", C.c_uint32),
+        ("n_out", C.c_uint32),
+        ("k", C.c_uint32),
+        ("accumulate", C.c_int32),
+        ("swiglu", C.c_int32),
+        ("status", C.c_void_p),
+    ]
+
+
 class AttnRopePromptArgs(C.Structure):
     _fields_ = [
         ("q_out", C.c_void_p),
@@ -340,6 +361,10 @@ def load() -> C.CDLL:
     lib.attn_gemm_f16.argtypes = [C.POINTER(AttnGemmArgs), C.c_void_p]
     lib.attn_gemm_pair.restype = C.c_int
     lib.attn_gemm_pair.argtypes = [C.POINTER(AttnGemmPairArgs), C.c_void_p]
+    lib.attn_gemm_q8_0.restype = C.c_int
+    lib.attn_gemm_q8_0.argtypes = [C.POINTER(AttnGemmQ8Args), C.c_void_p]
+    lib.attn_expand_q8_0.restype = C.c_int
+    lib.attn_expand_q8_0.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_uint64, C.c_uint32, C.c_void_p]
     lib.attn_rmsnorm_f16pair.restype = C.c_int
     lib.attn_rmsnorm_f16pair.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_uint32, C.c_uint32, C.c_float,
                                          C.c_void_p]
@@ -360,7 +385,7 @@ def load() -> C.CDLL:
     lib.attn_abi_struct_size.restype = C.c_size_t
     lib.attn_abi_struct_size.argtypes = [C.c_int]
     mirrors = (AttnDecodeArgs, AttnDecodeShardedArgs, AttnPrefillArgs, AttnRopeInsertArgs, AttnGemvArgs, AttnMergeArgs,
-               AttnGemmArgs, AttnRopePromptArgs, AttnGemmPairArgs)
+               AttnGemmArgs, AttnRopePromptArgs, AttnGemmPairArgs, AttnGemmQ8Args)
     for index, mirror in enumerate(mirrors):
         if lib.attn_abi_struct_size(index) != C.sizeof(mirror):
             raise RuntimeError(f"{mirror.__name__}: the ctypes mirror ({C.sizeof(mirror)} bytes) does not match the "

@@ -301,6 +301,7 @@ size_t attn_abi_struct_size(int which) {
         case 6: return sizeof(AttnGemmArgs);
         case 7: return sizeof(AttnRopePromptArgs);
         case 8: return sizeof(AttnGemmPairArgs);
+        case 9: return sizeof(AttnGemmQ8Args);
         default: return 0;
     }
 }

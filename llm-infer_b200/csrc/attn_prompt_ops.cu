@@ -5,7 +5,8 @@
 //   rmsnorm rows            -> activations as an fp16 value / fp16 residual pair of matrices (the GEMM's A operand)
 //   fp32 rows               -> the same pair (attention output before the output projection)
 //   stacked gate | up rows  -> silu(gate) * up as that pair (src/model/block.cpp:198-210)
-//   Q8_0 weight rows        -> fp16 value / residual pair (scale x int8 has up to 18 significant bits)
+//   Q8_0 weight rows        -> fp16 value / residual pair (scale x int8 has up to 18 significant bits), or the int8 values
+//                              as fp16 and the scales apart (attn_gemm_q8_0)
 //   rotary embedding of every token's q and k, fp16 insert of k and v into the token's cache row
 //                              (src/model/block.cpp:140-148 per token)
 //   row gather                 (the last token of every prompt continues into the classifier)
@@ -126,6 +127,33 @@ __global__ void __launch_bounds__(kRowThreads) dequant_q8_pair_kernel(__half* hi
         oh[1] = make_uint2(h[2], h[3]);
         ol[0] = make_uint2(l[0], l[1]);
         ol[1] = make_uint2(l[2], l[3]);
+    }
+}
+
+// Q8_0 blocks -> the int8 values as fp16 numbers (exact) and the blocks' scales, [rows][pitch]: what attn_gemm_q8_0
+// multiplies. One 16-byte store per thread and eight values; a block's first thread also copies its scale.
+__global__ void __launch_bounds__(kRowThreads) expand_q8_kernel(__half* q, uint16_t* d, const uint8_t* w, size_t n_eighths,
+                                                                uint32_t row_blocks, uint32_t pitch) {
+    grid_dep_launch_dependents();
+    grid_dep_wait();
+    for (size_t e = static_cast<size_t>(blockIdx.x) * kRowThreads + threadIdx.x; e < n_eighths;
+         e += static_cast<size_t>(gridDim.x) * kRowThreads) {
+        const size_t b = e >> 2;
+        // a block starts at an even address: 2-byte loads
+        const unsigned short* blk = reinterpret_cast<const unsigned short*>(w + b * 34);
+        const unsigned short* q16 = blk + 1 + 4 * (e & 3);
+        uint32_t h[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const unsigned short a = q16[i];
+            const __half2 hh = __halves2half2(__short2half_rn(static_cast<int8_t>(a & 0xff)), __short2half_rn(static_cast<int8_t>(a >> 8)));
+            h[i] = *reinterpret_cast<const uint32_t*>(&hh);
+        }
+        *reinterpret_cast<uint4*>(q + e * 8) = make_uint4(h[0], h[1], h[2], h[3]);
+        if ((e & 3) == 0) {
+            const size_t r = b / row_blocks;
+            d[r * pitch + (b - r * row_blocks)] = blk[0];
+        }
     }
 }
 
@@ -263,6 +291,18 @@ int attn_dequant_q8_0_f16pair(void* hi, void* lo, const void* w, uint64_t rows, 
     B200_CUDA_TRY(launch_dependent(dequant_q8_pair_kernel, dim3(stream_grid(n_eighths)), dim3(kRowThreads), 0,
                                    static_cast<cudaStream_t>(stream), static_cast<__half*>(hi), static_cast<__half*>(lo),
                                    static_cast<const uint8_t*>(w), n_eighths));
+    count_launch();
+    return ATTN_OK;
+}
+
+int attn_expand_q8_0(void* q, void* d, const void* w, uint64_t rows, uint32_t n, void* stream) {
+    if (!q || !d || !w || rows == 0 || n == 0) return ATTN_ERR_INVALID_ARG;
+    if (n % 32 != 0) return ATTN_ERR_UNSUPPORTED;
+    if (!aligned(q, 16) || !aligned(d, 16) || !aligned(w, 2)) return ATTN_ERR_ALIGNMENT;
+    const size_t n_eighths = static_cast<size_t>(rows) * (n / 8);
+    B200_CUDA_TRY(launch_dependent(expand_q8_kernel, dim3(stream_grid(n_eighths)), dim3(kRowThreads), 0,
+                                   static_cast<cudaStream_t>(stream), static_cast<__half*>(q), static_cast<uint16_t*>(d),
+                                   static_cast<const uint8_t*>(w), n_eighths, n / 32, (n / 32 + 7) & ~7u));
     count_launch();
     return ATTN_OK;
 }

@@ -236,8 +236,9 @@ class Llama:
 
     def prefill(self, prompts, exact: bool = True) -> None:
         """The prompt phase for all sequences at once instead of one token per step: the tokens of every prompt are
-        packed into one matrix of rows; per layer one tensor-core GEMM per projection (attn_gemm_pair, the SwiGLU product as
-        its epilogue; Q8_0 weights are expanded per matrix into an fp16 value / residual pair first), the rotary kernel that also fills the KV caches,
+        packed into one matrix of rows; per layer one tensor-core GEMM per projection (attn_gemm_pair, for Q8_0 weights
+        attn_gemm_q8_0 over the matrix's int8 values as fp16 and its scales, which a pass in front writes; the SwiGLU product as
+        the epilogue), the rotary kernel that also fills the KV caches,
         causal attention per sequence (attn_prefill_causal straight over that sequence's cache rows), and the
         row-wise norm / SwiGLU steps. Per token this is the engine's forward pass (src/model/block.cpp:105-223) with
         InferenceMode::Prefill for all but the last token of a prompt (src/model/model.cpp:74-76); the last tokens go
@@ -269,15 +270,23 @@ class Llama:
         qkv = e(T, q_dim + 2 * kv_dim)
         q16 = e(T, H, D, dtype=f16)
         att = e(T, H, D)
-        if q8:  # room for the largest matrix of a layer as an fp16 pair
-            biggest = max(w[k].shape[1] * (w[k].shape[2] // 34 * 32) for k in ("wqkv", "wo", "w13", "w2"))
-            w_hi, w_lo = e(biggest, dtype=f16), e(biggest, dtype=f16)
+        if q8:  # room for the largest matrix of a layer: its int8 values as fp16 and its scales, or an fp16 pair
+            shapes = [(w[k].shape[1], w[k].shape[2] // 34 * 32) for k in ("wqkv", "wo", "w13", "w2")]
+            biggest = max(rows * n for rows, n in shapes)
+            w_a = e(biggest, dtype=f16)
+            w_b = e(max(rows * ((n // 32 + 7) // 8 * 8) for rows, n in shapes) if exact else biggest, dtype=f16)
 
         def project(a_pair, wmat, out, **kw):
+            if q8 and exact:
+                rows, n, pitch = wmat.shape[0], wmat.shape[1] // 34 * 32, (wmat.shape[1] // 34 + 7) // 8 * 8
+                planes = (w_a[:rows * n].view(rows, n), w_b[:rows * pitch].view(rows, pitch))
+                A.expand_q8_0(wmat, out=planes)
+                A.gemm_q8_0(a_pair, planes, out=out, status=self.status, **kw)
+                return
             w_pair = (wmat, None)
             if q8:
                 rows, n = wmat.shape[0], wmat.shape[1] // 34 * 32
-                w_pair = (w_hi[:rows * n].view(rows, n), w_lo[:rows * n].view(rows, n))
+                w_pair = (w_a[:rows * n].view(rows, n), w_b[:rows * n].view(rows, n))
                 A.dequant_q8_0_pair(wmat, out=w_pair)
             if not exact:
                 a_pair, w_pair = (a_pair[0], None), (w_pair[0], None)

@@ -145,6 +145,54 @@ def test_gemm_several_tiles_per_cta(A, m, n_out, k, form):
     assert int(status.item()) == 0
 
 
+def _q8_blocks(g, rows, k):
+    import torch
+    q = torch.randint(-127, 128, (rows, k // 32, 32), generator=g, device="cuda", dtype=torch.int8)
+    d = (torch.rand((rows, k // 32, 1), generator=g, device="cuda") * k ** -0.5 / 64).half()
+    blocks = torch.empty((rows, k // 32, 34), dtype=torch.uint8, device="cuda")
+    blocks[..., :2], blocks[..., 2:] = d.view(torch.uint8), q.view(torch.uint8)
+    return blocks.view(rows, -1), (d.double() * q.double()).view(rows, k)
+
+
+# Rows and tokens around the tiles (64 and 128 tokens, 128 to 512 rows), k of two blocks, an odd number of block pairs and
+# no multiple of eight blocks, several tiles per CTA over several bands; all forms: one or two row parts, single CTAs and pairs.
+@pytest.mark.parametrize("m,n_out,k", [(1, 1, 64), (63, 130, 192), (128, 512, 256), (129, 513, 320), (700, 1056, 512),
+                                       (2500, 6200, 64), (9000, 520, 128), (500, 416, 14336), (40, 20000, 64)])
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_gemm_q8_0_against_float64(A, m, n_out, k, swiglu):
+    """attn_expand_q8_0 exactly, and attn_gemm_q8_0 against float64: a block's sum is cut once per MMA of 16 (four of them,
+    2^-23 of it at most), and the scaled sums of k / 32 blocks are rounded once each in fp32."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(m + n_out + k)
+    w, w64 = _q8_blocks(g, n_out * (2 if swiglu else 1), k)
+    q, d = A.expand_q8_0(w)
+    assert torch.equal((q.view(-1, k // 32, 32).double() * d[:, :k // 32, None].double()).view(-1, k), w64)
+    x = torch.randn((m, k), generator=g, device="cuda")
+    a = (x.half(), (x - x.half().float()).half())
+    a64 = a[0].double() + a[1].double()
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    prod = a64 @ w64.T
+    # k / 32 additions, each off by 2^-24 of the running sum at most, and 4 * 2^-23 of the blocks' sums; a running sum of terms
+    # of random sign stays within four of its standard deviations, |a| |w| / sqrt(k), or the largest result
+    sums = max(float(prod.abs().max()), 4 * float(a64.norm(dim=1).max() * w64.norm(dim=1).max()) * k ** -0.5)
+    tol = (k / 32 * 2.0 ** -24 + 2.0 ** -20) * sums
+    if swiglu:
+        out = tuple(torch.full((m, n_out), float("nan"), dtype=torch.float16, device="cuda") for _ in range(2))
+        A.gemm_q8_0(a, (q, d), out=out, swiglu=True, status=status)
+        gate, up = prod[:, :n_out], prod[:, n_out:]
+        want = gate / (1 + torch.exp(-gate)) * up
+        bound = 1.1 * tol * (up.abs() + gate.abs()) + 2.0 ** -20 * want.abs() + 2.0 ** -24
+        assert bool(((out[0].double() + out[1].double() - want).abs() <= bound).all())
+    else:
+        wide = torch.zeros((m, n_out + 3), device="cuda")
+        A.gemm_q8_0(a, (q, d), out=wide[:, :n_out], status=status)
+        assert float((wide[:, :n_out].double() - prod).abs().max()) <= tol
+        assert bool((wide[:, n_out:] == 0).all()), "nothing written past the row"
+        A.gemm_q8_0(a, (q, d), out=wide[:, :n_out], accumulate=True, status=status)
+        assert float((wide[:, :n_out].double() - 2 * prod).abs().max()) <= 3 * tol
+    assert int(status.item()) == 0
+
+
 def test_gemm_rows_equal_the_engine_matmul(A, checker):
     """Each token's row of the GEMM against the engine's own per-token matmul() on the fp32 activations."""
     import torch
