@@ -261,22 +261,18 @@ def test_max_ctas_limits_split_without_changing_result(attention, wl, checker):
 @pytest.mark.parametrize("H,Hkv,D", [(8, 8, 128), (21, 3, 64), (64, 8, 128), (16, 2, 64), (18, 2, 128)])
 @pytest.mark.parametrize("q_dtype,kv_dtype", [("f32", "f16"), ("f16", "f16"), ("f32", "bf16")])
 def test_residuals_in_the_idle_rows_against_products_of_their_own(attention, wl, H, Hkv, D, q_dtype, kv_dtype):
-    """Up to eight heads per kv head the residual products take the MMAs' rows 8-15; with a prepared output (and with more
-    heads) they are products of their own. Same sums in another order: fp32 rounding (2^-24 each, a few hundred), bf16
-    probabilities and residuals (2^-17), and the prepared form's 2^-21."""
+    """Up to eight heads per kv head the residual products take the MMAs' rows 8-15; in a generation step (kv_early, lengths
+    on the device) and with more heads they are products of their own. Same sums in another order: fp32 rounding (2^-24 each,
+    a few hundred), bf16 probabilities and residuals (2^-17)."""
     import torch
     from gpu_util import to_device
     q, k, v = _rand(wl, H + D, 3, H, Hkv, D, 777, q_dtype, kv_dtype)
     qd, kd, vd = to_device(q, q_dtype), to_device(k, kv_dtype), to_device(v, kv_dtype)
+    lens = torch.tensor([777, 16, 500], dtype=torch.int32, device="cuda")
     ws = attention.DecodeWorkspace(3, H, Hkv, D)
-    plain = attention.attn_decode(qd, kd, vd, workspace=ws, max_ctas=148).double()
-    words = torch.empty((3, H, D), dtype=torch.int32, device="cuda")
-    attention.attn_decode(qd, kd, vd, out=words, workspace=ws)
-    # words {hi(x0,x1), hi(x2,x3), lo(x0,x1), lo(x2,x3)} of four elements
-    h = words.view(torch.float16).view(3, H, D // 4, 2, 4).double()
-    prepared = (h[..., 0, :] + h[..., 1, :]).reshape(3, H, D)
-    rms = float(plain.pow(2).mean().sqrt())
-    assert float((plain - prepared).abs().max()) <= 3e-5 * rms + 2.0 ** -21 * float(plain.abs().max())
+    rows = attention.attn_decode(qd, kd, vd, lens, workspace=ws, max_ctas=148).double()
+    own = attention.attn_decode(qd, kd, vd, lens, workspace=ws, kv_early=True).double()
+    assert float((rows - own).abs().max()) <= 3e-5 * float(rows.pow(2).mean().sqrt())
     assert int(ws.status.item()) == 0
 
 
