@@ -106,7 +106,8 @@ typedef struct AttnDecodeArgs {
                           every tile that cannot hold that row before it waits for the previous kernel. 0 = wait first. */
     uint32_t kv_capacity; /* rows each sequence's caches hold (the engine's max_seq_len); 0 = not stated. When stated, a
                              length beyond it (a corrupted kv_len[] entry) is clamped to it on the device and
-                             ATTN_STATUS_BAD_SHAPE is ORed into *status, instead of reading past the cache. */
+                             ATTN_STATUS_BAD_SHAPE is ORed into *status, instead of reading past the cache. All
+                             stated rows must be readable; those behind kv_len may hold anything. */
 } AttnDecodeArgs;
 
 /* Scratch size for attn_decode with these dimensions on the current device. */
