@@ -94,7 +94,7 @@ typedef struct AttnDecodeArgs {
     uint64_t kv_row_stride;   /* elements between rows; 0 = n_kv_heads*head_dim */
     uint64_t kv_batch_stride; /* elements between sequences; may be 0 only when batch == 1 */
     float scale;              /* 0 = 1/sqrt(head_dim), as kernels_cpu.hpp:152 */
-    uint32_t max_ctas;        /* upper bound on the CTAs that share the KV rows; 0 = auto */
+    uint32_t max_ctas;        /* upper bound on the CTAs that share the KV rows; 0 = auto (see two_pass) */
     void* workspace;          /* device scratch, >= attn_decode_workspace_bytes(), 16-byte aligned */
     size_t workspace_bytes;
     uint32_t* status; /* optional device word, ATTN_STATUS_* bits are ORed in; NULL to skip */
@@ -108,12 +108,16 @@ typedef struct AttnDecodeArgs {
                              length beyond it (a corrupted kv_len[] entry) is clamped to it on the device and
                              ATTN_STATUS_BAD_SHAPE is ORed into *status, instead of reading past the cache. All
                              stated rows must be readable; those behind kv_len may hold anything. */
+    uint32_t two_pass; /* 0 = the fastest form for the shape, chosen by batch, heads, head_dim, kv_len_uniform or kv_capacity and
+                          max_ctas (a stated max_ctas always means the two launches). != 0: always the split pass and the merge
+                          pass, with every residual product an MMA of its own: one order of the sums for all capacities and
+                          group sizes. In either case neither kv_early nor o_dtype changes a bit of the result. */
 } AttnDecodeArgs;
 
 /* Scratch size for attn_decode with these dimensions on the current device. */
 size_t attn_decode_workspace_bytes(uint32_t batch, uint32_t n_heads, uint32_t n_kv_heads, uint32_t head_dim);
 
-/* Enqueue: split-KV pass (per-CTA partial O and LSE) + merge pass. */
+/* Enqueue: one launch of clusters, or split-KV pass (per-CTA partial O and LSE) + merge pass (see two_pass). */
 int attn_decode(const AttnDecodeArgs* args, void* stream);
 
 /* Causal prefill attention of whole prompts. The engine has no such kernel: its prefill is the decode step

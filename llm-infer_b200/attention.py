@@ -80,7 +80,7 @@ class DecodeWorkspace:
 
 
 def _decode_args(q, k_cache, v_cache, kv_len, out, lse, out_dtype, scale, workspace, max_ctas, stream=None,
-                 kv_early=False):
+                 kv_early=False, two_pass=False):
     """Validates the operands of a decode call and fills the C struct. Returns (args, out, workspace)."""
     _require_cuda(q, k_cache, v_cache)
     B, H, D = q.shape
@@ -111,19 +111,20 @@ def _decode_args(q, k_cache, v_cache, kv_len, out, lse, out_dtype, scale, worksp
             raise ValueError("kv_len must be an int32 CUDA tensor of shape [B]")
         kv_ptr, uniform = kv_len.data_ptr(), 0
     batch_stride, row_stride = k_cache.stride(0), k_cache.stride(1)
-    # (one positional construction: setting 23 fields by name costs three times as much)
+    # (one positional construction: setting 25 fields by name costs three times as much)
     a = _b.AttnDecodeArgs(
         out.data_ptr(), q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), lse.data_ptr() if lse is not None else None,
         _dtype_code(out), _dtype_code(q), _dtype_code(k_cache), B, H, Hkv, D, kv_ptr, uniform, row_stride,
         batch_stride if B > 1 else max(batch_stride, 0), float(scale), int(max_ctas), workspace.buf.data_ptr(),
         workspace.nbytes, workspace.status.data_ptr(), int(bool(kv_early)),
-        T)  # a device-side length beyond the cache is clamped and reported (ATTN_STATUS_BAD_SHAPE)
+        T,  # a device-side length beyond the cache is clamped and reported (ATTN_STATUS_BAD_SHAPE)
+        int(bool(two_pass)))
     return a, out, workspace, q
 
 
 def attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, kv_len=None, *, out=None, lse=None,
                 out_dtype=torch.float32, scale: float = 0.0, workspace: DecodeWorkspace | None = None,
-                max_ctas: int = 0, kv_early: bool = False, stream=None) -> torch.Tensor:
+                max_ctas: int = 0, kv_early: bool = False, two_pass: bool = False, stream=None) -> torch.Tensor:
     """Single-token attention of every query head over its sequence's KV cache.
 
     q        [B, H, D]        fp32 / fp16 / bf16, already rotated
@@ -133,10 +134,13 @@ def attn_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, k
              on the device: one beyond T is clamped to T there and sets ATTN_STATUS_BAD_SHAPE in workspace.status
     kv_early True when the lengths were in place before the previous kernel of the stream was launched and that kernel
              writes no K/V row other than each sequence's last valid one: streaming then starts before it has finished
+    max_ctas upper bound on the CTAs that share the KV rows (0: chosen here); any bound means the two launches
+    two_pass True: always the split pass and the merge pass with residual products of their own, whose order of sums does not
+             change with T or the heads; False: the fastest form for the shape. kv_early and out's type never change the sums
     returns  out [B, H, D] in out_dtype; fills ``lse`` [B, H] (fp32) when given
     """
     a, out, _, _q = _decode_args(q, k_cache, v_cache, kv_len, out, lse, out_dtype, scale, workspace, max_ctas, stream,
-                                 kv_early)
+                                 kv_early, two_pass)
     _call("attn_decode", out.device, stream, C.byref(a))
     return out
 

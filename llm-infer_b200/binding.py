@@ -116,6 +116,7 @@ class AttnDecodeArgs(C.Structure):
         ("status", C.c_void_p),
         ("kv_early", C.c_uint32),
         ("kv_capacity", C.c_uint32),
+        ("two_pass", C.c_uint32),
     ]
 
 

@@ -152,14 +152,12 @@ int decode_impl(const AttnDecodeArgs* a, void* stream_v, const Exchange* xchg) {
     const bool qsplit = a->q_dtype != ATTN_DTYPE_F16;
     // Up to eight query heads per kv head leave half of the MMAs' rows to the residual products (decode_body.cuh, PACK8): 7
     // sequences up to 2999 rows 18.6 -> 16.2 us, 8 x 2048 19.1 -> 17.6, 16 x 4096 49.3 -> 46.9 (graphs of calls). Sums come out in
-    // another order. The call between the layers of a generation step (kv_early, lengths on the device, prepared output) keeps the
-    // form without, and the two launches below: the sums' order decides ties of the following layers' fp16 cache rows, and a
-    // step's results (cache rows, picked tokens) stay what they were bit for bit.
-    const bool step = a->kv_early != 0 && a->kv_len != nullptr && a->o_dtype == ATTN_DTYPE_SPLIT16;
-    p.pack8 = plan.group <= 8 && !step ? 1u : 0u;
+    // another order; two_pass keeps the form without, and the two launches below.
+    const bool two_pass = a->two_pass != 0;
+    p.pack8 = plan.group <= 8 && !two_pass ? 1u : 0u;
     const uint32_t rows = a->kv_len ? a->kv_capacity : clamped_len(a->kv_len_uniform, a->kv_capacity);
     DecodeClusterPlan cl{};
-    if (!xchg && !step && a->max_ctas == 0 &&
+    if (!xchg && !two_pass && a->max_ctas == 0 &&
         pick_decode_cluster(a->batch, a->n_heads, a->n_kv_heads, a->head_dim, rows, a->kv_len != nullptr, dev, &cl)) {
         DecodeParams c = p;
         c.head_groups = a->n_kv_heads / cl.hpc;

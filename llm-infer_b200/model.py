@@ -208,8 +208,10 @@ class Llama:
             A.rope_kv_insert(self.q, self.k, self.v, self.k_cache[l], self.v_cache[l], self.pos, self.kv_pos,
                              theta=c.rope_theta, rotary_dim=c.rotary_dim, kv_sink=kv_sink, q_out=self.q,
                              pos_early=True)   # positions are copied in before the step's first kernel
+            # (two_pass: another order of the sums moves fp16 ties of the next layers' cache rows, so a step's results would
+            # change with max_seq_len, which the choice of the form looks at)
             A.attn_decode(self.q, self.k_cache[l], self.v_cache[l], self.kv_len, out=self.att,
-                          workspace=self.workspace, kv_early=self.kv_early)
+                          workspace=self.workspace, kv_early=self.kv_early, two_pass=True)
             gemv(att_flat, "wo", l, out=self.x, accumulate=True)           # x += Wo att
             A.rmsnorm(self.x, w["rms_ffn"][l], c.norm_eps, out=self.xb)
             gemv(self.xb, "w13", l, out=self.hb, swiglu=True)              # hb = silu(W1 xb) * (W3 xb)

@@ -261,9 +261,9 @@ def test_max_ctas_limits_split_without_changing_result(attention, wl, checker):
 @pytest.mark.parametrize("H,Hkv,D", [(8, 8, 128), (21, 3, 64), (64, 8, 128), (16, 2, 64), (18, 2, 128)])
 @pytest.mark.parametrize("q_dtype,kv_dtype", [("f32", "f16"), ("f16", "f16"), ("f32", "bf16")])
 def test_residuals_in_the_idle_rows_against_products_of_their_own(attention, wl, H, Hkv, D, q_dtype, kv_dtype):
-    """Up to eight heads per kv head the residual products take the MMAs' rows 8-15; in a generation step (kv_early, lengths
-    on the device, prepared output) and with more heads they are products of their own. Same sums in another order: fp32
-    rounding (2^-24 each, a few hundred), bf16 probabilities and residuals (2^-17), and the prepared form's 2^-21."""
+    """Up to eight heads per kv head the residual products take the MMAs' rows 8-15; with two_pass and with more heads they are
+    products of their own. Same sums in another order: fp32 rounding (2^-24 each, a few hundred) and bf16 probabilities and
+    residuals (2^-17)."""
     import torch
     from gpu_util import to_device
     q, k, v = _rand(wl, H + D, 3, H, Hkv, D, 777, q_dtype, kv_dtype)
@@ -271,12 +271,34 @@ def test_residuals_in_the_idle_rows_against_products_of_their_own(attention, wl,
     lens = torch.tensor([777, 16, 500], dtype=torch.int32, device="cuda")
     ws = attention.DecodeWorkspace(3, H, Hkv, D)
     rows = attention.attn_decode(qd, kd, vd, lens, workspace=ws, max_ctas=148).double()
-    words = torch.empty((3, H, D), dtype=torch.int32, device="cuda")
-    attention.attn_decode(qd, kd, vd, lens, out=words, workspace=ws, kv_early=True)
-    # words {hi(x0,x1), hi(x2,x3), lo(x0,x1), lo(x2,x3)} of four elements
-    h = words.view(torch.float16).view(3, H, D // 4, 2, 4).double()
-    own = (h[..., 0, :] + h[..., 1, :]).reshape(3, H, D)
-    assert float((rows - own).abs().max()) <= 3e-5 * float(rows.pow(2).mean().sqrt()) + 2.0 ** -21 * float(rows.abs().max())
+    own = attention.attn_decode(qd, kd, vd, lens, workspace=ws, two_pass=True).double()
+    assert float((rows - own).abs().max()) <= 3e-5 * float(rows.pow(2).mean().sqrt())
+    assert int(ws.status.item()) == 0
+
+
+@pytest.mark.parametrize("two_pass", [False, True])
+@pytest.mark.parametrize("H,Hkv,D,T,lens", [(32, 8, 128, 700, [700, 33, 257]), (32, 8, 128, 40000, [40000, 5, 12345]),
+                                            (8, 2, 64, 300, [1, 300, 0]), (18, 2, 128, 333, [333, 17, 48])])
+def test_neither_the_early_start_nor_the_output_type_changes_the_sums(attention, wl, H, Hkv, D, T, lens, two_pass):
+    """kv_early and the type of the result are no part of the choice between the forms: fp32 results are equal bit for bit, and
+    prepared words are the exact split of them. (Short contexts take the clusters, long ones and two_pass the two launches.)"""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(H + T)
+    q = torch.randn((3, H, D), generator=g, device="cuda")
+    k, v = (torch.randn((3, T, Hkv, D), generator=g, device="cuda").half() for _ in range(2))
+    kv_len = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    ws = attention.DecodeWorkspace(3, H, Hkv, D)
+    plain = attention.attn_decode(q, k, v, kv_len, workspace=ws, two_pass=two_pass)
+    x = plain.clamp(-65504, 65504)
+    hi = x.half()
+    lo = (x - hi.float()).half()
+    pairs = torch.stack([t.view(torch.int16).view(3, H, D // 4, 4) for t in (hi, lo)], dim=3)  # four values, then their residuals
+    want = pairs.contiguous().view(torch.int32).view(3, H, D)
+    for early in (False, True):
+        words = torch.empty((3, H, D), dtype=torch.int32, device="cuda")
+        attention.attn_decode(q, k, v, kv_len, out=words, workspace=ws, kv_early=early, two_pass=two_pass)
+        assert torch.equal(words, want), early
+    assert torch.equal(attention.attn_decode(q, k, v, kv_len, workspace=ws, kv_early=True, two_pass=two_pass), plain)
     assert int(ws.status.item()) == 0
 
 
