@@ -139,9 +139,10 @@ class Llama:
         self.next_token = z(B, dtype=torch.int32)
         self.tokens = z(B, dtype=torch.int32)   # the step's input tokens; a decode step writes its picks back here
         self._graphs = None
-        # The lengths are copied in before a step's first kernel and the kernel in front of the attention (rotary +
-        # insert) writes only each sequence's newest row: the attention may start streaming the older rows early
-        # (measured: 3.03 -> 3.00 ms per step of the 8B-shaped Q8_0 model at batch 8).
+        # The lengths are copied in before a step's first kernel and, outside the sliding window, the kernel in front of the
+        # attention (rotary + insert) writes only each sequence's newest row, its last valid one: the attention may start
+        # streaming the older rows early (measured: 3.03 -> 3.00 ms per step of the 8B-shaped Q8_0 model at batch 8). In the
+        # window that kernel writes a row inside the ring and all sink rows, so there the attention waits for it.
         self.kv_early = True
         self._positions = z(3, B, dtype=torch.int32)  # one buffer, so that a step copies its positions in at once
         self.pos, self.kv_pos, self.kv_len = self._positions.unbind(0)
@@ -211,7 +212,7 @@ class Llama:
             # (two_pass: another order of the sums moves fp16 ties of the next layers' cache rows, so a step's results would
             # change with max_seq_len, which the choice of the form looks at)
             A.attn_decode(self.q, self.k_cache[l], self.v_cache[l], self.kv_len, out=self.att,
-                          workspace=self.workspace, kv_early=self.kv_early, two_pass=True)
+                          workspace=self.workspace, kv_early=self.kv_early and kv_sink == 0, two_pass=True)
             gemv(att_flat, "wo", l, out=self.x, accumulate=True)           # x += Wo att
             A.rmsnorm(self.x, w["rms_ffn"][l], c.norm_eps, out=self.xb)
             gemv(self.xb, "w13", l, out=self.hb, swiglu=True)              # hb = silu(W1 xb) * (W3 xb)

@@ -43,3 +43,11 @@ def test_every_step_asks_for_the_form_with_one_order_of_sums(step, weight_type):
     """Whatever the weights: the order of the attention's sums decides fp16 ties of the next layers' cache rows."""
     attention = [kw for name, kw in step(weight_type, 0) if name == "attn_decode"]
     assert len(attention) == 2 and all(kw["two_pass"] for kw in attention)
+
+
+@pytest.mark.parametrize("kv_sink", [0, 4])
+def test_early_streaming_stops_at_the_sliding_window(step, kv_sink):
+    """In the window the rotary kernel writes a row inside the ring and turns the sink rows: no row may be read before it."""
+    calls = step("f16", kv_sink)
+    assert [kw["kv_sink"] for name, kw in calls if name == "rope_kv_insert"] == [kv_sink] * 2
+    assert [bool(kw["kv_early"]) for name, kw in calls if name == "attn_decode"] == [kv_sink == 0] * 2
