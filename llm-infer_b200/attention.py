@@ -116,9 +116,9 @@ def _decode_args(q, k_cache, v_cache, kv_len, out, lse, out_dtype, scale, worksp
         out.data_ptr(), q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), lse.data_ptr() if lse is not None else None,
         _dtype_code(out), _dtype_code(q), _dtype_code(k_cache), B, H, Hkv, D, kv_ptr, uniform, row_stride,
         batch_stride if B > 1 else max(batch_stride, 0), float(scale), int(max_ctas), workspace.buf.data_ptr(),
-        workspace.nbytes, workspace.status.data_ptr(), int(bool(kv_early)),
+        workspace.nbytes, workspace.status.data_ptr(), 1 if kv_early else 0,
         T,  # a device-side length beyond the cache is clamped and reported (ATTN_STATUS_BAD_SHAPE)
-        int(bool(two_pass)))
+        1 if two_pass else 0)
     return a, out, workspace, q
 
 

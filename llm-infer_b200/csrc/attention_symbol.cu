@@ -197,8 +197,7 @@ int attention_configure(uint32_t n_heads, uint32_t n_kv_heads, uint32_t head_dim
     B200_CUDA_TRY(cudaMemsetAsync(c.group_counters, 0, plan.group_counter_words * 4, stream));
     B200_CUDA_TRY(cudaMemcpyToSymbolAsync(g_cfg, &c, sizeof(c), 0, cudaMemcpyHostToDevice, stream));
     B200_CUDA_TRY(cudaStreamSynchronize(stream));  // c lives on this stack frame
-    B200_CUDA_TRY(cudaFuncSetAttribute(attention, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(plan.smem_bytes)));
+    B200_CUDA_TRY(allow_max_smem(attention));
     g_host_cfg[dev].ok = true;
     g_host_cfg[dev].grid = plan.grid;
     g_host_cfg[dev].smem = static_cast<uint32_t>(plan.smem_bytes);

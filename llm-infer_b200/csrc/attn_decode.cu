@@ -18,8 +18,7 @@ __global__ void __launch_bounds__(kThreads, 1) decode_split_kernel(const __grid_
 template <int D, int HPC, bool QSPLIT, bool BF16>
 int launch_one(const DecodeParams& p, uint32_t grid, size_t smem_bytes, cudaStream_t stream) {
     auto kernel = p.pack8 ? decode_split_kernel<D, HPC, QSPLIT, BF16, true> : decode_split_kernel<D, HPC, QSPLIT, BF16, false>;
-    B200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(smem_bytes)));
+    B200_CUDA_TRY(allow_max_smem(kernel));
     // launched as a programmatic dependent: the launch overlaps the previous kernel's tail; the kernel waits for that
     // kernel before it reads anything
     B200_CUDA_TRY(launch_dependent(kernel, dim3(grid), dim3(kThreads), smem_bytes, stream, p));

@@ -437,7 +437,7 @@ int launch_gemm(GemmParams& p, const void* a_hi, const void* a_lo, const void* w
                    : (wlo ? gemm_f16_kernel<P, false, true> : gemm_f16_kernel<P, false, false>);
     };
     auto kernel = t.pair ? pick(std::true_type{}) : pick(std::false_type{});
-    B200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    B200_CUDA_TRY(allow_max_smem(kernel));
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kGemmThreads);

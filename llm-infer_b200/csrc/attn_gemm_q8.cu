@@ -525,7 +525,7 @@ extern "C" int attn_gemm_q8_0(const AttnGemmQ8Args* a, void* stream_v) {
                             : (t.n_tile == 128 ? gemm_q8_kernel<P, 1, 128> : gemm_q8_kernel<P, 1, 64>);
     };
     auto kernel = t.pair ? pick(std::true_type{}) : pick(std::false_type{});
-    B200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    B200_CUDA_TRY(allow_max_smem(kernel));
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kThreads);

@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(kGemvThreads, 1) gemv_f16_kernel(const __grid_
 template <int BATCH>
 int launch_gemv(const GemvParams& p, int sm_count, size_t smem, cudaStream_t stream) {
     auto kernel = gemv_f16_kernel<BATCH>;
-    B200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    B200_CUDA_TRY(allow_max_smem(kernel));
     const uint32_t row_blocks = (p.d + kGemvWarps - 1) / kGemvWarps;
     const uint32_t grid = row_blocks < static_cast<uint32_t>(sm_count) ? row_blocks : static_cast<uint32_t>(sm_count);
     B200_CUDA_TRY(launch_dependent(kernel, dim3(grid), dim3(kGemvThreads), smem, stream, p));

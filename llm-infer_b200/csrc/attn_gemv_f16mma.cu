@@ -212,7 +212,7 @@ int b200::launch_gemv_f16_mma(const AttnGemvArgs* a, cudaStream_t stream) {
     p.acc_groups = (slices > 1 && k_split == 1) ? plan.groups_per_cta : 0;
     const uint64_t w_rows = static_cast<uint64_t>(a->d) * (a->swiglu ? 2 : 1);
     auto kernel = dual ? gemv_f16_mma_kernel<8> : gemv_f16_mma_kernel<16>;
-    B200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    B200_CUDA_TRY(allow_max_smem(kernel));
     B200_CUDA_TRY(launch_dependent(kernel, dim3(plan.grid), dim3(dual ? 256 : 512), smem, stream,
                                    static_cast<const uint16_t*>(a->w), w_rows, static_cast<uint64_t>(a->n), p));
     g_launch_count.fetch_add(1, std::memory_order_relaxed);

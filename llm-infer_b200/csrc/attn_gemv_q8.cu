@@ -461,7 +461,7 @@ int gemv_q8_0_launch(const AttnGemvArgs* a, void* stream_v, bool tiled) {
                   : regx     ? gemv_q8_0_kernel<8, kRegxWarps, true, false>
                   : plan.cb == 16 ? gemv_q8_0_kernel<16, kWarps, false, false> : gemv_q8_0_kernel<8, kWarps, false, false>;
     const uint32_t threads = regx_slice ? kRegxSliceWarps * 32 : regx ? kRegxWarps * 32 : kThreads;
-    B200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    B200_CUDA_TRY(allow_max_smem(kernel));
     B200_CUDA_TRY(launch_dependent(kernel, dim3(grid), dim3(threads), smem, stream, tm_w, p));
     g_launch_count.fetch_add(1, std::memory_order_relaxed);
     return ATTN_OK;

@@ -219,6 +219,15 @@ struct DeviceInfo {
 // Properties of the current device (cached per device; no allocation).
 int current_device_info(DeviceInfo* out);
 
+// Lets a kernel (without static shared memory) be launched with all the shared memory that a block of these parts can have. The
+// limit is the process's: set to each call's own size, it could be lowered by another host thread's smaller call between this
+// thread's setting and its launch, which is then refused.
+constexpr int kMaxDynamicSmem = 227 * 1024;
+template <typename Kernel>
+cudaError_t allow_max_smem(Kernel* kernel) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
+}
+
 int launch_decode_split(const DecodeParams& p, uint32_t head_dim, uint32_t hpc, bool qsplit, bool kv_bf16, uint32_t grid,
                         size_t smem_bytes, cudaStream_t stream);
 int launch_merge(const MergeParams& p, cudaStream_t stream, bool dependent_launch);

@@ -654,7 +654,7 @@ extern "C" int attn_prefill_causal(const AttnPrefillArgs* a, void* stream_v) {
     const dim3 grid(static_cast<uint32_t>(std::min<uint64_t>(items, static_cast<uint64_t>(dev.sm_count))));
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     auto launch = [&](auto kernel) -> int {
-        B200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemAlloc)));
+        B200_CUDA_TRY(allow_max_smem(kernel));
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = grid;
         cfg.blockDim = dim3(kThreads);

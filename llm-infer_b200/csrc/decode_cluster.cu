@@ -93,7 +93,7 @@ uint32_t resident_clusters(uint32_t cluster, const DeviceInfo& dev) {
         launch_config(cfg, attr, cluster, cluster, smem, nullptr);
         cfg.numAttrs = 1;
         int n = 0;
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess ||
+        if (allow_max_smem(kernel) != cudaSuccess ||
             cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
             (void)cudaGetLastError();
             n = 0;
@@ -164,7 +164,7 @@ int launch_decode_cluster(const DecodeParams& p, const DecodeClusterPlan& plan, 
         !cache_map(&tm_v, p.v, p, head_dim, plan.rows, plan.hpc, kv_bf16))
         return kClusterNotTaken;  // (strides beyond what a tensor map holds)
     const Kernel kernel = kernel_of(head_dim, plan.hpc, qsplit, kv_bf16);
-    B200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(plan.smem_bytes)));
+    B200_CUDA_TRY(allow_max_smem(kernel));
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr[2];
     launch_config(cfg, attr, plan.segments * plan.cluster, plan.cluster, plan.smem_bytes, stream);

@@ -111,3 +111,12 @@ def test_a_cluster_barrier_stands_before_the_first_remote_shared_memory_store():
             arrive, wait = kernel.find("barrier.cluster.arrive"), kernel.find("barrier.cluster.wait")
             assert 0 <= arrive < wait < at, f"{os.path.basename(path)}: remote store ahead of the cluster barrier"
     assert stores == 1  # argmax
+
+
+def test_no_call_lowers_a_kernels_shared_memory_limit():
+    """The limit of a kernel's dynamic shared memory belongs to the process: set to one call's size it could refuse another
+    thread's launch. Read from the sources: one place sets it, always to the same value."""
+    places = [(os.path.basename(path), line.strip()) for path in sorted(glob.glob(os.path.join(ROOT, "llm-infer_b200", "csrc", "*.cu*")))
+              for line in open(path) if "cudaFuncAttributeMaxDynamicSharedMemorySize" in line]
+    assert places == [("attn_internal.cuh", "return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, "
+                                            "kMaxDynamicSmem);")]

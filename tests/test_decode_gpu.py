@@ -459,3 +459,41 @@ def test_fused_exchange_times_out_cleanly_when_a_peer_never_arrives(attention, w
     torch.cuda.synchronize()
     check_close(wl, got.cpu().numpy(), want, "decode after a timed-out exchange")
     assert int(ws.status.item()) == 0
+
+
+def test_host_threads_with_calls_of_different_sizes(attention, pkg):
+    """Three threads, each with its own stream and workspace, whose calls take the same kernel with different amounts of shared
+    memory (4 to 32 KB of query rows): no launch is refused and every result stays the thread's own."""
+    import ctypes as C
+    import threading
+
+    import torch
+    lib, errors = pkg.binding.load(), []
+
+    def worker(H, max_ctas, start):
+        try:
+            stream = torch.cuda.Stream()
+            with torch.cuda.stream(stream):
+                g = torch.Generator(device="cuda").manual_seed(H)
+                q = torch.randn((1, H, 128), generator=g, device="cuda").half()
+                k, v = (torch.randn((1, 64, 8, 128), generator=g, device="cuda").half() for _ in range(2))
+                ws = attention.DecodeWorkspace(1, H, 8, 128)
+                first = attention.attn_decode(q, k, v, workspace=ws, max_ctas=max_ctas)
+                args, out, _, _ = attention._decode_args(q, k, v, None, torch.empty_like(first), None, None, 0.0, ws, max_ctas)
+                ref, raw, call = C.byref(args), stream.cuda_stream, lib.attn_decode
+                start.wait()
+                codes = {call(ref, raw) for _ in range(20000)}
+                stream.synchronize()
+                assert codes == {0}, codes
+                assert torch.equal(out, first) and int(ws.status.item()) == 0
+        except Exception as e:  # noqa: BLE001 (reported by the test's thread)
+            errors.append(e)
+
+    for max_ctas in (148, 0):
+        start = threading.Barrier(3, timeout=60)
+        threads = [threading.Thread(target=worker, args=(H, max_ctas, start)) for H in (8, 64, 32)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert not errors, errors
