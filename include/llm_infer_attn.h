@@ -88,8 +88,8 @@ typedef struct AttnDecodeArgs {
     uint32_t n_kv_heads;
     uint32_t head_dim;       /* 64 or 128 */
     const uint32_t* kv_len;  /* device pointer [batch], valid rows per sequence; NULL = kv_len_uniform for all. The
-                                values are read on the device and must not exceed the rows the caches hold: the
-                                kernel has no capacity to clamp them to */
+                                values are read on the device and must not exceed the rows the caches hold (see
+                                kv_capacity, to which they are clamped when it is stated) */
     uint32_t kv_len_uniform; /* used when kv_len == NULL */
     uint64_t kv_row_stride;   /* elements between rows; 0 = n_kv_heads*head_dim */
     uint64_t kv_batch_stride; /* elements between sequences; may be 0 only when batch == 1 */
@@ -106,8 +106,8 @@ typedef struct AttnDecodeArgs {
                           every tile that cannot hold that row before it waits for the previous kernel. 0 = wait first. */
     uint32_t kv_capacity; /* rows each sequence's caches hold (the engine's max_seq_len); 0 = not stated. When stated, a
                              length beyond it (a corrupted kv_len[] entry) is clamped to it on the device and
-                             ATTN_STATUS_BAD_SHAPE is ORed into *status, instead of reading past the cache. All
-                             stated rows must be readable; those behind kv_len may hold anything. */
+                             ATTN_STATUS_BAD_SHAPE is ORed into *status, instead of reading past the cache. Rows
+                             behind a sequence's (clamped) length are never read. */
     uint32_t two_pass; /* 0 = the fastest form for the shape, chosen by batch, heads, head_dim, kv_len_uniform or kv_capacity and
                           max_ctas (a stated max_ctas always means the two launches). != 0: always the split pass and the merge
                           pass, with every residual product an MMA of its own: one order of the sums for all capacities and

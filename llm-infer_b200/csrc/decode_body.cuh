@@ -316,7 +316,10 @@ __device__ __forceinline__ void decode_split_body(const DecodeParams& p, unsigne
                 mbar_arrive_expect_tx(bar_full_k + 8 * st, TT * ROWB);
                 mbar_arrive_expect_tx(bar_full_v + 8 * st, TT * ROWB);
                 if constexpr (CLUSTER) {
-                    const int row = static_cast<int>(tok0), head = static_cast<int>(seg.hg * HPC), b = static_cast<int>(seg.b);
+                    // The last tile is moved back to end with the sequence: rows behind its end need not be memory. The rows
+                    // that it repeats (in front of the first row: zeros from the copy engine) are masked by the consumers.
+                    const int row = min(static_cast<int>(tok0), static_cast<int>(seg.len) - TT);
+                    const int head = static_cast<int>(seg.hg * HPC), b = static_cast<int>(seg.b);
                     tma_load_5d_hint(kdst, tm_k, bar_full_k + 8 * st, row, 0, head, b, policy);
                     tma_load_5d_hint(vdst, tm_v, bar_full_v + 8 * st, row, 0, head, b, policy);
                 }
@@ -788,13 +791,15 @@ __device__ __forceinline__ void decode_split_body(const DecodeParams& p, unsigne
         }
 
         // ---- scale, mask rows past the sequence end ----
-        const uint32_t tok = (gt - seg.tile0) * TT + ts * 16 + cq * 2;  // row of s[0][0]; s[1][*] is +8
+        const uint32_t tok = (CLUSTER ? 0u : (gt - seg.tile0) * TT) + ts * 16 + cq * 2;  // row of s[0][0]; s[1][*] is +8
+        // cluster mode: rows of the tile (counted from its start) that an earlier tile has had, see issue_tile
+        const uint32_t repeated = CLUSTER && (gt + 1) * TT > seg.len ? (gt + 1) * TT - seg.len : 0u;
 #pragma unroll
         for (int n = 0; n < 2; ++n) {
 #pragma unroll
             for (int e = 0; e < (LOW8 || PACK8 ? 2 : 4); ++e) {
                 const uint32_t r = tok + n * 8 + (e & 1);
-                s[n][e] = r < seg.len ? s[n][e] * p.scale_log2 : -INFINITY;
+                s[n][e] = (CLUSTER ? r >= repeated : r < seg.len) ? s[n][e] * p.scale_log2 : -INFINITY;
             }
         }
 
@@ -859,13 +864,12 @@ __device__ __forceinline__ void decode_split_body(const DecodeParams& p, unsigne
         }
 
         if constexpr (CLUSTER) {
-            // Rows past the end of the sequence hold whatever the cache holds there: their probability is zero, but zero times
-            // a NaN is not. This warp's rows of the segment's last tile are cleared first (nobody else reads them).
-            const uint32_t row0 = (gt - seg.tile0) * TT + ts * 16;
-            if (row0 + 16 > seg.len) {
+            // The probability of a repeated row is zero, but zero times an infinity is not: this warp's share of those rows is
+            // cleared first (nobody else reads it).
+            if (repeated > ts * 16u) {
                 for (uint32_t c = lane; c < 16 * (D / 8); c += 32) {
                     const uint32_t r = c / (D / 8), at = c & (D / 8 - 1);
-                    if (row0 + r >= seg.len) st_shared_zero16(vbase + hh * HEADB + (at >> 3) * PART + (ts * 16 + r) * 128 + (at & 7) * 16);
+                    if (ts * 16 + r < repeated) st_shared_zero16(vbase + hh * HEADB + (at >> 3) * PART + (ts * 16 + r) * 128 + (at & 7) * 16);
                 }
                 __syncwarp();
             }

@@ -342,6 +342,44 @@ def test_cluster_form_against_the_split_form(attention, wl, B, H, Hkv, D, T, len
     assert int(ws.status.item()) == 0
 
 
+@pytest.mark.parametrize("H,Hkv,D", [(32, 8, 128), (12, 2, 128), (16, 4, 64), (7, 1, 64)])
+@pytest.mark.parametrize("q_dtype,kv_dtype", [("f16", "f16"), ("f32", "bf16")])
+def test_a_stated_capacity_is_no_promise_of_readable_rows(attention, pkg, wl, H, Hkv, D, q_dtype, kv_dtype):
+    """kv_capacity bounds the lengths and nothing else: here it is stated larger than the distance between two sequences, whose
+    last one ends with the memory itself, and the row pitch is wider than a row. A sequence's last tile is moved back to end
+    with the sequence: fewer rows than a tile, exactly one, one more, and remainders around the 16 rows of a warp."""
+    import ctypes as C
+
+    import torch
+    from gpu_util import to_device
+    T, spare, lib = 257, 8, pkg.binding.load()
+    for lens in ([257, 1, 128, 17], [256, 16, 129, 2], [15, 255, 0, 127], [3, 5, 9, 257]):
+        B = len(lens)
+        q, k, v = _rand(wl, H + lens[0], B, H, Hkv, D, T, q_dtype, kv_dtype)
+        qd, kd, vd = to_device(q, q_dtype), to_device(k, kv_dtype), to_device(v, kv_dtype)
+        pitch = Hkv * D + spare
+        flat = [torch.full((((B - 1) * T + lens[-1] - 1) * pitch + Hkv * D,), float("nan"), dtype=kd.dtype, device="cuda")
+                for _ in range(2)]
+        for buf, cache in zip(flat, (kd, vd)):
+            for b, n in enumerate(lens):
+                for i in range(n):
+                    buf[(b * T + i) * pitch:][:Hkv * D] = cache[b, i].reshape(-1)
+        kv_len = torch.tensor(lens, dtype=torch.int32, device="cuda")
+        ws = attention.DecodeWorkspace(B, H, Hkv, D)
+        got = []
+        for two_pass in (1, 0):
+            a, out, _, _ = attention._decode_args(qd, kd, vd, kv_len, None, None, torch.float32, 0.0, ws, 0)
+            a.k, a.v, a.kv_row_stride, a.kv_batch_stride = flat[0].data_ptr(), flat[1].data_ptr(), pitch, T * pitch
+            a.kv_capacity, a.two_pass = 600, two_pass
+            before = attention.kernel_launch_count()
+            assert lib.attn_decode(C.byref(a), torch.cuda.current_stream().cuda_stream) == 0
+            assert attention.kernel_launch_count() - before == 1 + two_pass
+            got.append(out.double())
+        rms = float(got[0].pow(2).mean().sqrt())
+        assert float((got[0] - got[1]).abs().max()) <= 3e-5 * rms  # another order of the sums, as in the test above
+        assert int(ws.status.item()) == 0
+
+
 def test_merge_entry_point(attention, wl, port):
     import torch
     q, k, v = wl.decode_inputs(wl.C4, kv_len=999)
