@@ -158,7 +158,8 @@ int decode_impl(const AttnDecodeArgs* a, void* stream_v, const Exchange* xchg) {
     const uint32_t rows = a->kv_len ? a->kv_capacity : clamped_len(a->kv_len_uniform, a->kv_capacity);
     DecodeClusterPlan cl{};
     if (!xchg && !two_pass && a->max_ctas == 0 &&
-        pick_decode_cluster(a->batch, a->n_heads, a->n_kv_heads, a->head_dim, rows, a->kv_len != nullptr, dev, &cl)) {
+        pick_decode_cluster(a->batch, a->n_heads, a->n_kv_heads, a->head_dim, rows, a->kv_len != nullptr, plan,
+                            p.min_tiles_per_cta, dev, &cl)) {
         DecodeParams c = p;
         c.head_groups = a->n_kv_heads / cl.hpc;
         c.nstages = cl.stages;

@@ -230,9 +230,11 @@ cudaError_t allow_max_smem(Kernel* kernel) {
 
 int launch_decode_split(const DecodeParams& p, uint32_t head_dim, uint32_t hpc, bool qsplit, bool kv_bf16, uint32_t grid,
                         size_t smem_bytes, cudaStream_t stream);
+constexpr uint32_t kMergeWarpRows = 256;  // from here on a warp of the merge pass folds a row's partials by itself
 int launch_merge(const MergeParams& p, cudaStream_t stream, bool dependent_launch);
+struct DecodePlan;
 // The same in one launch of clusters, one cluster per segment (decode_cluster.cu). pick_decode_cluster says whether a call
-// should take it and fills the plan.
+// should take it, given the plan of the split pass that would serve it otherwise, and fills the cluster form's.
 struct DecodeClusterPlan {
     uint32_t rows;      // rows that a sequence's caches hold at least
     uint32_t hpc;       // kv heads per CTA
@@ -241,7 +243,7 @@ struct DecodeClusterPlan {
     size_t smem_bytes;
 };
 bool pick_decode_cluster(uint32_t batch, uint32_t n_heads, uint32_t n_kv_heads, uint32_t head_dim, uint32_t rows, bool ragged,
-                         const DeviceInfo& dev, DecodeClusterPlan* plan);
+                         const DecodePlan& split, uint32_t split_min_tiles, const DeviceInfo& dev, DecodeClusterPlan* plan);
 constexpr int kClusterNotTaken = 1;  // nothing was launched: the other form has to serve the call
 int launch_decode_cluster(const DecodeParams& p, const DecodeClusterPlan& plan, uint32_t head_dim, bool qsplit, bool kv_bf16,
                           cudaStream_t stream);

@@ -335,7 +335,7 @@ int launch_merge(const MergeParams& p, cudaStream_t stream, bool dependent_launc
     if (p.head_dim % 32 != 0) return ATTN_ERR_UNSUPPORTED;
     // Many rows: the split pass's CTAs are shared out over many segments, so a row has few partials (on average
     // (CTAs + segments) / segments of them) and a warp folds them alone; likewise a caller's short stack of partials.
-    const bool few_parts = p.split_grid ? p.rows >= 256 : (p.rows >= 256 && p.n_parts <= 16);
+    const bool few_parts = p.rows >= kMergeWarpRows && (p.split_grid || p.n_parts <= 16);
     if (few_parts && p.xchg_world == 0) {
         switch (p.head_dim) {
             case 32: return launch_merge_rows<1, 1>(p, stream, dependent_launch);

@@ -24,12 +24,34 @@ constexpr uint32_t kMaxCluster = 8;  // portable
 
 // Bytes per ns: one SM over its own tiles (0.74 us per 64 KB tile), and the HBM.
 constexpr double kSmRate = 88, kHbmRate = 6500;
-// What the cluster form saves besides its streaming time, measured as the difference of the two forms' times in graphs of calls
-// beyond their streaming: 2.8 us with uniform lengths (8 x 2048 rows 17.6 -> 14.7 us, 1 x 4096 10.7 -> 9.6), 4.5 us with ragged
-// ones, where the split form also works out which CTAs share a segment (8 sequences up to 2048 15.9 -> 13.7); less a margin (1 x
-// 8192 rows: 12.8 split, 13.1 in clusters). Ragged lengths are on the device: the longest sequence is taken to be as long as
-// its cache, all of them together as kFill of it.
-constexpr double kGainNs = 1500, kRaggedGainNs = 3500, kCtaNs = 100, kFill = 0.56;
+// What the cluster form saves besides its streaming time with one length for all, measured as the difference of the two forms'
+// times in graphs of calls beyond their streaming: 2.8 us (8 x 2048 rows 17.6 -> 14.7 us, 1 x 4096 10.7 -> 9.6), less a margin (1 x
+// 8192 rows: 12.8 split, 13.1 in clusters).
+constexpr double kGainNs = 1500, kCtaNs = 100;
+
+// Ragged lengths are on the device; the host knows how long the caches are, not how they are filled. A segment's share of the
+// SMs is fixed here, so a long sequence among short ones is the worst that can happen (16 caches of 4096 rows, one of them
+// full: 32.6 us, split pass 22.0; all full: 44.0 and 49.4), and the rule looks at that: clusters only where they lose to the
+// split pass for no number of full caches. Both estimates without what each form always takes (kRaggedGainNs apart):
+//   clusters     the longest sequence's tiles on its own SMs (kTileNs each, under load)
+//   split pass   its tiles dealt over all SMs, a bulk copy per row and cache (kCopyNs + kCopyKbNs per KB), the HBM, and where
+//                a warp merges a row by itself (kMergeWarpRows) the partials of a row one after the other
+// Checked on 660 shapes (1 to 48 caches of 256 to 16384 rows, five head geometries, 1 to all of them full, the others 100
+// rows): of the ~ 350 that take the clusters one loses, by 3 % (1 x 8192 with 64 heads), and all fillings together run 1.6 times as
+// fast as in the split form. The rule before, which took every batch as 56 % full, took 550 and lost in 191, by up to 7 times.
+constexpr double kTileNs128 = 840, kTileNs64 = 580, kRaggedGainNs = 1850;
+constexpr double kCopyNs = 30, kCopyKbNs = 12, kPartialNs = 60;
+
+// The split form with `full` caches of `rows` rows and the others next to empty.
+double split_ns(const DecodePlan& s, uint32_t rows, uint32_t full, uint32_t merge_rows, uint32_t min_tiles, uint32_t head_dim) {
+    const uint64_t tiles = static_cast<uint64_t>(full) * s.head_groups * ((rows + s.tile_rows - 1) / s.tile_rows);
+    const uint32_t ctas = active_ctas(s.grid, 0, min_tiles, tiles);
+    const uint32_t row_bytes = s.hpc * head_dim * 2;
+    const double copies = static_cast<double>((tiles + ctas - 1) / ctas) * 2 * s.tile_rows * (kCopyNs + kCopyKbNs / 1024 * row_bytes);
+    const double streaming = 2.0 * full * rows * s.head_groups * row_bytes / kHbmRate;
+    const double merge = merge_rows >= kMergeWarpRows ? kPartialNs * ctas / (full * s.head_groups) : 0;
+    return std::max(copies, streaming) + merge;
+}
 
 template <int D, int HPC, bool QSPLIT, bool BF16>
 __global__ void __launch_bounds__(kThreads, 1) decode_cluster_kernel(const __grid_constant__ DecodeParams p,
@@ -123,23 +145,33 @@ bool cache_map(CUtensorMap* map, const void* cache, const DecodeParams& p, uint3
 }  // namespace
 
 bool pick_decode_cluster(uint32_t batch, uint32_t n_heads, uint32_t n_kv_heads, uint32_t head_dim, uint32_t rows, bool ragged,
-                         const DeviceInfo& dev, DecodeClusterPlan* plan) {
+                         const DecodePlan& split, uint32_t split_min_tiles, const DeviceInfo& dev, DecodeClusterPlan* plan) {
     if (rows == 0 || n_heads / n_kv_heads > 8) return false;
-    const double streaming = (ragged ? kFill : 1.0) * batch * rows * n_kv_heads * head_dim * 4 / kHbmRate;
+    const double one = 4.0 * rows * n_kv_heads * head_dim / kHbmRate;  // streaming of one full cache
+    const double streaming = ragged ? one : batch * one;
     double best = 1e30;
     uint32_t best_hpc = 0, best_cluster = 0;
     for (uint32_t hpc = 8; hpc >= 1; hpc /= 2) {
         if (n_kv_heads % hpc != 0) continue;
         const uint64_t segments = static_cast<uint64_t>(batch) * (n_kv_heads / hpc);
         const uint32_t tile_rows = 16 * (kConsumerWarps / hpc), tiles = (rows + tile_rows - 1) / tile_rows;
-        const double tile_ns = 4.0 * tile_rows * hpc * head_dim / kSmRate;
+        const double tile_ns = !ragged ? 4.0 * tile_rows * hpc * head_dim / kSmRate : head_dim == 128 ? kTileNs128 : kTileNs64;
         for (uint32_t c = kMaxCluster; c >= 1; --c) {
             if (segments > resident_clusters(c, dev)) continue;  // (all of them at once: a second round would double the time)
             const double t = std::max(((tiles + c - 1) / c) * tile_ns, streaming) + kCtaNs * c;
             if (t < best) best = t, best_hpc = hpc, best_cluster = c;
         }
     }
-    if (best_hpc == 0 || best > streaming + (ragged ? kRaggedGainNs : kGainNs)) return false;
+    if (best_hpc == 0) return false;
+    if (!ragged) {
+        if (best > streaming + kGainNs) return false;
+    } else {
+        for (uint32_t full = 1;; full = std::min(2 * full, batch)) {
+            const double split_time = split_ns(split, rows, full, batch * n_heads, split_min_tiles, head_dim);
+            if (std::max(best, full * one) > split_time + kRaggedGainNs) return false;
+            if (full == batch) break;
+        }
+    }
     // ring of K and V tiles, then as in the split pass: query rows of one segment, barriers, two words behind a prefix that
     // this form does not use; the base is aligned to 1024
     const size_t tile = static_cast<size_t>(16 * (kConsumerWarps / best_hpc)) * best_hpc * head_dim * 2;

@@ -342,6 +342,25 @@ def test_cluster_form_against_the_split_form(attention, wl, B, H, Hkv, D, T, len
     assert int(ws.status.item()) == 0
 
 
+# (caches, heads, kv heads, head_dim, rows of a cache): launches. One full cache among short ones keeps most of a cluster launch's
+# SMs idle: clusters are taken where that costs less than the second launch, whatever the lengths turn out to be.
+@pytest.mark.parametrize("B,H,Hkv,D,cap,launches", [
+    (1, 32, 8, 128, 4096, 1), (8, 32, 8, 128, 1024, 1), (16, 32, 8, 128, 512, 1), (16, 32, 4, 64, 2048, 1), (8, 8, 1, 128, 8192, 1),
+    (7, 32, 8, 128, 4096, 2), (16, 32, 8, 128, 2048, 2), (16, 32, 8, 128, 4096, 2), (32, 32, 8, 128, 4096, 2), (8, 16, 16, 64, 3000, 2),
+    (24, 32, 4, 64, 16384, 2)])
+def test_ragged_batches_take_the_clusters_only_where_no_filling_costs_more(attention, B, H, Hkv, D, cap, launches):
+    import torch
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the line lies elsewhere with another number of SMs")
+    cache = torch.zeros((B, cap, Hkv, D), dtype=torch.float16, device="cuda")
+    q = torch.zeros((B, H, D), dtype=torch.float16, device="cuda")
+    lens = torch.full((B,), 100, dtype=torch.int32, device="cuda")
+    before = attention.kernel_launch_count()
+    out = attention.attn_decode(q, cache, cache, lens)
+    assert attention.kernel_launch_count() - before == launches
+    assert bool((out == 0).all())
+
+
 @pytest.mark.parametrize("H,Hkv,D", [(32, 8, 128), (12, 2, 128), (16, 4, 64), (7, 1, 64)])
 @pytest.mark.parametrize("q_dtype,kv_dtype", [("f16", "f16"), ("f32", "bf16")])
 def test_a_stated_capacity_is_no_promise_of_readable_rows(attention, pkg, wl, H, Hkv, D, q_dtype, kv_dtype):
