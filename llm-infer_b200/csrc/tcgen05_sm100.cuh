@@ -80,9 +80,11 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar, uint32_t cta) 
         ::"r"(bar), "r"(cta)
         : "memory");
 }
-// One arrival on the barrier at a cluster address without release semantics, for a hand-back of tensor memory only (reads
-// completed by tcgen05.wait::ld, ordered by tcgen05.fence::before_thread_sync): the release form makes the thread wait until
-// everything it has in flight is visible, ~ 500 clocks where it happens once per block of 32.
+// One arrival on the barrier at a cluster address without release semantics, for a hand-back of tensor memory only. The PTX ISA's
+// pattern for tcgen05 accesses of different threads asks for no more: tcgen05.ld, tcgen05.wait::ld,
+// tcgen05.fence::before_thread_sync, mbarrier.arrive.relaxed.cluster here; try_wait, tcgen05.fence::after_thread_sync, tcgen05.mma
+// there. Every lane of the warp runs the wait and the fence, __syncwarp orders them before the one lane that arrives. The
+// release form makes the thread wait until everything it has in flight is visible, ~ 500 clocks where it happens once per block of 32.
 __device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_bar) {
     asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }

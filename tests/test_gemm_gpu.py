@@ -193,6 +193,31 @@ def test_gemm_q8_0_against_float64(A, m, n_out, k, swiglu):
     assert int(status.item()) == 0
 
 
+@pytest.mark.parametrize("m,n_out,k,swiglu", [(1003, 4096, 4096, False), (700, 2048, 14336, True)])
+def test_gemm_q8_0_hands_its_accumulators_back_in_order(A, m, n_out, k, swiglu):
+    """Four accumulators go round between the MMAs and the warps that read them, once per block of 32: every element is one fixed
+    order of sums, so a hundred calls agree bit for bit, and so does a call of which only a token tile's rows are asked for."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(k)
+    w, _ = _q8_blocks(g, n_out * (2 if swiglu else 1), k)
+    planes = A.expand_q8_0(w)
+    x = torch.randn((m, k), generator=g, device="cuda")
+    pair = (x.half(), (x - x.half().float()).half())
+
+    def call(rows):
+        shape = (rows, n_out)
+        out = tuple(torch.empty(shape, dtype=torch.float16, device="cuda") for _ in range(2)) if swiglu else torch.empty(shape, device="cuda")
+        A.gemm_q8_0(tuple(t[:rows] for t in pair), planes, out=out, swiglu=swiglu)
+        return torch.cat([t.float() for t in out]) if swiglu else out, out
+
+    first, parts = call(m)
+    for _ in range(100):
+        assert torch.equal(call(m)[0], first)
+    few = call(64)[1]  # other tiles, single CTAs or pairs as the cost rule has it
+    for got, want in zip(few, parts) if swiglu else [(few, parts)]:
+        assert torch.equal(got, want[:64])
+
+
 def test_gemm_rows_equal_the_engine_matmul(A, checker):
     """Each token's row of the GEMM against the engine's own per-token matmul() on the fp32 activations."""
     import torch
