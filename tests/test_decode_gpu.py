@@ -199,6 +199,75 @@ def test_length_beyond_the_cache_is_clamped_and_reported(attention, wl, checker)
     check_close(wl, out.cpu().numpy(), want, "clamped length")
 
 
+# The split pass and its merge serve every generation step, long contexts and sharded calls; short calls like those of the two
+# tests above take the clusters, so the two-launch form is asked for here in both ways there are. Prepared words are what a Q8_0
+# generation step has the attention write.
+@pytest.mark.parametrize("words", [False, True])
+@pytest.mark.parametrize("form", ["two_pass", "max_ctas"])
+@pytest.mark.parametrize("H,Hkv,D,lens", [(32, 8, 128, [700, 33, 257]), (18, 2, 64, [1, 700, 130])])
+def test_two_launches_behind_an_appending_kernel(attention, wl, checker, H, Hkv, D, lens, form, words):
+    import torch
+    from gpu_util import check_close, to_device
+    B, T = 3, 700
+    q, k, v = _rand(wl, 177, B, H, Hkv, D, T, "f32", "f16")
+    rng = np.random.default_rng(178)
+    new = [torch.from_numpy(rng.standard_normal((B, Hkv, D), dtype=np.float32)).cuda() for _ in range(2)]
+    qd, kd, vd = torch.from_numpy(q).cuda(), to_device(k, "f16"), to_device(v, "f16")
+    lens_d = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    ws = attention.DecodeWorkspace(B, H, Hkv, D)
+    kw = {"two_pass": True} if form == "two_pass" else {"max_ctas": torch.cuda.get_device_properties(0).multi_processor_count}
+    outs = []
+    for early in (False, True, True):
+        kc, vc = kd.clone(), vd.clone()
+        q_rot = attention.rope_kv_insert(qd.clone(), *new, kc, vc, lens_d - 1, lens_d - 1, theta=10000.0)
+        out = torch.empty((B, H, D), dtype=torch.int32 if words else torch.float32, device="cuda")
+        before = attention.kernel_launch_count()
+        attention.attn_decode(q_rot, kc, vc, lens_d, out=out, workspace=ws, kv_early=early, **kw)
+        assert attention.kernel_launch_count() - before == 2
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[1], outs[2])
+    got = outs[1]
+    if words:  # {hi(x0,x1), hi(x2,x3), lo(x0,x1), lo(x2,x3)} of four elements
+        h = got.view(torch.float16).view(B, H, D // 4, 2, 4).float()
+        got = (h[..., 0, :] + h[..., 1, :]).reshape(B, H, D)
+    want = checker.attn_decode(q_rot.cpu().numpy(), kc.cpu().numpy(), vc.cpu().numpy(), np.array(lens, np.uint32))
+    check_close(wl, got.cpu().numpy(), want, "two launches behind rope insert")
+    assert int(ws.status.item()) == 0
+
+
+@pytest.mark.parametrize("kw", [{"two_pass": True}, {"max_ctas": 148}, {"two_pass": True, "kv_early": True}])
+def test_two_launches_clamp_and_report_a_length_beyond_the_cache(attention, wl, checker, kw):
+    import torch
+    from gpu_util import check_close, to_device
+    q, k, v = _rand(wl, 91, 2, 32, 8, 128, 300)
+    lens = torch.tensor([100, 5000], dtype=torch.int32, device="cuda")
+    ws = attention.DecodeWorkspace(2, 32, 8, 128)
+    before = attention.kernel_launch_count()
+    out = attention.attn_decode(to_device(q, "f32"), to_device(k, "f16"), to_device(v, "f16"), lens, workspace=ws, **kw)
+    assert attention.kernel_launch_count() - before == 2
+    assert int(ws.status.item()) == 2  # ATTN_STATUS_BAD_SHAPE
+    check_close(wl, out.cpu().numpy(), checker.attn_decode(q, k, v, np.array([100, 300], np.uint32)), "clamped length")
+
+
+@pytest.mark.parametrize("two_pass", [False, True])
+@pytest.mark.parametrize("H,Hkv,D", [(32, 8, 128), (14, 2, 64)])
+def test_an_output_off_its_16_byte_boundary(attention, wl, H, Hkv, D, two_pass):
+    """fp32 results that start 4 bytes behind a boundary: element stores in the merges, the same bits, nothing beside them."""
+    import torch
+    from gpu_util import to_device
+    q, k, v = _rand(wl, H, 2, H, Hkv, D, 333)
+    qd, kd, vd = to_device(q, "f32"), to_device(k, "f16"), to_device(v, "f16")
+    ws = attention.DecodeWorkspace(2, H, Hkv, D)
+    want = attention.attn_decode(qd, kd, vd, workspace=ws, two_pass=two_pass)
+    flat = torch.full((2 * H * D + 5,), -7.0, device="cuda")
+    out = flat[1:1 + 2 * H * D].view(2, H, D)
+    before = attention.kernel_launch_count()
+    attention.attn_decode(qd, kd, vd, out=out, workspace=ws, two_pass=two_pass)
+    assert attention.kernel_launch_count() - before == 1 + two_pass
+    assert torch.equal(out, want) and bool((flat[:1] == -7).all()) and bool((flat[1 + 2 * H * D:] == -7).all())
+    assert int(ws.status.item()) == 0
+
+
 def test_checking_build_runs_clean(pkg, wl, checker, tmp_path):
     """The -DATTN_BOUNDS_CHECK build (the decode passes verify their workspace indices and report ATTN_STATUS_BAD_INDEX
     instead of accessing) gives the same results with no status bit on uniform, ragged and single-long-sequence
@@ -261,6 +330,28 @@ def test_max_ctas_limits_split_without_changing_result(attention, wl, checker):
 @pytest.mark.parametrize("H,Hkv,D", [(8, 8, 128), (21, 3, 64), (64, 8, 128), (16, 2, 64), (18, 2, 128)])
 @pytest.mark.parametrize("q_dtype,kv_dtype", [("f32", "f16"), ("f16", "f16"), ("f32", "bf16")])
 def test_residuals_in_the_idle_rows_against_products_of_their_own(attention, wl, H, Hkv, D, q_dtype, kv_dtype):
+    """Up to eight heads per kv head the residual products take the MMAs' rows 8-15; in a generation step (kv_early, lengths
+    on the device, prepared output) and with more heads they are products of their own. Same sums in another order: fp32
+    rounding (2^-24 each, a few hundred), bf16 probabilities and residuals (2^-17), and the prepared form's 2^-21."""
+    import torch
+    from gpu_util import to_device
+    q, k, v = _rand(wl, H + D, 3, H, Hkv, D, 777, q_dtype, kv_dtype)
+    qd, kd, vd = to_device(q, q_dtype), to_device(k, kv_dtype), to_device(v, kv_dtype)
+    lens = torch.tensor([777, 16, 500], dtype=torch.int32, device="cuda")
+    ws = attention.DecodeWorkspace(3, H, Hkv, D)
+    rows = attention.attn_decode(qd, kd, vd, lens, workspace=ws, max_ctas=148).double()
+    words = torch.empty((3, H, D), dtype=torch.int32, device="cuda")
+    attention.attn_decode(qd, kd, vd, lens, out=words, workspace=ws, kv_early=True)
+    # words {hi(x0,x1), hi(x2,x3), lo(x0,x1), lo(x2,x3)} of four elements
+    h = words.view(torch.float16).view(3, H, D // 4, 2, 4).double()
+    own = (h[..., 0, :] + h[..., 1, :]).reshape(3, H, D)
+    assert float((rows - own).abs().max()) <= 3e-5 * float(rows.pow(2).mean().sqrt()) + 2.0 ** -21 * float(rows.abs().max())
+    assert int(ws.status.item()) == 0
+
+
+@pytest.mark.parametrize("H,Hkv,D", [(8, 8, 128), (21, 3, 64), (64, 8, 128), (16, 2, 64), (18, 2, 128)])
+@pytest.mark.parametrize("q_dtype,kv_dtype", [("f32", "f16"), ("f16", "f16"), ("f32", "bf16")])
+def test_residuals_in_the_idle_rows_against_two_pass(attention, wl, H, Hkv, D, q_dtype, kv_dtype):
     """Up to eight heads per kv head the residual products take the MMAs' rows 8-15; with two_pass and with more heads they are
     products of their own. Same sums in another order: fp32 rounding (2^-24 each, a few hundred) and bf16 probabilities and
     residuals (2^-17)."""

@@ -115,16 +115,24 @@ def test_head_dim_128_gqa4_clip_and_partial_rotary(M, checker, prompt_mode):
     _run_case(M, checker, cfg, prompts, n_new=16, seed=2, prompt_mode=prompt_mode)
 
 
-@pytest.mark.parametrize("max_seq_len,prompt,n_new", [(16, 10, 20), (150, 140, 24)])
-def test_sliding_window_with_sink_rows(M, checker, max_seq_len, prompt, n_new):
+def test_sliding_window_with_sink_rows(M, checker):
     """Generation runs past max_seq_len: the cache becomes a ring behind four sink rows whose K is re-rotated every
-    step (src/model/model.cpp:66-68, src/model/block.cpp:150-155). One tile of the cache per sequence, and five of them, of
-    which the attention may ask for four early where that is allowed."""
+    step (src/model/model.cpp:66-68, src/model/block.cpp:150-155)."""
     cfg = M.ModelConfig(dim=512, hidden_dim=512, n_layers=2, n_heads=4, n_kv_heads=4, head_dim=128, vocab_size=500,
-                        max_seq_len=max_seq_len, norm_eps=1e-5, rope_theta=10000.0)
+                        max_seq_len=16, norm_eps=1e-5, rope_theta=10000.0)
     rng = np.random.default_rng(13)
-    prompts = [rng.integers(0, cfg.vocab_size, size=prompt).tolist() for _ in range(2)]
-    _run_case(M, checker, cfg, prompts, n_new=n_new, seed=3)
+    prompts = [rng.integers(0, cfg.vocab_size, size=10).tolist() for _ in range(2)]
+    _run_case(M, checker, cfg, prompts, n_new=20, seed=3)
+
+
+def test_sliding_window_of_several_tiles(M, checker):
+    """The same with a ring of five tiles of cache rows per sequence, of which the attention may ask for four early where that is
+    allowed: in the window the rotary kernel writes inside the ring and turns the sink rows."""
+    cfg = M.ModelConfig(dim=512, hidden_dim=512, n_layers=2, n_heads=4, n_kv_heads=4, head_dim=128, vocab_size=500,
+                        max_seq_len=150, norm_eps=1e-5, rope_theta=10000.0)
+    rng = np.random.default_rng(13)
+    prompts = [rng.integers(0, cfg.vocab_size, size=140).tolist() for _ in range(2)]
+    _run_case(M, checker, cfg, prompts, n_new=24, seed=3)
 
 
 @pytest.mark.parametrize("prompt_mode", ["token", "batched"])
