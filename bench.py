@@ -3,7 +3,7 @@
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 
-N = 1   one step = one batched decode-attention call (split-KV pass + merge pass) on the
+N = 1   one step = one batched decode-attention call (one launch of clusters) on the
         Llama-3-8B-shaped workload: batch 16, 32 query / 8 kv heads, head_dim 128, KV length 4096,
         fp16, inputs resident in HBM. Metric: algorithmic HBM GB/s of that call.
 N > 1   one step = one long-context decode with the KV sequence (131072 rows) sharded evenly over
@@ -367,12 +367,23 @@ def gemv_measure(torch, steps: int, warmup: int, hbm_peak: float, peak_kind: str
     return res
 
 
+def trace_points(stamps, names, t0: int, lowest: bool) -> dict:
+    """Time stamps [CTAs][slots] in ns (0 = not taken) -> name: [minimum,] median and maximum over CTAs in us after t0, for every
+    point that any CTA has passed (a call in one launch has no merge pass and fewer points)."""
+    res = {}
+    for i, name in enumerate(names):
+        rel = sorted((t - t0) / 1e3 for t in stamps[:, i].tolist() if t > 0)
+        if rel:
+            res[name] = [round(x, 2) for x in ([rel[0]] if lowest else []) + [rel[len(rel) // 2], rel[-1]]]
+    return res
+
+
 def decode_trace(torch):
     """Where the time of one attn_decode call goes. Needs the profiling build of the library (python
     llm-infer_b200/build.py --trace, loaded through LLM_INFER_ATTN_LIB): its kernels store the GPU's nanosecond timer
-    at a few points per CTA. For each shape one flushed call is traced five times; printed are, in microseconds after
-    the first CTA of the split pass started, the median and the maximum over CTAs of every point, for the run with the
-    median total."""
+    at a few points per CTA. For each shape, and each form that it can take, one flushed call is traced five times; printed are,
+    in microseconds after the first CTA of the split pass (or of the cluster launch) started, the median and the maximum over CTAs of
+    every point, for the run with the median total."""
     import ctypes as C
     from llm_infer_b200 import attention, binding
     lib = binding.load()
@@ -384,7 +395,7 @@ def decode_trace(torch):
     dev = torch.device("cuda", 0)
     H, Hkv, D = 32, 8, 128
     split_names = ["entry", "previous kernel done", "set-up done", "q in registers", "first K tile landed",
-                   "last tile computed", "partials written", "producer issued last copy"]
+                   "last tile computed", "partials written", "producer issued last copy"]  # clusters: "partials written" = merged and stored
     merge_names = ["entry", "split pass done, addresses ready", "partials folded", "row stored"]
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=dev)
     tr_split = torch.zeros(1024 * 8, dtype=torch.int64, device=dev)
@@ -405,52 +416,55 @@ def decode_trace(torch):
             floors[name].append(e0.elapsed_time(e1) * 1e3)
         floors[name] = round(sorted(floors[name])[3], 2)
     out["event_floor_us"] = floors
-    sms = torch.cuda.get_device_properties(dev).multi_processor_count  # (a stated limit: the two-launch form, which is traced)
+    def traced(calls):
+        """One traced run of `calls`: (event time, stamps of the CTAs that stream, stamps of the merge pass's, if it has any)."""
+        tr_split.zero_()
+        tr_merge.zero_()
+        torch.cuda.synchronize()
+        lib.attn_trace_set_buffers(tr_split.data_ptr(), tr_merge.data_ptr())
+        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        calls(e0, e1)
+        torch.cuda.synchronize()
+        lib.attn_trace_set_buffers(None, None)
+        sp, mg = (tr.view(-1, 8).cpu().numpy().astype("int64") for tr in (tr_split, tr_merge))
+        return round(e0.elapsed_time(e1) * 1e3, 2), sp[sp[:, 0] > 0], mg[mg[:, 0] > 0]
+
+    # Both forms of a call: a stated limit on the CTAs keeps the two launches, a plain call takes one launch of clusters where
+    # that is the faster form.
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count
     for b, t in ((1, 64), (1, 4096), (16, 4096), (1, 16384), (1, 32768), (1, 131072)):
         q = torch.randn((b, H, D), device=dev).half()
         k = torch.randn((b, t, Hkv, D), device=dev, dtype=torch.float16)
         v = torch.randn((b, t, Hkv, D), device=dev, dtype=torch.float16)
         o = torch.empty((b, H, D), device=dev)
         ws = attention.DecodeWorkspace(b, H, Hkv, D, dev)
-        lib.attn_trace_set_buffers(None, None)
-        for _ in range(3):
-            attention.attn_decode(q, k, v, out=o, workspace=ws, max_ctas=sms)
-        runs = []
-        for _ in range(5):
-            flush.zero_()
-            tr_split.zero_()
-            tr_merge.zero_()
-            torch.cuda.synchronize()
-            lib.attn_trace_set_buffers(tr_split.data_ptr(), tr_merge.data_ptr())
-            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            flush.zero_()
-            e0.record()
-            attention.attn_decode(q, k, v, out=o, workspace=ws, max_ctas=sms)
-            e1.record()
-            torch.cuda.synchronize()
+        for max_ctas in (sms, 0):
             lib.attn_trace_set_buffers(None, None)
-            sp = tr_split.view(-1, 8).cpu().numpy().astype("int64")
-            mg = tr_merge.view(-1, 8).cpu().numpy().astype("int64")
-            sp = sp[sp[:, 0] > 0]
-            mg = mg[mg[:, 0] > 0]
-            t0 = int(sp[:, 0].min())
-            rec = {"event_us": round(e0.elapsed_time(e1) * 1e3, 2), "split_ctas": int(len(sp)),
-                   "split_ctas_with_tiles": int((sp[:, 5] > 0).sum()), "merge_ctas": int(len(mg)), "split": {}, "merge": {}}
-            for i, name in enumerate(split_names):
-                col = sp[:, i][sp[:, i] > 0]
-                if len(col):
-                    rel = (col - t0) / 1e3
-                    rec["split"][name] = [round(float(sorted(rel)[len(rel) // 2]), 2), round(float(rel.max()), 2)]
-            for i, name in enumerate(merge_names):
-                col = mg[:, i][mg[:, i] > 0]
-                if len(col):
-                    rel = (col - t0) / 1e3
-                    rec["merge"][name] = [round(float(rel.min()), 2), round(float(sorted(rel)[len(rel) // 2]), 2),
-                                          round(float(rel.max()), 2)]
-            rec["total_us_first_entry_to_last_store"] = round((int(mg[:, 3].max()) - t0) / 1e3, 2)
-            runs.append(rec)
-        runs.sort(key=lambda r: r["event_us"])
-        out[f"b{b}_kv{t}"] = runs[len(runs) // 2]
+            for _ in range(3):
+                before = attention.kernel_launch_count()
+                attention.attn_decode(q, k, v, out=o, workspace=ws, max_ctas=max_ctas)
+                launches = attention.kernel_launch_count() - before
+            if max_ctas == 0 and launches == 2:
+                continue
+
+            def flushed_call(e0, e1):
+                flush.zero_()
+                e0.record()
+                attention.attn_decode(q, k, v, out=o, workspace=ws, max_ctas=max_ctas)
+                e1.record()
+
+            runs = []
+            for _ in range(5):
+                flush.zero_()
+                us, sp, mg = traced(flushed_call)
+                t0 = int(sp[:, 0].min())
+                rec = {"event_us": us, "split_ctas": int(len(sp)), "split_ctas_with_tiles": int((sp[:, 4] > 0).sum()),
+                       "merge_ctas": int(len(mg)), "split": trace_points(sp, split_names, t0, False), "merge": trace_points(mg, merge_names, t0, True)}
+                last = mg[:, 3].max() if len(mg) else sp[:, 6].max()
+                rec["total_us_first_entry_to_last_store"] = round((int(last) - t0) / 1e3, 2)
+                runs.append(rec)
+            runs.sort(key=lambda r: r["event_us"])
+            out[f"b{b}_kv{t}" + ("_clusters" if max_ctas == 0 else "")] = runs[len(runs) // 2]
         del q, k, v, o, ws
     # The same stamps for the LAST of four back-to-back steps on rotated inputs (no flush, no events in between): how
     # consecutive calls overlap through the programmatic-launch chain, with and without early K/V streaming.
@@ -459,37 +473,21 @@ def decode_trace(torch):
              torch.randn((b, t, Hkv, D), device=dev, dtype=torch.float16)) for _ in range(3)]
     o = torch.empty((b, H, D), device=dev)
     ws = attention.DecodeWorkspace(b, H, Hkv, D, dev)
-    for early in (False, True):
-        runs = []
-        for _ in range(5):
-            tr_split.zero_()
-            tr_merge.zero_()
-            torch.cuda.synchronize()
-            lib.attn_trace_set_buffers(tr_split.data_ptr(), tr_merge.data_ptr())
-            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    for max_ctas, early in ((sms, False), (sms, True), (0, False)):
+        def four_calls(e0, e1):
             e0.record()
             for i in range(4):
                 q, k, v = sets[i % 3]
-                attention.attn_decode(q, k, v, out=o, workspace=ws, kv_early=early)
+                attention.attn_decode(q, k, v, out=o, workspace=ws, max_ctas=max_ctas, kv_early=early)
             e1.record()
-            torch.cuda.synchronize()
-            lib.attn_trace_set_buffers(None, None)
-            sp = tr_split.view(-1, 8).cpu().numpy().astype("int64")
-            mg = tr_merge.view(-1, 8).cpu().numpy().astype("int64")
-            sp, mg = sp[sp[:, 0] > 0], mg[mg[:, 0] > 0]
+
+        runs = []
+        for _ in range(5):
+            us, sp, mg = traced(four_calls)
             t0 = int(sp[:, 0].min())
-            rec = {"four_steps_event_us": round(e0.elapsed_time(e1) * 1e3, 2), "split": {}, "merge": {}}
-            for i, name in enumerate(split_names):
-                col = sp[:, i][sp[:, i] > 0]
-                rel = (col - t0) / 1e3
-                rec["split"][name] = [round(float(rel.min()), 2), round(float(sorted(rel)[len(rel) // 2]), 2), round(float(rel.max()), 2)]
-            for i, name in enumerate(merge_names):
-                col = mg[:, i][mg[:, i] > 0]
-                rel = (col - t0) / 1e3
-                rec["merge"][name] = [round(float(rel.min()), 2), round(float(sorted(rel)[len(rel) // 2]), 2), round(float(rel.max()), 2)]
-            runs.append(rec)
+            runs.append({"four_steps_event_us": us, "split": trace_points(sp, split_names, t0, True), "merge": trace_points(mg, merge_names, t0, True)})
         runs.sort(key=lambda r: r["four_steps_event_us"])
-        out[f"loop_b16_kv4096_last_of_4_steps_kv_early={early}"] = runs[len(runs) // 2]
+        out[f"loop_b16_kv4096_last_of_4_steps_kv_early={early}" + ("_clusters" if max_ctas == 0 else "")] = runs[len(runs) // 2]
     print(json.dumps({"decode_trace": out, "legend": {"split": "[median, max] over CTAs, us after the first CTA's entry",
                                                         "merge": "[min, median, max] over CTAs, same origin"}}), flush=True)
 
@@ -559,8 +557,8 @@ def attention_symbol_measure(torch, hbm_peak: float):
 
 
 def gemm_measure(torch, steps: int, warmup: int, tflops_peak: float, peak_kind: str, small: bool = False):
-    """The projection GEMM of the whole-prompt path alone (attn_gemm_f16: tokens x weights on the tensor cores,
-    activations as an fp16 value + residual pair = two MMAs per k-step), on the four projections of a
+    """The projection GEMMs of the whole-prompt path alone (attn_gemm_f16 for fp16 weights, attn_gemm_q8_0 for Q8_0: tokens x
+    weights on the tensor cores, activations as an fp16 value + residual pair = two MMAs per k-step), on the four projections of a
     Llama-3-8B-shaped layer at the C5 prompt load (9101 tokens). Useful FLOPs = 2 m n k; the tensor cores do twice
     that. ``small`` = one 4096^3 case only (profiler captures)."""
     from llm_infer_b200 import attention as A
@@ -580,7 +578,20 @@ def gemm_measure(torch, steps: int, warmup: int, tflops_peak: float, peak_kind: 
         res[f"m{m}_n{n}_k{k}"] = {"us": round(ms * 1e3, 1), "useful_tflops": round(useful / ms / 1e9, 1),
                                   "tensor_tflops": round(2 * useful / ms / 1e9, 1),
                                   "tensor_frac_of_peak": round(2 * useful / ms / 1e9 / tflops_peak, 3)}
-        del hi, lo, ws, out
+        del ws
+        # the same shape with Q8_0 weights (attn_gemm_q8_0), what a Q8_0 model's prompt phase runs
+        planes = []
+        for i in range(2):
+            blocks = torch.randint(0, 256, (n, k // 32, 34), dtype=torch.uint8, device=dev)
+            blocks[..., :2] = torch.tensor([1e-3], device=dev).half().view(torch.uint8)
+            planes.append(A.expand_q8_0(blocks.view(n, k // 32 * 34)))
+        for i in range(max(3, warmup)):
+            A.gemm_q8_0((hi, lo), planes[i % 2], out=out)
+        ms = time_steps(torch, lambda i: A.gemm_q8_0((hi, lo), planes[i % 2], out=out), steps) / steps
+        res[f"q8_0_m{m}_n{n}_k{k}"] = {"us": round(ms * 1e3, 1), "useful_tflops": round(useful / ms / 1e9, 1),
+                                       "tensor_tflops": round(2 * useful / ms / 1e9, 1),
+                                       "tensor_frac_of_peak": round(2 * useful / ms / 1e9 / tflops_peak, 3)}
+        del hi, lo, planes, out
     res["note"] = (f"tensor_tflops = 2 x useful (value + residual MMAs); frac of {peak_kind} cuBLAS bf16 burst peak "
                    f"{tflops_peak:.0f} TFLOP/s")
     return res
@@ -806,7 +817,7 @@ def run_single(args):
         "roofline": {"bound": "hbm", "achieved": gbs, "peak": hbm_peak, "unit": "GB/s", "frac": gbs / hbm_peak,
                      "traffic": ncu_traffic_bytes(), "peak_kind": f"of {peak_kind}",
                      "frac_of_nominal_8tbs": gbs / 8000.0, "algorithmic_bytes_per_launch": alg_bytes,
-                     "note": "duration = CUDA-event time of one step (split pass + merge pass) / steps"},
+                     "note": "duration = CUDA-event time of one step (one launch of clusters) / steps"},
         "cpu_baseline": cpu_baseline,
         "e2e": e2e,
         "gpu_launches": int(launches),
