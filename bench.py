@@ -31,10 +31,10 @@ if ROOT not in sys.path:
 
 
 def ncu_traffic_bytes():
-    """dram__bytes_read.sum + dram__bytes_write.sum of one split-pass launch on the N=1 workload, recorded from a
+    """dram__bytes_read.sum + dram__bytes_write.sum of one decode launch (clusters) on the N=1 workload, recorded from a
     profiler capture together with a hash of the kernel's sources; None when the sources have changed since."""
     import hashlib
-    path = os.path.join(ROOT, "profiles", "decode_split_traffic.json")
+    path = os.path.join(ROOT, "profiles", "decode_traffic.json")
     try:
         with open(path) as f:
             rec = json.load(f)

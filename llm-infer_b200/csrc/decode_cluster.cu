@@ -5,8 +5,8 @@
 // L2 and the dependency between the two cost 3 to 5 us of device time and a launch, whatever the length. Here a segment's
 // share of the SMs is fixed, so ragged lengths leave SMs idle; that is the price, and an estimate of both decides
 // (pick_decode_cluster). What bounds it: up to a few tiles per CTA the chain launch - query - first tile - merge (5 us), then
-// one SM's rate over its own tiles (0.74 us per 64 KB) or the HBM: 16 x 4096 rows of 8 heads of 128 44.1 us (6.1 TB/s, 46.9 in
-// the two-launch form), 8 x 2048 14.7 (17.6), 1 x 4096 9.6 (10.7), 16 x up to 1000 of 4 heads of 64 7.8 (12.3).
+// one SM's rate over its own tiles (0.74 us per 64 KB) or the HBM: 16 x 4096 rows of 8 heads of 128 44.0 us (6.1 TB/s, 47.3 in
+// the two-launch form), 8 x 2048 14.7 (17.6), 1 x 4096 9.7 (10.8), 16 x up to 1000 of 4 heads of 64 7.8 (12.3).
 #include <algorithm>
 #include <atomic>
 
@@ -26,7 +26,9 @@ constexpr uint32_t kMaxCluster = 8;  // portable
 constexpr double kSmRate = 88, kHbmRate = 6500;
 // What the cluster form saves besides its streaming time with one length for all, measured as the difference of the two forms'
 // times in graphs of calls beyond their streaming: 2.8 us (8 x 2048 rows 17.6 -> 14.7 us, 1 x 4096 10.7 -> 9.6), less a margin (1 x
-// 8192 rows: 12.8 split, 13.1 in clusters).
+// 8192 rows: 12.8 split, 13.1 in clusters). kCtaNs: one more CTA in a cluster's barriers and merge (time stamps from the last tile to
+// the last store: 2.3 us with one CTA per cluster, 3.9 with eight, twice this value at most; it decides between plans whose
+// tiles take the same time).
 constexpr double kGainNs = 1500, kCtaNs = 100;
 
 // Ragged lengths are on the device; the host knows how long the caches are, not how they are filled. A segment's share of the
